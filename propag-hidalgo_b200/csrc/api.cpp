@@ -279,7 +279,7 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
   if (!jobs) return fail(PROPAG_ERR_INVALID, "null jobs");
   CK(cudaSetDevice(e->device));
   // ---- validate and lay out per-job scratch ----
-  std::vector<JobDev> jd(n_jobs);
+  std::vector<JobDev> jd(n_jobs, JobDev{});
   std::vector<size_t> off(n_jobs);
   std::vector<int> tw(n_jobs), th(n_jobs);
   size_t job_bytes = 0;
@@ -323,38 +323,15 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
     tw[i] = std::min<int>(T, (int)j.width);
     th[i] = std::min<int>(T, (int)j.height);
     off[i] = job_bytes;
-    // references, referrer boxes, boundary bits, 8 travel-time planes, the
-    // second state copy (time, references) and the pending bitmap of
-    // global-memory tiles
+    // fifteen words a cell, the boundary bits and the pending bitmap: packed
+    // records (fire and box_x0, two state copies, the other box corners) for
+    // global-memory tiles, or references, referrer boxes and travel-time
+    // planes for shared-memory ones
     job_bytes += align_up(N * 4, 256) * 15 + (j.boundaries ? 0 : align_up(words * 4, 256)) +
                  align_up(words * 4, 256);
     max_cells = std::max<uint64_t>(max_cells, N);
   }
   CK(e->job_scratch.reserve(job_bytes, stream));
-  for (uint32_t i = 0; i < n_jobs; ++i) {
-    const uint64_t N = (uint64_t)jd[i].W * jd[i].H;
-    size_t o = off[i];
-    uint32_t *arr[5];
-    for (int k = 0; k < 5; ++k) {
-      arr[k] = e->job_scratch.at<uint32_t>(o);
-      o += align_up(N * 4, 256);
-    }
-    jd[i].refs = arr[0];
-    jd[i].box_x0 = arr[1];
-    jd[i].box_y0 = arr[2];
-    jd[i].box_x1 = arr[3];
-    jd[i].box_y1 = arr[4];
-    jd[i].bnd = jobs[i].boundaries ? jobs[i].boundaries : e->job_scratch.at<uint32_t>(o);
-    if (!jobs[i].boundaries) o += align_up(((N + 31) / 32) * 4, 256);
-    jd[i].tt = e->job_scratch.at<float>(o);
-    jd[i].tt_plane = (int64_t)(align_up(N * 4, 256) / 4);
-    o += 8 * align_up(N * 4, 256);
-    jd[i].time1 = e->job_scratch.at<float>(o);
-    o += align_up(N * 4, 256);
-    jd[i].refs1 = e->job_scratch.at<uint32_t>(o);
-    o += align_up(N * 4, 256);
-    jd[i].pending = e->job_scratch.at<uint32_t>(o);  // kept below for global-memory tiles only
-  }
   // ---- cluster size and tile residency ----
   // A tile launch runs in the cluster's shared memory when the tile and its
   // halo fit in the dynamic shared-memory budget of the cluster's CTAs.
@@ -442,20 +419,48 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
   // First sweeps skip unchanged cells (pending bitmap) on global-memory tiles
   // of grids below 2^27 cells (a warp sums 32 referrer-box areas in 32 bits);
   // shared-memory tiles evaluate the whole tile in a launch's first sweep.
-  for (uint32_t i = 0; i < n_jobs; ++i)
-    if (jd[i].smem_tile != kSmemTileGlobal || (uint64_t)jd[i].W * jd[i].H >= (1ull << 27))
-      jd[i].pending = nullptr;
+  for (uint32_t i = 0; i < n_jobs; ++i) {
+    JobDev &d = jd[i];
+    const uint64_t N = (uint64_t)d.W * d.H;
+    const size_t plane = align_up(N * 4, 256), words = align_up((N + 31) / 32 * 4, 256);
+    size_t o = off[i];
+    auto take = [&](size_t bytes) {
+      char *at = e->job_scratch.at<char>(o);
+      o += bytes;
+      return at;
+    };
+    if (d.smem_tile == kSmemTileGlobal) {
+      d.fire4 = reinterpret_cast<float4 *>(take(4 * plane));
+      d.st0 = reinterpret_cast<CellState *>(take(4 * plane));
+      d.st1 = reinterpret_cast<CellState *>(take(4 * plane));
+      d.box_x0 = reinterpret_cast<uint32_t *>(d.fire4) + 3;
+      d.box_x0_step = 4;
+    } else {
+      d.tt = reinterpret_cast<float *>(take(8 * plane));
+      d.tt_plane = (int64_t)(plane / 4);
+      d.refs = reinterpret_cast<uint32_t *>(take(plane));
+      d.box_x0 = reinterpret_cast<uint32_t *>(take(plane));
+      d.box_x0_step = 1;
+    }
+    d.box_y0 = reinterpret_cast<uint32_t *>(take(plane));
+    d.box_x1 = reinterpret_cast<uint32_t *>(take(plane));
+    d.box_y1 = reinterpret_cast<uint32_t *>(take(plane));
+    d.bnd = jobs[i].boundaries ? jobs[i].boundaries : reinterpret_cast<uint32_t *>(take(words));
+    d.pending = nullptr;
+    if (d.smem_tile == kSmemTileGlobal && N < (1ull << 27)) d.pending = reinterpret_cast<uint32_t *>(take(words));
+  }
   e->last_cluster = group ? PROPAG_CLUSTER_GROUPS : csize;
   e->last_group = group;
   e->last_smem = smem;
-  const size_t words_max = tn_max / 32 + 1;
-  // global-memory tiles: each CTA of a team has its own update region
+  // global-memory tiles: each CTA of a team has its own words of the dirty
+  // bitmap and its own update region
   const size_t team_ctas = group ? group : (size_t)csize;
-  const size_t upd_max = tn_max + 32 * (team_ctas + 1);
+  const size_t words_max = (size_t)owner_words((uint32_t)tn_max, (uint32_t)team_ctas) * team_ctas;
+  const size_t upd_max = words_max * 32;
   const size_t ovf_list_bytes = align_up((size_t)csize * ovf_cap * 2, 256);
   const size_t ovf_upd_bytes = align_up((size_t)csize * ovf_cap * sizeof(Update), 256);
-  // three dirty bitmaps (in rotation) and two update arrays (by sweep parity)
-  const size_t slot_bytes = 3 * align_up(words_max * 4, 256) + 2 * align_up(upd_max * sizeof(TileUpdate), 256) +
+  // two dirty bitmaps (alternating) and two update arrays (by sweep parity)
+  const size_t slot_bytes = 2 * align_up(words_max * 4, 256) + 2 * align_up(upd_max * sizeof(TileUpdate), 256) +
                             256 + ovf_list_bytes + ovf_upd_bytes;
   CK(e->slot_scratch.reserve(slot_bytes * n_slots, stream));
   // meta: jobs, slots, stats, queue
@@ -494,7 +499,7 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
     sd.dirty = e->slot_scratch.at<uint32_t>(o);
     sd.dirty_words = (uint32_t)(align_up(words_max * 4, 256) / 4);
     sd.pad0 = 0;
-    o += 3 * align_up(words_max * 4, 256);
+    o += 2 * align_up(words_max * 4, 256);
     sd.upd = e->slot_scratch.at<TileUpdate>(o);
     o += 2 * align_up(upd_max * sizeof(TileUpdate), 256);
     sd.ctr = e->slot_scratch.at<uint32_t>(o);
@@ -505,7 +510,7 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
     sd.ovf_cap = (uint32_t)ovf_cap;
     sd.pad = 0;
     // the dirty bitmap and counters must start cleared
-    CK(cudaMemsetAsync(sd.dirty, 0, 3 * align_up(words_max * 4, 256), stream));
+    CK(cudaMemsetAsync(sd.dirty, 0, 2 * align_up(words_max * 4, 256), stream));
     CK(cudaMemsetAsync(sd.ctr, 0, 64, stream));  // counters and barrier arrivals
   }
   JobDev *d_jobs = e->meta.at<JobDev>(0);
@@ -931,6 +936,7 @@ extern "C" int propag_run_device_static(const PropagJob *job, void *stream_ptr, 
   uint32_t *cells = reinterpret_cast<uint32_t *>(base + kStaticCellsOff);
   d.refs = cells;
   d.box_x0 = cells + kStaticMaxCells;
+  d.box_x0_step = 1;
   d.box_y0 = cells + 2 * kStaticMaxCells;
   d.box_x1 = cells + 3 * kStaticMaxCells;
   d.box_y1 = cells + 4 * kStaticMaxCells;

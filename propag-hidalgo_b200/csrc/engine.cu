@@ -45,6 +45,7 @@
 #include <cfloat>
 #include <cstdint>
 
+#include "dda_columns.cuh"
 #include "engine.cuh"
 #include "propag_device.cuh"
 
@@ -122,17 +123,20 @@ __global__ void __launch_bounds__(256) prep_kernel(const JobDev *__restrict__ jo
           b |= !similar_fires(nb, me) && me.speed_max < nb.speed_max;
         }
       }
-      if (j.tt && me.speed_max != 0.0f) {
+      if (j.fire4) {  // packed records of global-memory tiles
+        j.fire4[i] = make_float4(me.speed_max, me.azimuth_max, me.eccentricity, __uint_as_float(kEmptyBox));
+        const CellState none{FLT_MAX, kNoRef, 0u, 0u};
+        j.st0[i] = none;
+        j.st1[i] = none;
+      } else {
+        if (j.tt && me.speed_max != 0.0f) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) j.tt[k * j.tt_plane + i] = dir_inv_speed(dc, k, me, refm);
+          for (int k = 0; k < 8; ++k) j.tt[k * j.tt_plane + i] = dir_inv_speed(dc, k, me, refm);
+        }
+        j.time[i] = FLT_MAX;
+        j.refs[i] = kNoRef;
+        j.box_x0[i] = kEmptyBox;
       }
-      j.time[i] = FLT_MAX;
-      j.refs[i] = kNoRef;
-      if (j.time1) {
-        j.time1[i] = FLT_MAX;
-        j.refs1[i] = kNoRef;
-      }
-      j.box_x0[i] = kEmptyBox;
       j.box_y0[i] = kEmptyBox;
       j.box_x1[i] = 0u;
       j.box_y1[i] = 0u;
@@ -157,29 +161,40 @@ __global__ void ignite_kernel(const JobDev *__restrict__ jobs) {
     float t;
   };
   const Ign *ign = (const Ign *)j.ignitions;
+  const bool packed = j.fire4 != nullptr;
   for (uint32_t k = 0; k < j.n_ignitions; ++k) {
     if (ign[k].x >= (uint32_t)j.W || ign[k].y >= (uint32_t)j.H) continue;
-    j.time[ign[k].x + (int64_t)ign[k].y * j.W] = ign[k].t;
+    const int64_t c = ign[k].x + (int64_t)ign[k].y * j.W;
+    if (packed)
+      j.st0[c].time = ign[k].t;
+    else
+      j.time[c] = ign[k].t;
   }
   for (uint32_t k = 0; k < j.n_ignitions; ++k) {
     if (ign[k].x >= (uint32_t)j.W || ign[k].y >= (uint32_t)j.H) continue;
     const int64_t c = ign[k].x + (int64_t)ign[k].y * j.W;
-    if (j.time[c] != FLT_MAX) {
-      j.refs[c] = pack_ref(ign[k].x, ign[k].y);
-      j.box_x0[c] = j.box_x1[c] = ign[k].x;
+    const float t = packed ? j.st0[c].time : j.time[c];
+    if (t != FLT_MAX) {
+      const uint32_t r = pack_ref(ign[k].x, ign[k].y);
+      if (packed) {
+        // a cell that references itself visits itself twice, or is blocked at once
+        const bool b = (j.bnd[c >> 5] >> (c & 31)) & 1u;
+        j.st0[c].ref = r;
+        j.st0[c].los = b ? kLosBlocked | 1u : 2u;
+      } else {
+        j.refs[c] = r;
+      }
+      j.box_x0[c * j.box_x0_step] = j.box_x1[c] = ign[k].x;
       j.box_y0[c] = j.box_y1[c] = ign[k].y;
     }
-    if (j.time1) {  // the second state copy starts equal
-      j.time1[c] = j.time[c];
-      j.refs1[c] = j.refs[c];
-    }
+    if (packed) j.st1[c] = j.st0[c];  // the second state copy starts equal
   }
   // the neighbours of the burning cells are the cells that can improve first
   if (j.pending) {
     for (uint32_t k = 0; k < j.n_ignitions; ++k) {
       if (ign[k].x >= (uint32_t)j.W || ign[k].y >= (uint32_t)j.H) continue;
       const int64_t c = ign[k].x + (int64_t)ign[k].y * j.W;
-      if (!(j.time[c] < j.max_time && j.speed[c] != 0.0f)) continue;
+      if (!(j.st0[c].time < j.max_time && j.speed[c] != 0.0f)) continue;
       for (int dy = -1; dy <= 1; ++dy)
         for (int dx = -1; dx <= 1; ++dx) {
           const int ax = (int)ign[k].x + dx, ay = (int)ign[k].y + dy;
@@ -220,20 +235,6 @@ struct Counters {
 // cell's own time); only the walks the sequential loop performs (candidate
 // also faster than every earlier offer) are counted, so the counters match
 // the reference's order exactly.  Called by all 32 lanes.
-struct GlobalAcc {
-  const JobDev &j;
-  const float *time;  // the state copy this sweep reads
-  const uint32_t *refs;
-  __device__ __forceinline__ void cell(int x, int y, float &t, uint32_t &r) const {
-    const int64_t n = x + (int64_t)y * j.W;
-    t = __ldcg(time + n);
-    r = __ldcg(refs + n);
-  }
-  __device__ __forceinline__ float time_of(uint32_t r) const {
-    return __ldcg(time + ref_x(r) + (int64_t)ref_y(r) * j.W);
-  }
-};
-
 template <typename Acc>
 __device__ __forceinline__ Best evaluate_coop(const JobDev &j, const DirConst &dc, const Acc &acc,
                                               int x, int y, Best own, bool valid, uint32_t lane,
@@ -406,9 +407,119 @@ __device__ __forceinline__ void warp_scan_boxes(ScanBox *sb, const Box &box, uin
   __syncwarp();
 }
 
-__device__ __forceinline__ void sync_cluster() {
-  __threadfence();
-  cg::this_cluster().sync();
+// Division of any 32-bit value by a small divisor (the team's CTA count, the
+// tile's width) with a multiplication: the estimate is at most one short.
+struct FastDiv {
+  uint32_t d, m;  // m = floor((2^32 - 1) / d)
+  __device__ __forceinline__ explicit FastDiv(uint32_t v) : d(v), m(0xFFFFFFFFu / v) {}
+  __device__ __forceinline__ uint32_t div(uint32_t v, uint32_t &rem) const {
+    uint32_t q = __umulhi(v, m);
+    rem = v - q * d;
+    if (rem >= d) {
+      rem -= d;
+      ++q;
+    }
+    return q;
+  }
+};
+
+// Referrer boxes too large for a warp's scan, left to the whole CTA at the end
+// of the sweep's evaluations (corners and the referenced cell, 16 bits each).
+struct ScanItem {
+  uint32_t lo, hi, want;
+};
+constexpr uint32_t kScanQueue = 512;
+// Boxes up to this many cells are scanned at once by the warp that found them;
+// larger ones by the CTA.  The largest box of a sweep set the sweep's time
+// while one warp scanned it (4096^2 scenario: the slowest warp's scans took
+// 4.7 us of a 10.7 us sweep on average, 12.6 us in a tenth of the sweeps).
+constexpr uint32_t kScanInline = 32;
+
+// Whether cell (xx, yy) references `want` and burns in the state X: a cell
+// that does not burn is skipped by its neighbours, and requiring it makes the
+// marked set independent of the order of this sweep's commits.
+__device__ __forceinline__ bool referrer(const JobDev &j, const CellState *__restrict__ X, int xx, int yy,
+                                         uint32_t want) {
+  const int64_t c = xx + (int64_t)yy * j.W;
+  const uint2 s = __ldcg(reinterpret_cast<const uint2 *>(X + c));
+  return s.y == want && __uint_as_float(s.x) < j.max_time && __ldg(&j.fire4[c].x) != 0.0f;
+}
+
+// The referrer boxes of a warp's four cells (a box is common to its cell's
+// eight lanes): the large ones go to the CTA's queue, the others are scanned
+// as one concatenation, 32 cells per step.  hit_fn is called by the lanes
+// whose cell is a referrer.
+template <typename HitFn>
+__device__ __forceinline__ void warp_scan_boxes4(const Box &box, uint32_t want, const JobDev &j,
+                                                 const CellState *__restrict__ X, uint32_t lane,
+                                                 Counters &cnt, ScanItem *queue, uint32_t *queue_ctr,
+                                                 HitFn hit_fn) {
+  uint32_t area = box.area();
+  if ((lane & 7u) == 0) {
+    cnt.scans += area ? 1 : 0;
+    cnt.scan_cells += area;
+  }
+  if (area > kScanInline) {
+    uint32_t at = 0;
+    if ((lane & 7u) == 0) {
+      at = atomicAdd(queue_ctr, 1u);
+      if (at < kScanQueue)
+        queue[at] = ScanItem{(uint32_t)box.x0 | ((uint32_t)box.y0 << 16), (uint32_t)box.x1 | ((uint32_t)box.y1 << 16), want};
+    }
+    at = __shfl_sync(0xFFu << (lane & 24u), at, lane & 24u);
+    if (at < kScanQueue) area = 0;  // a full queue: scanned here after all
+  }
+  __syncwarp();
+  uint32_t end[4];  // ends of the four boxes in the concatenation
+#pragma unroll
+  for (int g = 0; g < 4; ++g) end[g] = __shfl_sync(kFull, area, 8 * g) + (g ? end[g - 1] : 0u);
+  for (uint32_t q0 = 0; q0 < end[3]; q0 += 32) {
+    const uint32_t q = q0 + lane;
+    const int g = (q >= end[0]) + (q >= end[1]) + (q >= end[2]);
+    const uint32_t begin = g == 0 ? 0u : g == 1 ? end[0] : g == 2 ? end[1] : end[2];
+    const int bx0 = __shfl_sync(kFull, box.x0, 8 * g), by0 = __shfl_sync(kFull, box.y0, 8 * g);
+    const int bx1 = __shfl_sync(kFull, box.x1, 8 * g);
+    const uint32_t w = __shfl_sync(kFull, want, 8 * g);
+    if (q < end[3]) {
+      const uint32_t bw = (uint32_t)(bx1 - bx0 + 1), a = q - begin;
+      const int xx = bx0 + (int)(a % bw), yy = by0 + (int)(a / bw);
+      if (referrer(j, X, xx, yy, w)) hit_fn(xx, yy);
+    }
+  }
+}
+
+// The CTA's queued boxes, kScanRun cells a thread in flight.
+constexpr int kScanRun = 4;
+template <typename HitFn>
+__device__ __forceinline__ void cta_scan_boxes(const ScanItem *queue, uint32_t n, const JobDev &j,
+                                               const CellState *__restrict__ X, HitFn hit_fn) {
+  for (uint32_t i = 0; i < n; ++i) {
+    const ScanItem it = queue[i];
+    const int bx0 = (int)(it.lo & 0xFFFFu), by0 = (int)(it.lo >> 16);
+    const uint32_t bw = (it.hi & 0xFFFFu) - (it.lo & 0xFFFFu) + 1u;
+    const uint32_t area = bw * ((it.hi >> 16) - (it.lo >> 16) + 1u);
+    const FastDiv by_w(bw);
+    for (uint32_t a0 = threadIdx.x; a0 < area; a0 += kScanRun * blockDim.x) {
+      uint2 s[kScanRun];
+#pragma unroll
+      for (int r = 0; r < kScanRun; ++r) {
+        const uint32_t a = a0 + (uint32_t)r * blockDim.x;
+        s[r] = make_uint2(0u, ~it.want);
+        if (a < area) {
+          uint32_t col;
+          const uint32_t row = by_w.div(a, col);
+          s[r] = __ldcg(reinterpret_cast<const uint2 *>(X + (bx0 + (int)col) + (int64_t)(by0 + (int)row) * j.W));
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < kScanRun; ++r) {
+        if (s[r].y != it.want) continue;
+        uint32_t col;
+        const int yy = by0 + (int)by_w.div(a0 + (uint32_t)r * blockDim.x, col), xx = bx0 + (int)col;
+        if (__uint_as_float(s[r].x) < j.max_time && __ldg(&j.fire4[xx + (int64_t)yy * j.W].x) != 0.0f) hit_fn(xx, yy);
+      }
+    }
+  }
 }
 
 // ---- team synchronisation ----
@@ -460,15 +571,20 @@ struct Team {
   // passed barrier k + 1, which the leader reaches after the clear.
   uint32_t *cnt3 = nullptr;
   bool cnt_leader = false;
-  uint32_t dsweep = 0;  // every thread: sweeps of global-memory tiles (dirty bitmap rotation)
+  uint32_t dsweep = 0;  // every thread: sweeps of global-memory tiles (which dirty bitmap is read)
   uint32_t cnt_phase = 0;  // thread 0: counting barriers passed, mod 3
   // global_fence = false: cluster mode orders shared-memory accesses only.
-  // improved: this CTA improved a cell in the phase that ends here;
-  // *improving receives the number of the team's CTAs that did.
-  __device__ bool sync(bool global_fence = true, bool improved = false, uint32_t *improving = nullptr) {
+  // *improved (shared memory, may be null) is not zero when this CTA improved
+  // a cell in the phase that ends here; *improving receives the number of the
+  // team's CTAs that did.
+  __device__ bool sync(bool global_fence = true, const uint32_t *improved_ctr = nullptr,
+                       uint32_t *improving = nullptr) {
     const long long t0 = threadIdx.x == 0 ? clock64() : 0;
     if (!bar) {
-      if (improving && threadIdx.x == 0 && improved) atomicAdd(cnt3 + cnt_phase, 1u);
+      if (improving) {
+        __syncthreads();  // the CTA's updates are counted
+        if (threadIdx.x == 0 && *improved_ctr) atomicAdd(cnt3 + cnt_phase, 1u);
+      }
       if (global_fence || improving) __threadfence();
       cg::this_cluster().sync();
       if (threadIdx.x == 0) {
@@ -487,6 +603,7 @@ struct Team {
     }
     __syncthreads();
     if (threadIdx.x == 0) {
+      const bool improved = improved_ctr && *improved_ctr != 0u;
       const uint32_t w = phase & 1u;
       ++phase;
       target[w] += G;  // every CTA of the group passes the same barriers
@@ -533,78 +650,107 @@ struct TileDesc {
 };
 
 // ================================================ global-memory tiles ====
-// The tile's state stays in global memory (L2), in two copies X0 (the job's
-// arrays) and X1: sweep s reads X[s & 1] and writes X[(s + 1) & 1], so that a
-// sweep is a single phase between two team barriers.  The cells are dealt to
-// the team's R CTAs by 32-cell words of the dirty bitmap, word w to CTA
-// w % R, and only a cell's owner writes it.  In sweep s a CTA
-//   1. compacts the marked cells of its words in bitmap D[s & 1] (all its
-//      cells on the first sweep) into a work list in shared memory, a chunk
-//      of blockDim.x words at a time, clearing the words;
-//   2. evaluates them against X[s & 1] and appends its improvements to its
-//      update region of parity s & 1;
-//   3. copies its improvements of sweep s - 1 (already in X[s & 1]) into
-//      X[(s + 1) & 1], then writes this sweep's improvements there, marks
-//      the 3x3 neighbourhoods of the burning ones in D[(s + 1) & 1] and scans
-//      their referrer boxes (reading X[s & 1]);
-//   4. adds its improvement count to the team's and meets the team.
+// The tile's state stays in global memory (L2), in two copies X0 and X1 of
+// packed records (time, reference, line of sight): sweep s reads X[s & 1] and
+// writes X[(s + 1) & 1], so that a sweep is a single phase between two team
+// barriers.  The cells are dealt to the team's R CTAs in groups of four (see
+// owner_words), and only a cell's owner writes it.  In sweep s a CTA
+//   1. loads its words of the dirty bitmap D[s & 1] (its pending cells on the
+//      first sweep), clears them and turns the bits into a work list in
+//      shared memory, a chunk at a time; meanwhile it copies its improvements
+//      of sweep s - 1 (already in X[s & 1]) into X[(s + 1) & 1];
+//   2. evaluates the listed cells against X[s & 1], eight lanes to a cell, and
+//      commits each improvement at once, by the lanes that found it: they
+//      walk the line of sight to the new reference, write the record to
+//      X[(s + 1) & 1], grow the reference's box, mark the 3x3 neighbourhood of
+//      a burning cell in D[(s + 1) & 1] and scan the cell's referrer box
+//      (reading X[s & 1]);
+//   3. meets the team; the barrier reports how many CTAs improved a cell.
 // After a sweep without improvements both copies hold the same state.  Marks
-// are bit reductions without a return value; the improvement count is the
-// only global atomic a CTA makes per sweep.  The referrer scans read the
+// are bit reductions without a return value.  The referrer scans read the
 // references as the sweep started: a referrer whose reference changes in this
 // sweep improved, so its neighbourhood is marked anyway, and one that did not
 // reads the same reference either way -- the marks are those of scans run
 // after the commits.
+//
+// What bounds it: a sweep of a few thousand cells over 148 CTAs is a chain of
+// dependent L2 round trips (0.3-0.4 us each) between two barriers (1.3 us), so
+// every step above is there to shorten that chain.  The line of sight is
+// walked when a cell adopts its reference, by the eight lanes of the cell at
+// once, instead of by every neighbour in every later evaluation.
 
-// Marks the 3x3 neighbourhood of tile cell (lx, ly), centre excluded, in the
-// dirty bitmap: per row the (up to) three cells are consecutive bits, so a
-// row takes one reduction, two where it straddles a word.
-__device__ __forceinline__ void mark3x3_bits(uint32_t *dirty, int lx, int ly, int TW, int TH) {
-  const int xa = max(lx - 1, 0), xb = min(lx + 1, TW - 1);  // columns of the 3x3 inside the tile
-  if (xa > xb) return;
-#pragma unroll
-  for (int dy = -1; dy <= 1; ++dy) {
-    const int ay = ly + dy;
-    if (ay < 0 || ay >= TH) continue;
+// Where the cells of a global-memory tile keep their dirty bits.
+struct TileBits {
+  int TW, TH;
+  uint32_t wpo;  // words per owner
+  FastDiv by_r, by_tw;
+  __device__ __forceinline__ TileBits(int tw, int th, uint32_t R)
+      : TW(tw), TH(th), wpo(owner_words((uint32_t)tw * (uint32_t)th, R)), by_r(R), by_tw((uint32_t)tw) {}
+  // The (up to) three cells of row dy - 1 of the 3x3 neighbourhood of tile
+  // cell (lx, ly), centre excluded: bit i of `run` is tile cell k0 + i, with
+  // k0 the first cell of a group (so the run spans one group or two).
+  __device__ __forceinline__ uint32_t row_run(int lx, int ly, int dy, uint32_t &g) const {
+    const int xa = max(lx - 1, 0), xb = min(lx + 1, TW - 1);  // columns inside the tile
+    const int ay = ly + dy - 1;
+    if (xa > xb || ay < 0 || ay >= TH) return 0u;
+    uint32_t run = (2u << (xb - xa)) - 1u;
+    if (dy == 1 && lx >= xa && lx <= xb) run &= ~(1u << (lx - xa));
     const uint32_t k0 = (uint32_t)xa + (uint32_t)ay * (uint32_t)TW;
-    // bits of columns xa..xb, without the centre on the middle row
-    uint32_t run = (1u << (xb - xa + 1)) - 1u;
-    if (dy == 0 && lx >= xa && lx <= xb) run &= ~(1u << (lx - xa));
-    const uint32_t w = k0 >> 5, b = k0 & 31;
-    const uint32_t lo = run << b;
-    if (lo) atomicOr(dirty + w, lo);
-    if (b + (uint32_t)(xb - xa) >= 32) {
-      const uint32_t hi = run >> (32 - b);
-      if (hi) atomicOr(dirty + w + 1, hi);
+    g = k0 / kOwnGroup;
+    return run << (k0 & (kOwnGroup - 1));
+  }
+  // half 0 raises the run's first group, half 1 its second
+  __device__ __forceinline__ void mark_half(uint32_t *dirty, int lx, int ly, int dy, int half) const {
+    uint32_t g = 0, owner;
+    const uint32_t run = row_run(lx, ly, dy, g);
+    const uint32_t bits = half ? run >> kOwnGroup : run & ((1u << kOwnGroup) - 1u);
+    if (!bits) return;
+    const uint32_t l = by_r.div(g + (uint32_t)half, owner);
+    atomicOr(dirty + owner * wpo + (l >> 3), bits << ((l & 7u) * kOwnGroup));
+  }
+  __device__ __forceinline__ void mark_row(uint32_t *dirty, int lx, int ly, int dy) const {
+    uint32_t g = 0, owner;
+    const uint32_t run = row_run(lx, ly, dy, g);
+    if (!run) return;
+    uint32_t l = by_r.div(g, owner);
+    const uint32_t lo = run & ((1u << kOwnGroup) - 1u), hi = run >> kOwnGroup;
+    if (lo) atomicOr(dirty + owner * wpo + (l >> 3), lo << ((l & 7u) * kOwnGroup));
+    if (hi) {  // the next group: the next CTA's
+      if (++owner == by_r.d) {
+        owner = 0;
+        ++l;
+      }
+      atomicOr(dirty + owner * wpo + (l >> 3), hi << ((l & 7u) * kOwnGroup));
     }
   }
-}
-
-// As mark3x3_bits, and the neighbours outside the tile (inside the grid) into
-// the grid-wide pending bitmap (one reduction per cell: only cells on or
-// beyond the tile's border have such neighbours).  (lx, ly) may lie anywhere
-// in the grid, relative to the tile's corner (x0, y0).
-__device__ __forceinline__ void mark3x3_pending(uint32_t *dirty, uint32_t *pending, const JobDev &j,
-                                                int x0, int y0, int lx, int ly, int TW, int TH) {
-  mark3x3_bits(dirty, lx, ly, TW, TH);
-  if (lx > 0 && ly > 0 && lx < TW - 1 && ly < TH - 1) return;
+  __device__ __forceinline__ void mark3x3(uint32_t *dirty, int lx, int ly) const {
 #pragma unroll
-  for (int t = 0; t < 9; ++t) {
-    const int ax = lx + t % 3 - 1, ay = ly + t / 3 - 1;
-    if (t == 4 || (ax >= 0 && ay >= 0 && ax < TW && ay < TH)) continue;
-    const int gx = x0 + ax, gy = y0 + ay;
-    if (gx < 0 || gy < 0 || gx >= j.W || gy >= j.H) continue;
-    const int64_t g = gx + (int64_t)gy * j.W;
-    atomicOr(pending + (g >> 5), 1u << (g & 31));
+    for (int dy = 0; dy < 3; ++dy) mark_row(dirty, lx, ly, dy);
   }
+};
+
+// Neighbour t (0..8, row-major, 4 the centre) of tile cell (lx, ly) when it
+// lies outside the tile but inside the grid: raises its bit in the grid-wide
+// pending bitmap.  (lx, ly) may lie anywhere in the grid.
+__device__ __forceinline__ void mark_pending(uint32_t *pending, const JobDev &j, int x0, int y0, int lx,
+                                             int ly, int TW, int TH, int t) {
+  const int ax = lx + t % 3 - 1, ay = ly + t / 3 - 1;
+  if (t == 4 || (ax >= 0 && ay >= 0 && ax < TW && ay < TH)) return;
+  const int gx = x0 + ax, gy = y0 + ay;
+  if (gx < 0 || gy < 0 || gx >= j.W || gy >= j.H) return;
+  const int64_t g = gx + (int64_t)gy * j.W;
+  atomicOr(pending + (g >> 5), 1u << (g & 31));
+}
+__device__ __forceinline__ bool tile_border(int lx, int ly, int TW, int TH) {
+  return lx <= 0 || ly <= 0 || lx >= TW - 1 || ly >= TH - 1;
 }
 
 // Takes (reads and clears) the pending bits of tile cells k0 .. k0 + n - 1
-// (n <= 32, tile-linear order) selected by mask (bit i: cell k0 + i) from
-// the grid-wide bitmap; bit i of the result is cell k0 + i.  The cells of one tile row are consecutive grid
-// cells, so each row segment is a funnel shift of two words.
+// (n <= 32, tile-linear order) from the grid-wide bitmap; bit i of the result
+// is cell k0 + i.  The cells of one tile row are consecutive grid cells, so
+// each row segment is a funnel shift of two words.
 __device__ __forceinline__ uint32_t take_pending(uint32_t *pending, const JobDev &j, int x0, int y0,
-                                                 int TW, uint32_t k0, uint32_t n, uint32_t mask) {
+                                                 int TW, uint32_t k0, uint32_t n) {
   uint32_t out = 0, done = 0;
   while (done < n) {
     const uint32_t k = k0 + done;
@@ -617,7 +763,7 @@ __device__ __forceinline__ uint32_t take_pending(uint32_t *pending, const JobDev
     const uint64_t w2 =
         (uint64_t)__ldcg(pending + wi) | (two ? (uint64_t)__ldcg(pending + wi + 1) << 32 : 0ull);
     const uint32_t m = seg >= 32 ? 0xFFFFFFFFu : (1u << seg) - 1u;
-    const uint32_t bits = (uint32_t)(w2 >> sh) & m & (mask >> done);
+    const uint32_t bits = (uint32_t)(w2 >> sh) & m;
     if (bits) {
       const uint64_t cm = (uint64_t)bits << sh;
       if ((uint32_t)cm) atomicAnd(pending + wi, ~(uint32_t)cm);
@@ -646,54 +792,240 @@ struct SweepCtx {
   }
 };
 
-// Ownership of a global-memory tile's cells: the tile-linear cells are cut
-// into groups of kOwnGroup consecutive cells, and group g belongs to CTA
-// g mod R of the team, so that the cells of a front spread over the CTAs
-// while a CTA's cells still come in short runs (its neighbour reads share
-// L1 lines).  Tile word w (cells 32 w .. 32 w + 31) holds kGroupsPerWord
-// groups; CTA `rank` owns those at offsets first, first + R, ... of the word.
-// Groups of 4 cells measured fastest on the 4096^2 scenario with 148 CTAs
-// (769 ms; 1 cell: 787 ms; whole 32-cell words dealt round-robin, with
-// the scan of every word: slower still).
-constexpr uint32_t kOwnGroup = 4;  // a power of two, at most 32
-constexpr uint32_t kGroupsPerWord = 32u / kOwnGroup;
-__device__ __forceinline__ uint32_t owned_first(uint32_t w, uint32_t rank, uint32_t R) {
-  return (rank + R - (w * kGroupsPerWord) % R) % R;  // offset of the first owned group of word w
+__device__ __forceinline__ CellState ld_state(const CellState *p) {
+  const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(p));
+  return CellState{__uint_as_float(v.x), v.y, v.z, v.w};
 }
-__device__ __forceinline__ uint32_t owned_mask(uint32_t first, uint32_t R) {
-  constexpr uint32_t g = kOwnGroup == 32u ? 0xFFFFFFFFu : (1u << kOwnGroup) - 1u;
-  uint32_t m = 0;
-  for (uint32_t i = first; i < kGroupsPerWord; i += R) m |= g << (i * kOwnGroup);
-  return m;
+__device__ __forceinline__ void st_state(CellState *p, const CellState &s) {
+  *reinterpret_cast<uint4 *>(p) = make_uint4(__float_as_uint(s.time), s.ref, s.los, s.pad);
 }
-// Owned cells of one word at most: kOwnGroup per owned group.
-__host__ __device__ inline uint32_t owned_per_word(uint32_t R) {
-  return kOwnGroup * ((kGroupsPerWord + R - 1) / R);
-}
-constexpr int kScanBatch = 8;  // dirty words a thread loads at once
 
 // A global-memory tile's update entries of one sweep: this CTA's first
 // kTileUpdSmem in shared memory, the rest in its global update region.
-__device__ __forceinline__ TileUpdate get_update(const TileUpdate *sm_upd, const TileUpdate *g_upd,
-                                                 uint32_t u) {
-  if (u < (uint32_t)kTileUpdSmem) return sm_upd[u];
-  const uint4 *q = reinterpret_cast<const uint4 *>(g_upd + u);
-  const uint4 a = __ldcg(q), b = __ldcg(q + 1);
-  return TileUpdate{a.x, __uint_as_float(a.y), a.z, a.w, b.x, b.y, 0u, 0u};
+__device__ __forceinline__ CellState get_update(const TileUpdate *sm_upd, const TileUpdate *g_upd,
+                                                uint32_t u) {
+  return u < (uint32_t)kTileUpdSmem ? sm_upd[u] : ld_state(g_upd + u);
+}
+
+// find_neighbor_which_reaches_first (propag.cu:124-190) by the eight lanes of
+// a cell, as evaluate_coop, on packed records: the neighbour's line of sight
+// to its reference is read with its state instead of walked.  All arithmetic
+// but the last sum of the candidate's time is independent of the reference's
+// time, and runs while that load is in flight.  own: the cell's state; the
+// result is the lanes' common view (best.time < own.time: improved).
+__device__ __forceinline__ Best evaluate_packed(const JobDev &j, const DirConst &dc,
+                                                const CellState *__restrict__ X, int x, int y, Best own,
+                                                bool valid, uint32_t lane, Counters &cnt) {
+  const float kInf = __int_as_float(0x7f800000);
+  const int k = (int)(lane & 7u);
+  const int kk = k < 4 ? k : k + 1;
+  const int nx = x + kk % 3 - 1, ny = y + kk / 3 - 1;
+  const bool refm = j.refm != 0;
+  CellState n{FLT_MAX, kNoRef, 0u, 0u};
+  Fire f{0.0f, 0.0f, 0.0f};
+  if (valid && nx >= 0 && ny >= 0 && nx < j.W && ny < j.H) {
+    const int64_t c = nx + (int64_t)ny * j.W;
+    n = ld_state(X + c);
+    const float4 v = __ldg(j.fire4 + c);
+    f = Fire{v.x, v.y, v.z};
+  }
+  const int rx = ref_x(n.ref), ry = ref_y(n.ref);
+  const bool act = n.time < j.max_time && f.speed_max != 0.0f && !(rx == x && ry == y);
+  float rt = FLT_MAX;
+  if (act) rt = __ldcg(&X[rx + (int64_t)ry * j.W].time);
+  cnt.gat += act ? 1u : 0u;
+  float offer = kInf, cand = kInf;
+  uint32_t oref = 0;
+  bool walked = false;
+  if (act) {
+    offer = step_time(n.time, dc.dist[k], dir_inv_speed(dc, k, f, refm), refm);
+    oref = pack_ref(nx, ny);
+    const float inv = inv_speed(bearing(rx, ry, x, y, j.north_up != 0, refm), f, refm);
+    const float dist = cell_distance(rx - x, ry - y, j.gdx, j.gdy, refm);
+    cand = step_time(rt, dist, inv, refm);
+    if (cand < offer) {
+      walked = cand < own.time;
+      if (!(walked && (n.los & kLosBlocked))) {
+        offer = cand;
+        oref = n.ref;
+      }
+    }
+  }
+  // running best of the sequential loop before neighbour k (exclusive min),
+  // and the first minimum of the offers
+  float pm = offer, bv = offer;
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
+    const float t = __shfl_up_sync(kFull, pm, o);
+    const float ov = __shfl_xor_sync(kFull, bv, o);
+    if (k >= o && t < pm) pm = t;
+    if (ov < bv) bv = ov;
+  }
+  float before = __shfl_up_sync(kFull, pm, 1);
+  if (k == 0) before = kInf;
+  if (walked && cand < before) {
+    const uint32_t steps = n.los & ~kLosBlocked;
+    cnt.dda += steps;
+    cnt.walk_max = max(cnt.walk_max, steps);
+  }
+  const uint32_t g0 = lane & 24u;
+  bv = __shfl_sync(kFull, bv, g0);
+  const uint32_t at = (__ballot_sync(kFull, offer == bv) >> g0) & 0xFFu;
+  const uint32_t br = __shfl_sync(kFull, oref, g0 + (at ? (uint32_t)__ffs(at) - 1u : 0u));
+  return bv < own.time ? Best{bv, br} : own;
+}
+
+// The line of sight from cell (fx, fy) to (tx, ty) (line_blocked's walk, same
+// cells, same count) by the eight lanes of a cell; the result is a CellState's
+// los.  Called by all 32 lanes; `on` is uniform in each group of eight.
+//
+// Step by step, for offsets beyond kColumnsMax: every lane generates the walk,
+// lane i of the eight looks up the visited cells i, i + 8, ... of each run of
+// kCoopSteps, whose bitmap words are thus loaded together.  In remaining
+// counts (ri, rj) the walk's end conditions are signs: the target is the only
+// cell with both zero, and every step from it leaves the walk's box.
+constexpr int kCoopSteps = 16;
+__device__ __noinline__ uint32_t walk_los_steps(const uint32_t *__restrict__ bnd, int W, int fx, int fy,
+                                                int tx, int ty, bool on, uint32_t lane) {
+  const int sx = (tx > fx) - (tx < fx), sy = (ty > fy) - (ty < fy);
+  const int adx = abs(tx - fx), ady = abs(ty - fy);
+  int ri = on ? adx : -1, rj = ady;
+  // 1 / |d|: the float nearest to the reference's double quotient (a quotient
+  // of integers below 2^16 lies too far from a midpoint of floats to round
+  // differently in one step or two)
+  const float ddx = __frcp_rn((float)adx), ddy = __frcp_rn((float)ady);
+  float tmx = ddx, tmy = ddy;
+  const float kTie = __int_as_float(0x3089705F);  // the largest float below 1e-9
+  uint32_t cur = (uint32_t)fx + (uint32_t)fy * (uint32_t)W;  // grids below 2^32 cells
+  const uint32_t stepx = (uint32_t)sx, stepy = (uint32_t)(sy * W);
+  const uint32_t k = lane & 7u, g0 = lane & 24u;
+  uint32_t steps = 0, los = 0;
+  while (__any_sync(kFull, (ri | rj) >= 0)) {
+    uint32_t ix[kCoopSteps / 8];
+    uint32_t mine = 0, nv = 0;  // my visited cells (bit per eight), cells visited in this run
+#pragma unroll
+    for (int i = 0; i < kCoopSteps; ++i) {
+      const bool live = (ri | rj) >= 0;
+      if (live) ++nv;
+      if (live && k == (uint32_t)(i & 7)) {
+        ix[i >> 3] = cur;
+        mine |= 1u << (i >> 3);
+      }
+      const float t = __fsub_rn(tmx, tmy);
+      if (t <= kTie) {  // x first, or a tie (a diagonal step)
+        tmx = __fadd_rn(tmx, ddx);
+        cur += stepx;
+        --ri;
+      }
+      if (t >= -kTie) {
+        tmy = __fadd_rn(tmy, ddy);
+        cur += stepy;
+        --rj;
+      }
+    }
+    uint32_t w[kCoopSteps / 8];
+#pragma unroll
+    for (int b = 0; b < kCoopSteps / 8; ++b) w[b] = (mine >> b) & 1u ? __ldg(bnd + (ix[b] >> 5)) : 0u;
+#pragma unroll
+    for (int b = 0; b < kCoopSteps / 8; ++b) {
+      const bool hit = ((mine >> b) & 1u) && ((w[b] >> (ix[b] & 31u)) & 1u);
+      const uint32_t m = (__ballot_sync(kFull, hit) >> g0) & 0xFFu;
+      if (m && !los) los = kLosBlocked | (steps + (uint32_t)b * 8u + (uint32_t)__ffs(m));
+    }
+    steps += nv;
+    if (los) ri = -1;
+    // a walk from a cell to itself visits it twice (no step leaves it)
+    if (adx + ady == 0 && ri >= 0) {
+      steps = 2;
+      ri = -1;
+    }
+  }
+  return los ? los : steps;
+}
+
+// In closed form (dda_columns.cuh), lane i of the eight taking columns i, i +
+// 8, ..., four at a time (kColumnRun columns a group): all bitmap words of a
+// run are loaded together, and no step waits for the one before.
+constexpr int kColumnRun = 32;
+__device__ __forceinline__ uint32_t walk_los(const uint32_t *__restrict__ bnd, const float *cross, int W,
+                                             int fx, int fy, int tx, int ty, bool on, uint32_t lane) {
+  const int dx = tx - fx, dy = ty - fy;
+  const int adx = abs(dx), ady = abs(dy);
+  const int P = max(adx, ady), Q = min(adx, ady);
+  if (__any_sync(kFull, on && (P > kColumnsMax || P == 0)))
+    return walk_los_steps(bnd, W, fx, fy, tx, ty, on, lane);
+  const int sx = dx < 0 ? -1 : 1, sy = dy < 0 ? -W : W;
+  const int step_p = adx >= ady ? sx : sy, step_q = adx >= ady ? sy : sx;
+  const uint32_t start = (uint32_t)fx + (uint32_t)fy * (uint32_t)W;  // grids below 2^32 cells
+  const float inv_p = __frcp_rn((float)P);
+  const uint32_t k = lane & 7u, g0 = lane & 24u;
+  const int last = on ? P : -1;
+  uint32_t D = 0, los = 0;  // diagonal steps so far; the result once blocked
+  for (int c0 = 0; __any_sync(kFull, c0 <= last && !los); c0 += kColumnRun) {
+    uint32_t hit_in = 0, hit_out = 0, diags = 0;  // bit b: column c0 + 8 b + k
+    uint32_t ia[4], wa[4], wb[4];
+    int two[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const int c = c0 + 8 * b + (int)k;
+      wa[b] = wb[b] = 0u;
+      ia[b] = 0u;
+      two[b] = 0;
+      if (c <= last) {
+        int jin, jout;
+        bool diag;
+        walk_column(cross, P, Q, c, inv_p, jin, jout, diag);
+        ia[b] = start + (uint32_t)(c * step_p) + (uint32_t)(jin * step_q);
+        two[b] = jout - jin ? step_q : 0;
+        if (diag) diags |= 1u << b;
+        wa[b] = __ldg(bnd + (ia[b] >> 5));
+        wb[b] = __ldg(bnd + ((ia[b] + (uint32_t)two[b]) >> 5));
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      hit_in |= ((wa[b] >> (ia[b] & 31u)) & 1u) << b;
+      hit_out |= ((wb[b] >> ((ia[b] + (uint32_t)two[b]) & 31u)) & 1u) << b;
+    }
+    const bool hit = (hit_in | hit_out) != 0u;
+    if (__any_sync(kFull, hit)) {
+      // the first boundary's column in this run, from the lanes' masks
+      uint32_t first = 0xFFFFu;
+      if (hit) first = 8u * (uint32_t)(__ffs(hit_in | hit_out) - 1) + k;
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) first = min(first, __shfl_xor_sync(kFull, first, o));
+      uint32_t before = 0;  // diagonal steps up to and including that column
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const uint32_t m = (__ballot_sync(kFull, (diags >> b) & 1u) >> g0) & 0xFFu;
+        const int upto = (int)first - 8 * b;  // bits 0 .. upto count
+        before += (uint32_t)__popc(upto >= 7 ? m : upto >= 0 ? m & ((2u << upto) - 1u) : 0u);
+      }
+      const uint32_t in_hits = __shfl_sync(kFull, hit_in, g0 + (first & 7u));
+      if (first != 0xFFFFu && !los) {
+        int jin, jout;
+        bool diag;
+        walk_column(cross, P, Q, c0 + (int)first, inv_p, jin, jout, diag);
+        const int r = (in_hits >> (first >> 3)) & 1u ? jin : jout;
+        los = kLosBlocked | (uint32_t)(c0 + (int)first + r + 1 - (int)(D + before));
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < 4; ++b) D += (uint32_t)__popc((__ballot_sync(kFull, (diags >> b) & 1u) >> g0) & 0xFFu);
+  }
+  return los ? los : (uint32_t)(P + Q + 1) - D;
 }
 
 // One tile launch with the state in global memory, by a team of R CTAs
-// (this one is `rank`).  `list` is shared memory for blockDim.x * 32 u16
-// entries, `sm_upd` for two sweeps' kTileUpdSmem update entries, `cta_ctr`
-// two shared counters.  Returns whether any sweep improved a cell.
+// (this one is `rank`).  `list` is shared memory for blockDim.x * 32 entries,
+// `sm_upd` for two sweeps' kTileUpdSmem update entries, `cta_ctr` five shared
+// counters, `queue` kScanQueue boxes, `cross` the crossing times of the line-of-sight walks.  Returns
+// whether any sweep improved a cell.
 //
-// An update entry carries what the commit needs besides the new time and
-// reference: whether the cell burns (its neighbours read it) and its
-// referrer box, both read while the cell is evaluated, so that the commit
-// makes no dependent global reads.  The box read then (before or during
-// other CTAs' commits of the sweep) holds every referrer adopted in earlier
-// sweeps (their growth happened before the last barrier); referrers that
-// adopt the cell in this sweep improved, and mark their neighbourhoods
+// The referrer box a commit scans is read while the cell is evaluated (before
+// or during other commits of the sweep): it holds every referrer adopted in
+// earlier sweeps (their growth happened before the last barrier); referrers
+// that adopt the cell in this sweep improved, and mark their neighbourhoods
 // themselves.  Concurrent growth can only widen the box (a box created in
 // this sweep may show the empty marker in a corner: corners are clamped to
 // the grid), which costs scan work, never a mark: a scan hits the cells that
@@ -702,208 +1034,187 @@ __device__ __forceinline__ TileUpdate get_update(const TileUpdate *sm_upd, const
 // writes only its tile's cells, and both copies agree everywhere when a
 // launch ends, so outside the tile X[0] and X[1] hold the same state.
 __device__ bool tile_global(const JobDev &j, const DirConst &dc, const SlotDev &s, const TileDesc &td,
-                            ScanBox *scan_boxes, uint32_t *list, TileUpdate *sm_upd, uint32_t *cta_ctr,
+                            uint32_t *list, TileUpdate *sm_upd, uint32_t *cta_ctr, ScanItem *queue, const float *cross,
                             uint32_t rank, uint32_t R, SweepCtx &cx, Team &team) {
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const uint32_t k8 = lane & 7u, g0 = lane & 24u;
   const int x0 = td.x0, y0 = td.y0, TW = td.TW, TH = td.TH;
   const uint32_t TN = (uint32_t)TW * (uint32_t)TH;
-  const uint32_t nwords = (TN + 31) / 32;
-  // a chunk of words yields at most the list's capacity of owned cells: the
-  // whole tile when this CTA's share fits, else a bounded run of words
+  const TileBits tb(TW, TH, R);
+  const uint32_t ngroups = (TN + kOwnGroup - 1) / kOwnGroup;
   const uint32_t cap = global_tile_upd_cap(TN, R);
-  const uint32_t chunk_words = cap <= global_tile_list_cap(blockDim.x)
-                                   ? nwords
-                                   : global_tile_list_cap(blockDim.x) / owned_per_word(R);
-  float *const tm[2] = {j.time, j.time1};
-  uint32_t *const rf[2] = {j.refs, j.refs1};
+  // the work list holds a chunk of words at a time: usually all of them
+  const uint32_t chunk = global_tile_list_cap(blockDim.x) / 32u;
+  const CellState *const X[2] = {j.st0, j.st1};
   // the launch's counters in registers (the context may live in local memory)
   Counters cnt = cx.cnt;
   bool first = true, worked = false;
-  uint32_t prev_upd = 0;  // this CTA's improvements of the previous sweep
-  int p = 0;              // sweep parity: read X[p], write X[p ^ 1]
+  uint32_t q = 0;  // list counter of this chunk: cta_ctr[q]
+  int p = 0;       // sweep parity: read X[p], write X[p ^ 1]
+  if (threadIdx.x < 1)
+    for (int i = 0; i < 5; ++i) cta_ctr[i] = 0u;
+  __syncthreads();
   for (;;) {
     ++cx.sweeps;  // every thread counts, so the abort below is uniform
-    const float *const rt = tm[p];
-    const uint32_t *const rr = rf[p];
-    float *const wt = tm[p ^ 1];
-    uint32_t *const wr = rf[p ^ 1];
-    // dirty bitmaps in rotation by the team's sweep count d: read D[d % 3],
-    // mark D[(d + 1) % 3], clear D[(d + 2) % 3] (read in sweep d - 1)
+    const CellState *const rs = X[p];
+    CellState *const ws = const_cast<CellState *>(X[p ^ 1]);
+    // dirty bitmaps by the team's sweep count d: read and clear D[d & 1], mark
+    // D[(d + 1) & 1] (cleared by its readers in sweep d - 1)
     const uint32_t dsw = team.dsweep++;
-    uint32_t *const dirty = s.dirty + (size_t)(dsw % 3) * s.dirty_words;
-    uint32_t *const dirty_next = s.dirty + (size_t)((dsw + 1) % 3) * s.dirty_words;
-    uint32_t *const dirty_old = s.dirty + (size_t)((dsw + 2) % 3) * s.dirty_words;
+    uint32_t *const dirty = s.dirty + (size_t)(dsw & 1u) * s.dirty_words + (size_t)rank * tb.wpo;
+    uint32_t *const dirty_next = s.dirty + (size_t)((dsw + 1u) & 1u) * s.dirty_words;
     TileUpdate *const upd = s.upd + ((size_t)p * R + rank) * cap;
-    const TileUpdate *const upd_prev = s.upd + ((size_t)(p ^ 1) * R + rank) * cap;
     TileUpdate *const supd = sm_upd + p * kTileUpdSmem;
-    const TileUpdate *const supd_prev = sm_upd + (p ^ 1) * kTileUpdSmem;
-    // ---- 1, 2: compact and evaluate (nothing is written to X[p]) ----
-    // the bitmap read two sweeps ago is cleared now (its marks come in the
-    // next sweep): the words w = rank mod R of the slot's bitmap
-    for (uint32_t w = rank + threadIdx.x * R; w < s.dirty_words; w += blockDim.x * R) dirty_old[w] = 0u;
-    if (threadIdx.x == 0) cta_ctr[1] = 0;
-    for (uint32_t c0 = 0; c0 < nwords; c0 += chunk_words) {
-      __syncthreads();  // the previous chunk's list is consumed
-      if (threadIdx.x == 0) cta_ctr[0] = 0;
-      __syncthreads();
-      const uint32_t c1 = min(nwords, c0 + chunk_words);
-      // this thread's words w = c0 + threadIdx.x + i blockDim.x, in batches of
-      // kScanBatch whose loads all go out before any is used; the offset of
-      // the first owned group of word w steps by a constant from one word to
-      // the next of the thread
-      uint32_t fo = owned_first(c0 + threadIdx.x, rank, R);
-      const uint32_t fstep = (R - (kGroupsPerWord * blockDim.x) % R) % R;
-      for (uint32_t wb = c0 + threadIdx.x; wb < c1; wb += kScanBatch * blockDim.x) {
-        uint32_t v[kScanBatch];
-#pragma unroll
-        for (int i = 0; i < kScanBatch; ++i) {
-          const uint32_t w = wb + (uint32_t)i * blockDim.x;
-          v[i] = 0u;
-          if (w < c1) {
-            if (!first) {
-              v[i] = __ldcg(dirty + w);
-            } else if (!j.pending) {  // the whole tile
-              const uint32_t nb = (w == nwords - 1 && (TN & 31)) ? (TN & 31) : 32u;
-              v[i] = nb == 32 ? 0xFFFFFFFFu : (1u << nb) - 1u;
-            }
+    uint32_t *const upd_ctr = cta_ctr + 2 + p;
+    const uint32_t prev_upd = cta_ctr[2 + (p ^ 1)];  // this CTA's improvements of the previous sweep
+    // the neighbours of a referrer
+    auto mark_around = [&](int xx, int yy) {
+      tb.mark3x3(dirty_next, xx - x0, yy - y0);
+      if (j.pending && tile_border(xx - x0, yy - y0, TW, TH))
+        for (int t = 0; t < 9; ++t) mark_pending(j.pending, j, x0, y0, xx - x0, yy - y0, TW, TH, t);
+    };
+    for (uint32_t c0 = 0; c0 < tb.wpo; c0 += chunk) {
+      if (c0) __syncthreads();  // the previous chunk's list is consumed
+      const uint32_t c1 = min(tb.wpo, c0 + chunk);
+      // ---- 1: this CTA's marked cells into the list ----
+      if (!first) {
+        // a thread per group: short runs of bits, over as many lanes as there are
+        for (uint32_t l = c0 * 8u + threadIdx.x; l < c1 * 8u; l += blockDim.x) {
+          const uint32_t v = __ldcg(dirty + (l >> 3));
+          uint32_t bits = (v >> ((l & 7u) * kOwnGroup)) & ((1u << kOwnGroup) - 1u);
+          if (bits) {
+            uint32_t at = atomicAdd(cta_ctr + q, (uint32_t)__popc(bits));
+            const uint32_t k0 = (l * R + rank) * kOwnGroup;
+            for (; bits; bits &= bits - 1) list[at++] = k0 + (uint32_t)(__ffs(bits) - 1);
           }
         }
-#pragma unroll
-        for (int i = 0; i < kScanBatch; ++i) {
-          const uint32_t w = wb + (uint32_t)i * blockDim.x;
-          const uint32_t own = owned_mask(fo, R);
-          fo += fstep;
-          if (fo >= R) fo -= R;
-          if (w >= c1) continue;
-          uint32_t bits = v[i] & own;
-          if (first && j.pending) {
-            // the cells whose inputs changed since their last evaluation
-            const uint32_t nb = (w == nwords - 1 && (TN & 31)) ? (TN & 31) : 32u;
-            bits = take_pending(j.pending, j, x0, y0, TW, w * 32, nb, own);
-          }
+      } else {
+        // the tile's pending cells (inputs changed since their last
+        // evaluation), or every cell
+        for (uint32_t l = c0 * 8u + threadIdx.x; l < c1 * 8u; l += blockDim.x) {
+          const uint32_t g = l * R + rank;
+          if (g >= ngroups) break;
+          const uint32_t n = min(kOwnGroup, TN - g * kOwnGroup);
+          uint32_t bits = j.pending ? take_pending(j.pending, j, x0, y0, TW, g * kOwnGroup, n) : (1u << n) - 1u;
           if (bits) {
-            uint32_t at = atomicAdd(cta_ctr + 0, (uint32_t)__popc(bits));
-            for (; bits; bits &= bits - 1) list[at++] = w * 32 + (uint32_t)(__ffs(bits) - 1);
+            uint32_t at = atomicAdd(cta_ctr + q, (uint32_t)__popc(bits));
+            for (; bits; bits &= bits - 1) list[at++] = g * kOwnGroup + (uint32_t)(__ffs(bits) - 1);
           }
         }
       }
+      // the previous sweep's improvements into X[p ^ 1], before this sweep's
+      // improvements of the same cells (ordered by the barrier below)
+      if (c0 == 0)
+        for (uint32_t u = threadIdx.x; u < prev_upd; u += blockDim.x) {
+          CellState e = get_update(sm_upd + (p ^ 1) * kTileUpdSmem, s.upd + ((size_t)(p ^ 1) * R + rank) * cap, u);
+          uint32_t col;
+          const uint32_t row = tb.by_tw.div(e.pad, col);
+          st_state(ws + (x0 + (int)col) + (int64_t)(y0 + (int)row) * j.W, e);
+        }
       __syncthreads();
-      const uint32_t nlist = cta_ctr[0];
-      if (threadIdx.x == 0) cnt.evals += nlist;
-      // four cells per warp, eight lanes per cell
-      for (uint32_t base = warp * 4; base < nlist; base += nwarps * 4) {
+      for (uint32_t w = c0 + threadIdx.x; w < c1; w += blockDim.x) dirty[w] = 0u;  // marked again in the next sweep at the earliest
+      const uint32_t nlist = cta_ctr[q];
+      q ^= 1u;
+      if (threadIdx.x == 0) {
+        cnt.evals += nlist;
+        cta_ctr[q] = 0u;  // the next chunk's or sweep's counter (read before the last barrier)
+        if (c0 == 0) cta_ctr[2 + (p ^ 1)] = 0u;
+      }
+      // ---- 2: evaluate and commit, up to four cells a warp, spread over the
+      // CTA's warps (a warp's walks and scans take as long as its longest) ----
+      const uint32_t per = min(4u, (nlist + nwarps - 1) / nwarps);
+      for (uint32_t base = warp * per; base < nlist; base += nwarps * per) {
         const uint32_t ci = base + (lane >> 3);
-        const bool valid = ci < nlist;
+        const bool valid = (lane >> 3) < per && ci < nlist;
         uint32_t k = 0;
-        int x = 0, y = 0;
+        int lx = 0, ly = 0, x = 0, y = 0;
+        int64_t c = 0;
         Best own{FLT_MAX, kNoRef};
-        uint32_t bx0 = kEmptyBox, by0 = 0, bx1 = 0, by1 = 0;
+        uint32_t corner = 0;  // lanes 0..3 of the cell: x0, y0, x1, y1 of its referrer box
         float own_speed = 0.0f;
         if (valid) {
           k = list[ci];
-          x = x0 + (int)(k % (uint32_t)TW);
-          y = y0 + (int)(k / (uint32_t)TW);
-          const int64_t c = x + (int64_t)y * j.W;
-          own = Best{__ldcg(rt + c), __ldcg(rr + c)};
-          if ((lane & 7) == 0) {  // what the commit needs if the cell improves
-            own_speed = __ldg(j.speed + c);
-            bx0 = __ldcg(j.box_x0 + c);
-            by0 = __ldcg(j.box_y0 + c);
-            bx1 = __ldcg(j.box_x1 + c);
-            by1 = __ldcg(j.box_y1 + c);
+          uint32_t col;
+          ly = (int)tb.by_tw.div(k, col);
+          lx = (int)col;
+          x = x0 + lx;
+          y = y0 + ly;
+          c = x + (int64_t)y * j.W;
+          const CellState o = ld_state(rs + c);
+          own = Best{o.time, o.ref};
+          if (k8 < 4) {
+            const uint32_t *const b = k8 == 0   ? j.box_x0 + c * j.box_x0_step
+                                      : k8 == 1 ? j.box_y0 + c
+                                      : k8 == 2 ? j.box_x1 + c
+                                                : j.box_y1 + c;
+            corner = __ldcg(b);
           }
+          own_speed = __ldg(&j.fire4[c].x);
         }
-        const Best b = evaluate_coop(j, dc, GlobalAcc{j, rt, rr}, x, y, own, valid, lane, cnt);
-        const bool improved = valid && (lane & 7) == 0 && b.time < own.time;
-        const uint32_t ai = warp_append(cta_ctr + 1, improved ? 1u : 0u, lane);
+        const Best b = evaluate_packed(j, dc, rs, x, y, own, valid, lane, cnt);
+        const bool improved = valid && b.time < own.time;  // common to the cell's lanes
+        if (!__any_sync(kFull, improved)) continue;
+        // referrer box (whole with a pending bitmap: referrers anywhere mark
+        // pending cells; else clipped to the tile grown by one cell)
+        Box box;
+        box.x0 = (int)__shfl_sync(kFull, corner, g0);
+        box.y0 = (int)__shfl_sync(kFull, corner, g0 + 1);
+        box.x1 = (int)__shfl_sync(kFull, corner, g0 + 2);
+        box.y1 = (int)__shfl_sync(kFull, corner, g0 + 3);
+        if (!improved || (uint32_t)box.x0 == kEmptyBox)
+          box = Box{1, 1, 0, 0};
+        else if (j.pending)
+          box = Box{max(box.x0, 0), max(box.y0, 0), min(box.x1, j.W - 1), min(box.y1, j.H - 1)};
+        else
+          box = clip_box(box.x0, box.y0, box.x1, box.y1, x0, y0, TW, TH, j.W, j.H);
+        const uint32_t los = walk_los(j.bnd, cross, j.W, x, y, ref_x(b.ref), ref_y(b.ref), improved, lane);
+        const uint32_t adds = __ballot_sync(kFull, improved && k8 == 0);
+        uint32_t ai = 0;
+        if (lane == 0) ai = atomicAdd(upd_ctr, (uint32_t)__popc(adds));
+        ai = __shfl_sync(kFull, ai, 0) + (uint32_t)__popc(adds & ((1u << lane) - 1u));
         if (improved) {
-          Box box{1, 1, 0, 0};
-          if (bx0 != kEmptyBox) {
-            if (j.pending)  // the whole box: referrers anywhere mark pending cells
-              box = Box{max((int)bx0, 0), max((int)by0, 0), min((int)bx1, j.W - 1), min((int)by1, j.H - 1)};
+          if (k8 == 0) {
+            st_state(ws + c, CellState{b.time, b.ref, los, 0u});
+            const CellState e{b.time, b.ref, los, k};
+            if (ai < (uint32_t)kTileUpdSmem)
+              supd[ai] = e;
             else
-              box = clip_box((int)bx0, (int)by0, (int)bx1, (int)by1, x0, y0, TW, TH, j.W, j.H);
+              st_state(upd + ai, e);
           }
-          // corners in 16 bits (grids up to 65534 cells a side); an empty box
-          // as x0 = 0xFFFF > x1
-          const bool empty = box.x0 > box.x1 || box.y0 > box.y1;
-          const uint32_t b01 = empty ? 0xFFFFu : (uint32_t)box.x0 | ((uint32_t)box.y0 << 16);
-          const uint32_t b23 = empty ? 0u : (uint32_t)box.x1 | ((uint32_t)box.y1 << 16);
+          // the reference's box grows to hold (x, y), a corner a lane
+          const int64_t rc = ref_x(b.ref) + (int64_t)ref_y(b.ref) * j.W;
+          if (k8 == 0) atomicMin(j.box_x0 + rc * j.box_x0_step, (uint32_t)x);
+          if (k8 == 1) atomicMin(j.box_y0 + rc, (uint32_t)y);
+          if (k8 == 2) atomicMax(j.box_x1 + rc, (uint32_t)x);
+          if (k8 == 3) atomicMax(j.box_y1 + rc, (uint32_t)y);
           // only a burning cell is read by its neighbours
-          const uint32_t burn = b.time < j.max_time && own_speed != 0.0f ? 1u : 0u;
-          if (ai < (uint32_t)kTileUpdSmem) {
-            supd[ai] = TileUpdate{k, b.time, b.ref, burn, b01, b23, 0u, 0u};
-          } else {
-            uint4 *q = reinterpret_cast<uint4 *>(upd + ai);
-            q[0] = make_uint4(k, __float_as_uint(b.time), b.ref, burn);
-            q[1] = make_uint4(b01, b23, 0u, 0u);
+          if (b.time < j.max_time && own_speed != 0.0f) {
+            if (k8 < 6) tb.mark_half(dirty_next, lx, ly, (int)(k8 >> 1), (int)(k8 & 1u));
+            if (j.pending && tile_border(lx, ly, TW, TH))
+              mark_pending(j.pending, j, x0, y0, lx, ly, TW, TH, (int)(k8 < 4 ? k8 : k8 + 1));
           }
         }
+        warp_scan_boxes4(box, pack_ref(x, y), j, rs, lane, cnt, queue, cta_ctr + 4, mark_around);
       }
     }
-    __syncthreads();
-    const uint32_t my_upd = cta_ctr[1];
-    // ---- 3a: the previous sweep's improvements into X[p ^ 1] ----
-    for (uint32_t u = threadIdx.x; u < prev_upd; u += blockDim.x) {
-      const TileUpdate e = get_update(supd_prev, upd_prev, u);
-      const int64_t c = (x0 + (int)(e.k % (uint32_t)TW)) + (int64_t)(y0 + (int)(e.k / (uint32_t)TW)) * j.W;
-      wt[c] = e.time;
-      wr[c] = e.ref;
+    __syncthreads();  // the queue is complete
+    const uint32_t queued = min(cta_ctr[4], kScanQueue);
+    if (queued) {
+      cta_scan_boxes(queue, queued, j, rs, mark_around);
+      __syncthreads();
+      if (threadIdx.x == 0) cta_ctr[4] = 0u;
     }
-    __syncthreads();  // this sweep's improvements of the same cells land after
-    // ---- 3b: commit (update_point / commit_point), mark, referrer scans.
-    // Updates are dealt `per` to a warp, as few as spreads them over the
-    // CTA's warps (a warp's referrer scans run one after another).
-    const uint32_t per = min(32u, (my_upd + nwarps - 1) / nwarps);
-    for (uint32_t base = warp * per; base < my_upd; base += nwarps * per) {
-      const uint32_t u = base + lane;
-      const bool valid = lane < per && u < my_upd;
-      uint32_t want = 0;
-      Box box{1, 1, 0, 0};
-      if (valid) {
-        const TileUpdate e = get_update(supd, upd, u);
-        const int lx = (int)(e.k % (uint32_t)TW), ly = (int)(e.k / (uint32_t)TW);
-        const int x = x0 + lx, y = y0 + ly;
-        const int64_t c = x + (int64_t)y * j.W;
-        wt[c] = e.time;
-        wr[c] = e.ref;
-        box_expand_global(j, e.ref, x, y);
-        if (e.burn) {
-          if (j.pending)
-            mark3x3_pending(dirty_next, j.pending, j, x0, y0, lx, ly, TW, TH);
-          else
-            mark3x3_bits(dirty_next, lx, ly, TW, TH);
-        }
-        want = pack_ref(x, y);
-        if ((e.b01 & 0xFFFFu) != 0xFFFFu)
-          box = Box{(int)(e.b01 & 0xFFFFu), (int)(e.b01 >> 16), (int)(e.b23 & 0xFFFFu), (int)(e.b23 >> 16)};
-      }
-      warp_scan_boxes(
-          scan_boxes + (threadIdx.x & ~31u), box, want, j, lane, cnt,
-          [&](int xx, int yy, float &t) {
-            const int64_t n = xx + (int64_t)yy * j.W;
-            t = __ldcg(rt + n);
-            return __ldcg(rr + n);
-          },
-          [&](bool hit, int xx, int yy) {
-            if (!hit) return;
-            if (j.pending)
-              mark3x3_pending(dirty_next, j.pending, j, x0, y0, xx - x0, yy - y0, TW, TH);
-            else
-              mark3x3_bits(dirty_next, xx - x0, yy - y0, TW, TH);
-          });
-    }
-    // ---- 4: meet; the barrier reports how many CTAs improved a cell ----
+    // ---- 3: meet; the barrier reports how many CTAs improved a cell ----
     uint32_t improving = 0;
-    if (!team.sync(true, my_upd > 0, &improving)) {
+    const bool met = team.sync(true, upd_ctr, &improving);
+    cx.tick(first ? 0 : 1);
+    if (!met) {
       cx.failed = cx.abort = true;
       break;
     }
-    cx.tick(first ? 0 : 1);
-    if (threadIdx.x == 0) cx.improvements += my_upd;  // summed over the team at the job's end
+    if (threadIdx.x == 0) cx.improvements += *upd_ctr;  // summed over the team at the job's end
     if (improving == 0) break;  // X[p ^ 1] got the last improvements: both copies agree
     worked = true;
-    prev_upd = my_upd;
     p ^= 1;
     first = false;
     if (cx.sweeps > cx.max_sweeps) {
@@ -911,6 +1222,9 @@ __device__ bool tile_global(const JobDev &j, const DirConst &dc, const SlotDev &
       break;
     }
   }
+  // an abandoned launch leaves marks behind: the slot's next tile starts clean
+  if (cx.abort)
+    for (uint32_t w = rank * blockDim.x + threadIdx.x; w < 2u * s.dirty_words; w += R * blockDim.x) s.dirty[w] = 0u;
   cx.cnt = cnt;
   return worked;
 }
@@ -1378,13 +1692,15 @@ __global__ void __launch_bounds__(kEngineThreads, 1) engine_kernel(const JobDev 
   const uint32_t lane = threadIdx.x & 31;
   __shared__ DirConst dc;
   __shared__ JobDev js;
-  __shared__ ScanBox scan_boxes[kEngineThreads];
+  __shared__ ScanBox scan_boxes[kEngineThreads];  // or the scan queue of global-memory tiles
+  static_assert(sizeof(ScanItem) * kScanQueue <= sizeof(ScanBox) * kEngineThreads, "the scan queue fits");
   __shared__ int team_ok[2];
-  __shared__ uint32_t cta_ctr[2];  // global-memory tiles: work list and update counts
+  __shared__ uint32_t cta_ctr[5];  // global-memory tiles: work-list and update counts (two each), scan queue
   Team team{grouped ? reinterpret_cast<unsigned long long *>(s.ctr + 8) : nullptr, queue + 1,
             team_ok, csize};
   team.cnt3 = s.ctr + 5;  // cluster mode: slot counters 5..7
   team.cnt_leader = rank == 0;
+  float *const cross = reinterpret_cast<float *>(dyn_smem + global_tile_cross_off(blockDim.x));
   uint32_t taken = 0xFFFFFFFFu;  // tid 0: the queue position it took last
 
   for (;;) {
@@ -1405,6 +1721,14 @@ __global__ void __launch_bounds__(kEngineThreads, 1) engine_kernel(const JobDev 
     }
     __syncthreads();
     const JobDev &j = js;  // shared-memory copy: frees registers
+    // accumulated crossing times of the line-of-sight walks (a shared-memory
+    // tile of another job may have used the space since the last time)
+    if (j.smem_tile == kSmemTileGlobal)
+      for (int n = 1 + (int)threadIdx.x; n <= kColumnsMax; n += blockDim.x) {
+        const float step = __frcp_rn((float)n);
+        float t = step;
+        for (int i = 1; i <= n; ++i, t = __fadd_rn(t, step)) cross[cross_at(n, i)] = t;
+      }
     StatsDev *st = stats + jid;
     if (tid == 0) st->t_start_ns = globaltimer_ns();
     SweepCtx cx;
@@ -1426,11 +1750,10 @@ __global__ void __launch_bounds__(kEngineThreads, 1) engine_kernel(const JobDev 
                            ? tile_smem<BoxExact>(j, dc, dyn_smem, s, td, scan_boxes, cx, team)
                        : j.smem_tile == kSmemTileCoarse
                            ? tile_smem<BoxCoarse>(j, dc, dyn_smem, s, td, scan_boxes, cx, team)
-                           : tile_global(j, dc, s, td, scan_boxes,
-                                         reinterpret_cast<uint32_t *>(dyn_smem),
+                           : tile_global(j, dc, s, td, reinterpret_cast<uint32_t *>(dyn_smem),
                                          reinterpret_cast<TileUpdate *>(
                                              dyn_smem + global_tile_list_bytes(blockDim.x)),
-                                         cta_ctr, rank, csize, cx, team);
+                                         cta_ctr, reinterpret_cast<ScanItem *>(scan_boxes), cross, rank, csize, cx, team);
         round_worked |= w;
       }
       if (!round_worked || cx.abort) break;
@@ -1490,11 +1813,19 @@ __global__ void __launch_bounds__(256) post_kernel(const JobDev *__restrict__ jo
   unsigned long long burned = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N;
        i += (int64_t)gridDim.x * blockDim.x) {
-    float t = j.time[i];
+    float t;
+    uint32_t r;
+    if (j.st0) {
+      const uint2 v = *reinterpret_cast<const uint2 *>(j.st0 + i);
+      t = __uint_as_float(v.x);
+      r = v.y;
+    } else {
+      t = j.time[i];
+      r = j.refs[i];
+    }
     if (__ldg(j.speed + i) == 0.0f || t > j.max_time) t = FLT_MAX;
     j.time[i] = t;
     burned += t < FLT_MAX;
-    const uint32_t r = j.refs[i];
     if (j.out_rx) j.out_rx[i] = (uint16_t)(r & 0xFFFFu);
     if (j.out_ry) j.out_ry[i] = (uint16_t)(r >> 16);
   }

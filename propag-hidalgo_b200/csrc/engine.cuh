@@ -1,9 +1,25 @@
 // Internal interface between the host code and the propagation kernels.
 #pragma once
 
+#include <cuda_runtime.h>
+
 #include <cstdint>
 
+#include "dda_columns.cuh"
+
 namespace propag {
+
+// A cell of a global-memory tile.  los is the cell's line of sight to its
+// reference, walked once when the cell adopts it (boundaries do not change):
+// the cells the walk visits, up to and including the first boundary, and
+// kLosBlocked when it met one.
+struct alignas(16) CellState {
+  float time;
+  uint32_t ref;  // packed x | y << 16
+  uint32_t los;
+  uint32_t pad;
+};
+constexpr uint32_t kLosBlocked = 0x80000000u;
 
 // One scenario as the device sees it.
 struct JobDev {
@@ -15,8 +31,8 @@ struct JobDev {
   int32_t smem_tile;  // kSmemTile*: where tile launches keep the tile's state
   int32_t refm;       // 1: the reference's arithmetic in time_from, 0: portable
   const float *speed, *az, *ecc;
-  float *time;         // state, becomes the output after the post pass
-  uint32_t *refs;      // state: packed x | y << 16
+  float *time;         // the output; shared-memory tiles also keep their state here
+  uint32_t *refs;      // state of shared-memory tiles: packed x | y << 16
   uint32_t *bnd;       // boundary bits (written by the prep pass)
   // referrer box of every cell (the cells that ever adopted it as their
   // reference): min and max corner, 0xFFFFFFFF in box_x0 = empty
@@ -32,10 +48,12 @@ struct JobDev {
   // tt_plane.
   float *tt;
   int64_t tt_plane;
-  // Second copy of the state for global-memory tiles (sweeps alternate
-  // between the copies); null when every tile is resident in shared memory.
-  float *time1;
-  uint32_t *refs1;
+  // Global-memory tiles keep their state in two copies of packed cell records
+  // (sweeps alternate between them) and the fire fields packed beside box_x0;
+  // null when every tile is resident in shared memory.
+  CellState *st0, *st1;
+  float4 *fire4;  // speed, azimuth, eccentricity; w holds box_x0 (as bits)
+  int64_t box_x0_step;  // words between the box_x0 of consecutive cells (4 inside fire4, else 1)
   // Grid-wide pending bitmap of global-memory tiles (bit x + y W): cells whose
   // inputs changed since they were last evaluated, outside the tile that
   // changed them; a tile launch's first sweep evaluates only its pending
@@ -51,34 +69,24 @@ struct Update {
 };
 static_assert(sizeof(Update) == 16, "an update is read back as one 16-byte load");
 
-// An improvement of a global-memory tile's sweep, with what its commit needs:
-// burn = the cell burns (time < max_time, own fire not null); its referrer
-// box as read during the evaluation, corners (x0, y0), (x1, y1) in 16 bits
-// each (b01 = x0 | y0 << 16, b23 = x1 | y1 << 16; x0 = 0xFFFF: empty).
-struct TileUpdate {
-  uint32_t k;  // cell index inside the tile
-  float time;
-  uint32_t ref;
-  uint32_t burn;
-  uint32_t b01, b23;
-  uint32_t pad[2];
-};
-static_assert(sizeof(TileUpdate) == 32, "two 16-byte halves");
+// An improvement of a global-memory tile's sweep: the cell's new state and its
+// index inside the tile (in CellState's spare word).
+using TileUpdate = CellState;
 // Update entries a CTA keeps in shared memory per sweep parity (the rest go
 // to its global update region).
 constexpr int kTileUpdSmem = 1024;
 
 // Global-memory scratch of one team slot.  dirty/upd serve tile launches
-// whose state stays in global memory: the tile's dirty bitmaps (read by
-// every CTA of the team: a tile's cells are dealt to the CTAs in groups) and the
-// update arrays (one per sweep parity), CTA r of an R-CTA team using entries
-// from (parity * R + r) * cap on (cap = global_tile_upd_cap; the first
+// whose state stays in global memory: the tile's dirty bitmaps (owner-major:
+// each CTA's cells are consecutive bits, see owner_words) and the update
+// arrays (one per sweep parity), CTA r of an R-CTA team using entries from
+// (parity * R + r) * cap on (cap = global_tile_upd_cap; the first
 // kTileUpdSmem of them stay in shared memory); ovf_list/ovf_upd take the
 // work-list and update-list entries of shared-memory tiles beyond their
 // shared-memory capacity (ovf_cap entries per CTA of the cluster, CTA r at
 // offset r * ovf_cap).
 struct SlotDev {
-  uint32_t *dirty;        // three bitmaps of dirty_words words (in rotation by sweep)
+  uint32_t *dirty;        // two bitmaps of dirty_words words (alternating by sweep)
   uint32_t dirty_words;
   uint32_t pad0;
   TileUpdate *upd;
@@ -92,23 +100,38 @@ struct SlotDev {
   uint32_t pad;
 };
 
+// Ownership of a global-memory tile's cells: the tile-linear cells are cut
+// into groups of kOwnGroup consecutive cells, and group g belongs to CTA
+// g mod R of the team, so that the cells of a front spread over the CTAs
+// while a CTA's cells still come in short runs (its neighbour reads share
+// sectors).  Groups of 4 cells measured fastest on the 4096^2 scenario with
+// 148 CTAs (1 cell and whole 32-cell words were slower).
+// The dirty bitmap is owner-major: CTA r's owner_words words start at word
+// r * owner_words, and the cells of its l-th group are bits 4 l .. 4 l + 3, so
+// that a CTA reads only its own words (23 of them for a 323^2 tile and 148
+// CTAs, where a bitmap in tile order has 3 261).
+constexpr uint32_t kOwnGroup = 4;
+__host__ __device__ inline uint32_t owner_words(uint32_t TN, uint32_t R) {
+  return (((TN + kOwnGroup - 1) / kOwnGroup + R - 1) / R + 7) / 8;
+}
 // Update-array entries a CTA of an R-CTA team may need in one sweep of a
-// global-memory tile of TN cells (the cells it owns: groups of up to 32
-// consecutive cells dealt round-robin); the team needs R times that, at most
-// TN + 32 R.
+// global-memory tile of TN cells: the cells it owns.
 __host__ __device__ inline uint32_t global_tile_upd_cap(uint32_t TN, uint32_t R) {
-  return ((TN + 31) / 32 + R - 1) / R * 32;
+  return owner_words(TN, R) * 32;
 }
 
 // Shared memory a CTA needs for a global-memory tile launch: the work list
-// of one chunk (tile cell indices, 32 per thread), then two sweeps' update
-// entries.
+// of one chunk (tile cell indices, 32 per thread), two sweeps' update entries
+// and the crossing times of the line-of-sight walks.
 __host__ __device__ inline uint32_t global_tile_list_cap(int threads) { return (uint32_t)threads * 32u; }
 __host__ __device__ inline size_t global_tile_list_bytes(int threads) {
   return (size_t)global_tile_list_cap(threads) * 4;
 }
-__host__ __device__ inline size_t global_tile_smem(int threads) {
+__host__ __device__ inline size_t global_tile_cross_off(int threads) {
   return global_tile_list_bytes(threads) + 2 * kTileUpdSmem * sizeof(TileUpdate);
+}
+__host__ __device__ inline size_t global_tile_smem(int threads) {
+  return global_tile_cross_off(threads) + (size_t)kCrossTableLen * 4;
 }
 
 // Per-job statistics accumulated on the device (PropagStats order).
