@@ -37,8 +37,8 @@ cudaError_t launch_ignite(const JobDev *jobs, uint32_t n_jobs, cudaStream_t stre
 cudaError_t launch_engine(const JobDev *jobs, uint32_t n_jobs, const SlotDev *slots,
                           uint32_t n_slots, int csize, int threads, size_t smem, uint32_t *queue,
                           StatsDev *stats, unsigned long long max_sweeps, const uint32_t *order,
-                          uint32_t group, uint32_t phantom, cudaStream_t stream);
-cudaError_t engine_max_clusters(int csize, int threads, size_t smem, int *n);
+                          uint32_t group, uint32_t phantom, int arith, cudaStream_t stream);
+cudaError_t engine_max_clusters(int csize, int threads, size_t smem, int arith, bool group, int *n);
 cudaError_t launch_post(const JobDev *jobs, uint32_t n_jobs, uint64_t max_cells, int sms,
                         StatsDev *stats, cudaStream_t stream);
 cudaError_t launch_fire_weather(uint64_t n, int hour, int month, const float *t, const float *rh,
@@ -331,6 +331,9 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
                  align_up(words * 4, 256);
     max_cells = std::max<uint64_t>(max_cells, N);
   }
+  int arith = jd[0].refm;  // the jobs' common arithmetic, or 2: mixed
+  for (uint32_t i = 1; i < n_jobs; ++i)
+    if (jd[i].refm != arith) arith = 2;
   CK(e->job_scratch.reserve(job_bytes, stream));
   // ---- cluster size and tile residency ----
   // A tile launch runs in the cluster's shared memory when the tile and its
@@ -347,7 +350,7 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
     // 120 ms on a 16-CTA cluster; 64 members 408 ms (teams of 8) against
     // 514 (8-CTA clusters); 256 members 1 082 ms (teams of 4) against 1 531.
     int ctas = 0;
-    CK(engine_max_clusters(1, e->threads, global_tile_smem(e->threads), &ctas));
+    CK(engine_max_clusters(1, e->threads, global_tile_smem(e->threads), arith, true, &ctas));
     if (ctas >= 8) csize = -std::max(4, ctas / (int)std::max<uint32_t>(n_jobs, 1));
   }
   if (csize == 0) {
@@ -366,7 +369,7 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
       }
       if (!all) continue;
       int mc = 0;
-      CK(engine_max_clusters(c, e->threads, need, &mc));
+      CK(engine_max_clusters(c, e->threads, need, arith, false, &mc));
       const uint32_t conc = std::min<uint32_t>(n_jobs, (uint32_t)std::max(mc, 0));
       if (conc > best_conc) {
         best_conc = conc;
@@ -375,7 +378,7 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
     }
     if (csize == 0) {
       int ctas = 0;
-      CK(engine_max_clusters(1, e->threads, 0, &ctas));
+      CK(engine_max_clusters(1, e->threads, 0, arith, false, &ctas));
       csize = 1;
       while (csize < 16 && (uint64_t)(csize * 2) * n_jobs <= (uint64_t)std::max(ctas, 1)) csize *= 2;
     }
@@ -388,7 +391,7 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
     // global memory
     smem = global_tile_smem(e->threads);
     int ctas = 0;
-    CK(engine_max_clusters(1, e->threads, smem, &ctas));
+    CK(engine_max_clusters(1, e->threads, smem, arith, true, &ctas));
     if (ctas < 2) return fail(PROPAG_ERR_CUDA, "group mode needs at least 2 resident CTAs");
     const int team = csize == PROPAG_CLUSTER_GROUPS ? 32 : std::max(2, -csize);
     n_slots = std::min<uint32_t>(n_jobs, (uint32_t)std::max(1, ctas / team));
@@ -412,7 +415,7 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
       }
     }
     int max_clusters = 0;
-    CK(engine_max_clusters(csize, e->threads, smem, &max_clusters));
+    CK(engine_max_clusters(csize, e->threads, smem, arith, false, &max_clusters));
     if (max_clusters < 1) return fail(PROPAG_ERR_CUDA, "cluster size " + std::to_string(csize) + " cannot be resident");
     n_slots = std::min<uint32_t>(n_jobs, (uint32_t)max_clusters);
   }
@@ -534,7 +537,7 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
   CK(launch_ignite(d_jobs, n_jobs, stream));
   if (live) CK(cudaEventRecord(e->ev[1], stream));
   CK(launch_engine(d_jobs, n_jobs, d_slots, n_slots, csize, e->threads, smem, d_queue, d_stats,
-                   max_sweeps(), d_order, group, group ? e->phantom : 0u, stream));
+                   max_sweeps(), d_order, group, group ? e->phantom : 0u, arith, stream));
   if (live) CK(cudaEventRecord(e->ev[2], stream));
   CK(launch_post(d_jobs, n_jobs, max_cells, e->sms, d_stats, stream));
   if (live) CK(cudaEventRecord(e->ev[3], stream));
@@ -910,7 +913,8 @@ extern "C" int propag_run_device_static(const PropagJob *job, void *stream_ptr, 
     base = static_cast<char *>(g_static_base[dev]);
   }
   int max_clusters = 0;
-  CK(engine_max_clusters(csize, engine_threads(), smem, &max_clusters));
+  const int refm = j.arith == PROPAG_ARITH_REFERENCE ? 1 : 0;
+  CK(engine_max_clusters(csize, engine_threads(), smem, refm, false, &max_clusters));
   if (max_clusters < 1) return fail(PROPAG_ERR_CUDA, "cluster size " + std::to_string(csize) + " cannot be resident");
   JobDev d{};
   d.W = (int)j.width;
@@ -922,7 +926,7 @@ extern "C" int propag_run_device_static(const PropagJob *job, void *stream_ptr, 
   d.TX = (int)((j.width + T - 1) / T);
   d.TY = (int)((j.height + T - 1) / T);
   d.north_up = j.dy < 0 ? 1 : 0;
-  d.refm = j.arith == PROPAG_ARITH_REFERENCE ? 1 : 0;
+  d.refm = refm;
   d.smem_tile = exact ? kSmemTileExact : kSmemTileCoarse;
   d.speed = j.speed_max;
   d.az = j.azimuth_max;
@@ -955,7 +959,7 @@ extern "C" int propag_run_device_static(const PropagJob *job, void *stream_ptr, 
   CK(launch_prep(d_job, 1, N, sms, stream));
   CK(launch_ignite(d_job, 1, stream));
   CK(launch_engine(d_job, 1, d_slot, 1, csize, engine_threads(), smem, d_queue, d_stats, max_sweeps(),
-                   nullptr, 0u, 0u, stream));
+                   nullptr, 0u, 0u, d.refm, stream));
   CK(launch_post(d_job, 1, N, sms, d_stats, stream));
   if (stats) {
     StatsDev h;

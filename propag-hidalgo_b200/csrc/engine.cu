@@ -208,6 +208,17 @@ __global__ void ignite_kernel(const JobDev *__restrict__ jobs) {
 }
 
 // ------------------------------------------------------- common pieces ----
+// The engine kernel is compiled for batches whose jobs all use one arithmetic
+// of time_from (PROPAG_ARITH_*: kArithRef, kArithPortable) and for mixed ones
+// (kArithMixed, chosen per job): a sweep is one pass of each warp through
+// straight-line code, so code that a batch does not use costs instruction
+// fetches.
+constexpr int kArithPortable = 0, kArithRef = 1, kArithMixed = 2;
+template <int kArith>
+__device__ __forceinline__ bool arith_of(const JobDev &j) {
+  return kArith == kArithMixed ? j.refm != 0 : kArith == kArithRef;
+}
+
 struct Best {
   float time;
   uint32_t ref;
@@ -235,7 +246,7 @@ struct Counters {
 // cell's own time); only the walks the sequential loop performs (candidate
 // also faster than every earlier offer) are counted, so the counters match
 // the reference's order exactly.  Called by all 32 lanes.
-template <typename Acc>
+template <int kArith, typename Acc>
 __device__ __forceinline__ Best evaluate_coop(const JobDev &j, const DirConst &dc, const Acc &acc,
                                               int x, int y, Best own, bool valid, uint32_t lane,
                                               Counters &cnt) {
@@ -265,7 +276,7 @@ __device__ __forceinline__ Best evaluate_coop(const JobDev &j, const DirConst &d
   uint32_t oref = 0, steps = 0;
   bool walked = false;
   if (act) {
-    const bool refm = j.refm != 0;
+    const bool refm = arith_of<kArith>(j);
     const float ntime =
         step_time(nt, dc.dist[k], j.tt ? tt : dir_inv_speed(dc, k, f, refm), refm);
     cand = time_from(ref_x(nr), ref_y(nr), rt, x, y, f, j.gdx, j.gdy, j.north_up != 0, refm);
@@ -440,7 +451,7 @@ constexpr uint32_t kScanInline = 32;
 // marked set independent of the order of this sweep's commits.
 __device__ __forceinline__ bool referrer(const JobDev &j, const CellState *__restrict__ X, int xx, int yy,
                                          uint32_t want) {
-  const int64_t c = xx + (int64_t)yy * j.W;
+  const uint32_t c = (uint32_t)xx + (uint32_t)yy * (uint32_t)j.W;
   const uint2 s = __ldcg(reinterpret_cast<const uint2 *>(X + c));
   return s.y == want && __uint_as_float(s.x) < j.max_time && __ldg(&j.fire4[c].x) != 0.0f;
 }
@@ -555,8 +566,9 @@ __device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t *p) {
   return v;
 }
 
+template <bool kGroup>
 struct Team {
-  unsigned long long *bar;  // group mode: the two arrival words; null = cluster
+  unsigned long long *bar;  // group mode: the two arrival words
   uint32_t *err;            // group mode: the launch's error flag
   int *ok;                  // shared: [0] this CTA's outcome of the last wait, [1] improving CTAs
   uint32_t G;               // CTAs in the group
@@ -580,7 +592,7 @@ struct Team {
   __device__ bool sync(bool global_fence = true, const uint32_t *improved_ctr = nullptr,
                        uint32_t *improving = nullptr) {
     const long long t0 = threadIdx.x == 0 ? clock64() : 0;
-    if (!bar) {
+    if constexpr (!kGroup) {
       if (improving) {
         __syncthreads();  // the CTA's updates are counted
         if (threadIdx.x == 0 && *improved_ctr) atomicAdd(cnt3 + cnt_phase, 1u);
@@ -600,7 +612,7 @@ struct Team {
         *improving = (uint32_t)ok[1];
       }
       return true;
-    }
+    } else {
     __syncthreads();
     if (threadIdx.x == 0) {
       const bool improved = improved_ctr && *improved_ctr != 0u;
@@ -632,6 +644,7 @@ struct Team {
     __syncthreads();
     if (improving) *improving = (uint32_t)ok[1];
     return ok[0] != 0;
+    }
   }
 };
 
@@ -813,35 +826,45 @@ __device__ __forceinline__ CellState get_update(const TileUpdate *sm_upd, const 
 // but the last sum of the candidate's time is independent of the reference's
 // time, and runs while that load is in flight.  own: the cell's state; the
 // result is the lanes' common view (best.time < own.time: improved).
-__device__ __forceinline__ Best evaluate_packed(const JobDev &j, const DirConst &dc,
+// hot: the job's fields that every evaluation reads, and this lane's
+// neighbour, in registers (the job itself lives in shared memory).
+struct Hot {
+  int W, H, dx, dy;  // grid; offset of the lane's neighbour
+  float max_time, gdx, gdy;
+  float bearing, dist;  // from the neighbour to the cell
+  bool north_up;
+  const float4 *fire4;
+};
+
+template <int kArith>
+__device__ __forceinline__ Best evaluate_packed(const JobDev &j, const Hot &h,
                                                 const CellState *__restrict__ X, int x, int y, Best own,
                                                 bool valid, uint32_t lane, Counters &cnt) {
   const float kInf = __int_as_float(0x7f800000);
   const int k = (int)(lane & 7u);
-  const int kk = k < 4 ? k : k + 1;
-  const int nx = x + kk % 3 - 1, ny = y + kk / 3 - 1;
-  const bool refm = j.refm != 0;
+  const int nx = x + h.dx, ny = y + h.dy;
+  const bool refm = arith_of<kArith>(j);
   CellState n{FLT_MAX, kNoRef, 0u, 0u};
   Fire f{0.0f, 0.0f, 0.0f};
-  if (valid && nx >= 0 && ny >= 0 && nx < j.W && ny < j.H) {
-    const int64_t c = nx + (int64_t)ny * j.W;
+  if (valid && (uint32_t)nx < (uint32_t)h.W && (uint32_t)ny < (uint32_t)h.H) {
+    const uint32_t c = (uint32_t)nx + (uint32_t)ny * (uint32_t)h.W;  // grids below 2^32 cells
     n = ld_state(X + c);
-    const float4 v = __ldg(j.fire4 + c);
+    const float4 v = __ldg(h.fire4 + c);
     f = Fire{v.x, v.y, v.z};
   }
   const int rx = ref_x(n.ref), ry = ref_y(n.ref);
-  const bool act = n.time < j.max_time && f.speed_max != 0.0f && !(rx == x && ry == y);
+  const bool act = n.time < h.max_time && f.speed_max != 0.0f && n.ref != pack_ref(x, y);
   float rt = FLT_MAX;
-  if (act) rt = __ldcg(&X[rx + (int64_t)ry * j.W].time);
+  if (act) rt = __ldcg(&X[(uint32_t)rx + (uint32_t)ry * (uint32_t)h.W].time);
   cnt.gat += act ? 1u : 0u;
   float offer = kInf, cand = kInf;
   uint32_t oref = 0;
   bool walked = false;
   if (act) {
-    offer = step_time(n.time, dc.dist[k], dir_inv_speed(dc, k, f, refm), refm);
+    offer = step_time(n.time, h.dist, inv_speed(h.bearing, f, refm), refm);
     oref = pack_ref(nx, ny);
-    const float inv = inv_speed(bearing(rx, ry, x, y, j.north_up != 0, refm), f, refm);
-    const float dist = cell_distance(rx - x, ry - y, j.gdx, j.gdy, refm);
+    const float inv = inv_speed(bearing(rx, ry, x, y, h.north_up, refm), f, refm);
+    const float dist = cell_distance(rx - x, ry - y, h.gdx, h.gdy, refm);
     cand = step_time(rt, dist, inv, refm);
     if (cand < offer) {
       walked = cand < own.time;
@@ -1033,9 +1056,10 @@ __device__ __forceinline__ uint32_t walk_los(const uint32_t *__restrict__ bnd, c
 // scans read referrers outside the launching tile too, from X[p]: a launch
 // writes only its tile's cells, and both copies agree everywhere when a
 // launch ends, so outside the tile X[0] and X[1] hold the same state.
-__device__ bool tile_global(const JobDev &j, const DirConst &dc, const SlotDev &s, const TileDesc &td,
+template <int kArith, bool kGroup>
+__device__ __forceinline__ bool tile_global(const JobDev &j, const DirConst &dc, const SlotDev &s, const TileDesc &td,
                             uint32_t *list, TileUpdate *sm_upd, uint32_t *cta_ctr, ScanItem *queue, const float *cross,
-                            uint32_t rank, uint32_t R, SweepCtx &cx, Team &team) {
+                            uint32_t rank, uint32_t R, SweepCtx &cx, Team<kGroup> &team) {
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const uint32_t k8 = lane & 7u, g0 = lane & 24u;
   const int x0 = td.x0, y0 = td.y0, TW = td.TW, TH = td.TH;
@@ -1046,6 +1070,23 @@ __device__ bool tile_global(const JobDev &j, const DirConst &dc, const SlotDev &
   // the work list holds a chunk of words at a time: usually all of them
   const uint32_t chunk = global_tile_list_cap(blockDim.x) / 32u;
   const CellState *const X[2] = {j.st0, j.st1};
+  Hot h;
+  {
+    const int kk = k8 < 4 ? (int)k8 : (int)k8 + 1;
+    h.W = j.W;
+    h.H = j.H;
+    h.dx = kk % 3 - 1;
+    h.dy = kk / 3 - 1;
+    h.max_time = j.max_time;
+    h.gdx = j.gdx;
+    h.gdy = j.gdy;
+    h.bearing = dc.bearing[k8];
+    h.dist = dc.dist[k8];
+    h.north_up = j.north_up != 0;
+    h.fire4 = j.fire4;
+  }
+  uint32_t *const pending = j.pending;
+  const uint32_t *const bnd = j.bnd;
   // the launch's counters in registers (the context may live in local memory)
   Counters cnt = cx.cnt;
   bool first = true, worked = false;
@@ -1070,8 +1111,8 @@ __device__ bool tile_global(const JobDev &j, const DirConst &dc, const SlotDev &
     // the neighbours of a referrer
     auto mark_around = [&](int xx, int yy) {
       tb.mark3x3(dirty_next, xx - x0, yy - y0);
-      if (j.pending && tile_border(xx - x0, yy - y0, TW, TH))
-        for (int t = 0; t < 9; ++t) mark_pending(j.pending, j, x0, y0, xx - x0, yy - y0, TW, TH, t);
+      if (pending && tile_border(xx - x0, yy - y0, TW, TH))
+        for (int t = 0; t < 9; ++t) mark_pending(pending, j, x0, y0, xx - x0, yy - y0, TW, TH, t);
     };
     for (uint32_t c0 = 0; c0 < tb.wpo; c0 += chunk) {
       if (c0) __syncthreads();  // the previous chunk's list is consumed
@@ -1095,7 +1136,7 @@ __device__ bool tile_global(const JobDev &j, const DirConst &dc, const SlotDev &
           const uint32_t g = l * R + rank;
           if (g >= ngroups) break;
           const uint32_t n = min(kOwnGroup, TN - g * kOwnGroup);
-          uint32_t bits = j.pending ? take_pending(j.pending, j, x0, y0, TW, g * kOwnGroup, n) : (1u << n) - 1u;
+          uint32_t bits = pending ? take_pending(pending, j, x0, y0, TW, g * kOwnGroup, n) : (1u << n) - 1u;
           if (bits) {
             uint32_t at = atomicAdd(cta_ctr + q, (uint32_t)__popc(bits));
             for (; bits; bits &= bits - 1) list[at++] = g * kOwnGroup + (uint32_t)(__ffs(bits) - 1);
@@ -1109,7 +1150,7 @@ __device__ bool tile_global(const JobDev &j, const DirConst &dc, const SlotDev &
           CellState e = get_update(sm_upd + (p ^ 1) * kTileUpdSmem, s.upd + ((size_t)(p ^ 1) * R + rank) * cap, u);
           uint32_t col;
           const uint32_t row = tb.by_tw.div(e.pad, col);
-          st_state(ws + (x0 + (int)col) + (int64_t)(y0 + (int)row) * j.W, e);
+          st_state(ws + ((uint32_t)x0 + col + ((uint32_t)y0 + row) * (uint32_t)h.W), e);
         }
       __syncthreads();
       for (uint32_t w = c0 + threadIdx.x; w < c1; w += blockDim.x) dirty[w] = 0u;  // marked again in the next sweep at the earliest
@@ -1128,7 +1169,7 @@ __device__ bool tile_global(const JobDev &j, const DirConst &dc, const SlotDev &
         const bool valid = (lane >> 3) < per && ci < nlist;
         uint32_t k = 0;
         int lx = 0, ly = 0, x = 0, y = 0;
-        int64_t c = 0;
+        uint32_t c = 0;
         Best own{FLT_MAX, kNoRef};
         uint32_t corner = 0;  // lanes 0..3 of the cell: x0, y0, x1, y1 of its referrer box
         float own_speed = 0.0f;
@@ -1139,19 +1180,19 @@ __device__ bool tile_global(const JobDev &j, const DirConst &dc, const SlotDev &
           lx = (int)col;
           x = x0 + lx;
           y = y0 + ly;
-          c = x + (int64_t)y * j.W;
+          c = (uint32_t)x + (uint32_t)y * (uint32_t)h.W;
           const CellState o = ld_state(rs + c);
           own = Best{o.time, o.ref};
           if (k8 < 4) {
-            const uint32_t *const b = k8 == 0   ? j.box_x0 + c * j.box_x0_step
+            const uint32_t *const b = k8 == 0   ? reinterpret_cast<const uint32_t *>(h.fire4 + c) + 3
                                       : k8 == 1 ? j.box_y0 + c
                                       : k8 == 2 ? j.box_x1 + c
                                                 : j.box_y1 + c;
             corner = __ldcg(b);
           }
-          own_speed = __ldg(&j.fire4[c].x);
+          own_speed = __ldg(&h.fire4[c].x);
         }
-        const Best b = evaluate_packed(j, dc, rs, x, y, own, valid, lane, cnt);
+        const Best b = evaluate_packed<kArith>(j, h, rs, x, y, own, valid, lane, cnt);
         const bool improved = valid && b.time < own.time;  // common to the cell's lanes
         if (!__any_sync(kFull, improved)) continue;
         // referrer box (whole with a pending bitmap: referrers anywhere mark
@@ -1163,11 +1204,11 @@ __device__ bool tile_global(const JobDev &j, const DirConst &dc, const SlotDev &
         box.y1 = (int)__shfl_sync(kFull, corner, g0 + 3);
         if (!improved || (uint32_t)box.x0 == kEmptyBox)
           box = Box{1, 1, 0, 0};
-        else if (j.pending)
+        else if (pending)
           box = Box{max(box.x0, 0), max(box.y0, 0), min(box.x1, j.W - 1), min(box.y1, j.H - 1)};
         else
           box = clip_box(box.x0, box.y0, box.x1, box.y1, x0, y0, TW, TH, j.W, j.H);
-        const uint32_t los = walk_los(j.bnd, cross, j.W, x, y, ref_x(b.ref), ref_y(b.ref), improved, lane);
+        const uint32_t los = walk_los(bnd, cross, h.W, x, y, ref_x(b.ref), ref_y(b.ref), improved, lane);
         const uint32_t adds = __ballot_sync(kFull, improved && k8 == 0);
         uint32_t ai = 0;
         if (lane == 0) ai = atomicAdd(upd_ctr, (uint32_t)__popc(adds));
@@ -1182,16 +1223,16 @@ __device__ bool tile_global(const JobDev &j, const DirConst &dc, const SlotDev &
               st_state(upd + ai, e);
           }
           // the reference's box grows to hold (x, y), a corner a lane
-          const int64_t rc = ref_x(b.ref) + (int64_t)ref_y(b.ref) * j.W;
-          if (k8 == 0) atomicMin(j.box_x0 + rc * j.box_x0_step, (uint32_t)x);
+          const uint32_t rc = (uint32_t)ref_x(b.ref) + (uint32_t)ref_y(b.ref) * (uint32_t)h.W;
+          if (k8 == 0) atomicMin(j.box_x0 + 4 * (size_t)rc, (uint32_t)x);
           if (k8 == 1) atomicMin(j.box_y0 + rc, (uint32_t)y);
           if (k8 == 2) atomicMax(j.box_x1 + rc, (uint32_t)x);
           if (k8 == 3) atomicMax(j.box_y1 + rc, (uint32_t)y);
           // only a burning cell is read by its neighbours
-          if (b.time < j.max_time && own_speed != 0.0f) {
+          if (b.time < h.max_time && own_speed != 0.0f) {
             if (k8 < 6) tb.mark_half(dirty_next, lx, ly, (int)(k8 >> 1), (int)(k8 & 1u));
-            if (j.pending && tile_border(lx, ly, TW, TH))
-              mark_pending(j.pending, j, x0, y0, lx, ly, TW, TH, (int)(k8 < 4 ? k8 : k8 + 1));
+            if (pending && tile_border(lx, ly, TW, TH))
+              mark_pending(pending, j, x0, y0, lx, ly, TW, TH, (int)(k8 < 4 ? k8 : k8 + 1));
           }
         }
         warp_scan_boxes4(box, pack_ref(x, y), j, rs, lane, cnt, queue, cta_ctr + 4, mark_around);
@@ -1451,9 +1492,9 @@ struct SmemAcc {
 
 // One tile launch resident in the cluster's shared memory; B is the staged
 // referrer-box codec.
-template <class B>
+template <class B, int kArith>
 __device__ bool tile_smem(const JobDev &j, const DirConst &dc, char *smem, const SlotDev &slot,
-                          const TileDesc &td, ScanBox *scan_boxes, SweepCtx &cx, Team &team) {
+                          const TileDesc &td, ScanBox *scan_boxes, SweepCtx &cx, Team<false> &team) {
   using BoxT = typename B::T;
   cg::cluster_group cluster = cg::this_cluster();
   SmemGeom g;
@@ -1551,7 +1592,7 @@ __device__ bool tile_smem(const JobDev &j, const DirConst &dc, char *smem, const
         y = g.y0 - 1 + hy;
         own = Best{sm.time[s], sm.ref[s]};
       }
-      const Best b = evaluate_coop(j, dc, SmemAcc{j, sm, g}, x, y, own, valid, lane, cnt);
+      const Best b = evaluate_coop<kArith>(j, dc, SmemAcc{j, sm, g}, x, y, own, valid, lane, cnt);
       const bool improved = valid && (lane & 7) == 0 && b.time < own.time;
       const uint32_t at = warp_append(sm.ctr + 1, improved ? 1u : 0u, lane);
       if (improved) upd_put(sm, at, s, b.time, b.ref);
@@ -1673,21 +1714,16 @@ __device__ bool tile_smem(const JobDev &j, const DirConst &dc, char *smem, const
 // (group = G > 1, launched cooperatively without clusters): CTAs
 // [g * G, (g + 1) * G) form team g, which keeps its tiles in global memory
 // and meets at the bounded counter barrier of its slot.
-__global__ void __launch_bounds__(kEngineThreads, 1) engine_kernel(const JobDev *__restrict__ jobs,
-                                                         uint32_t n_jobs,
-                                                         const SlotDev *__restrict__ slots,
-                                                         uint32_t *__restrict__ queue,
-                                                         StatsDev *__restrict__ stats,
-                                                         unsigned long long max_sweeps,
-                                                         const uint32_t *__restrict__ order,
-                                                         uint32_t group) {
+template <int kArith, bool kGroup>
+__global__ void __launch_bounds__(kEngineThreads, 1)
+    engine_kernel(const JobDev *__restrict__ jobs, uint32_t n_jobs, const SlotDev *__restrict__ slots,
+                  uint32_t *__restrict__ queue, StatsDev *__restrict__ stats,
+                  unsigned long long max_sweeps, const uint32_t *__restrict__ order, uint32_t group) {
   extern __shared__ __align__(16) char dyn_smem[];
-  cg::cluster_group cluster = cg::this_cluster();
-  const bool grouped = group > 1;
-  const uint32_t csize = grouped ? group : cluster.num_blocks();
+  const uint32_t csize = kGroup ? group : cg::this_cluster().num_blocks();
   const uint32_t slot_id = blockIdx.x / csize;
   const SlotDev s = slots[slot_id];
-  const uint32_t rank = grouped ? blockIdx.x % csize : cluster.block_rank();
+  const uint32_t rank = kGroup ? blockIdx.x % csize : cg::this_cluster().block_rank();
   const uint32_t tid = rank * blockDim.x + threadIdx.x;
   const uint32_t lane = threadIdx.x & 31;
   __shared__ DirConst dc;
@@ -1696,8 +1732,7 @@ __global__ void __launch_bounds__(kEngineThreads, 1) engine_kernel(const JobDev 
   static_assert(sizeof(ScanItem) * kScanQueue <= sizeof(ScanBox) * kEngineThreads, "the scan queue fits");
   __shared__ int team_ok[2];
   __shared__ uint32_t cta_ctr[5];  // global-memory tiles: work-list and update counts (two each), scan queue
-  Team team{grouped ? reinterpret_cast<unsigned long long *>(s.ctr + 8) : nullptr, queue + 1,
-            team_ok, csize};
+  Team<kGroup> team{reinterpret_cast<unsigned long long *>(s.ctr + 8), queue + 1, team_ok, csize};
   team.cnt3 = s.ctr + 5;  // cluster mode: slot counters 5..7
   team.cnt_leader = rank == 0;
   float *const cross = reinterpret_cast<float *>(dyn_smem + global_tile_cross_off(blockDim.x));
@@ -1746,14 +1781,18 @@ __global__ void __launch_bounds__(kEngineThreads, 1) engine_kernel(const JobDev 
         td.y0 = (t / j.TX) * j.T;
         td.TW = min(j.T, j.W - td.x0);
         td.TH = min(j.T, j.H - td.y0);
-        const bool w = j.smem_tile == kSmemTileExact
-                           ? tile_smem<BoxExact>(j, dc, dyn_smem, s, td, scan_boxes, cx, team)
-                       : j.smem_tile == kSmemTileCoarse
-                           ? tile_smem<BoxCoarse>(j, dc, dyn_smem, s, td, scan_boxes, cx, team)
-                           : tile_global(j, dc, s, td, reinterpret_cast<uint32_t *>(dyn_smem),
-                                         reinterpret_cast<TileUpdate *>(
-                                             dyn_smem + global_tile_list_bytes(blockDim.x)),
-                                         cta_ctr, reinterpret_cast<ScanItem *>(scan_boxes), cross, rank, csize, cx, team);
+        bool w = false;
+        if constexpr (!kGroup) {
+          if (j.smem_tile == kSmemTileExact)
+            w = tile_smem<BoxExact, kArith>(j, dc, dyn_smem, s, td, scan_boxes, cx, team);
+          else if (j.smem_tile == kSmemTileCoarse)
+            w = tile_smem<BoxCoarse, kArith>(j, dc, dyn_smem, s, td, scan_boxes, cx, team);
+        }
+        if (kGroup || j.smem_tile == kSmemTileGlobal)
+          w = tile_global<kArith, kGroup>(
+              j, dc, s, td, reinterpret_cast<uint32_t *>(dyn_smem),
+              reinterpret_cast<TileUpdate *>(dyn_smem + global_tile_list_bytes(blockDim.x)), cta_ctr,
+              reinterpret_cast<ScanItem *>(scan_boxes), cross, rank, csize, cx, team);
         round_worked |= w;
       }
       if (!round_worked || cx.abort) break;
@@ -1869,22 +1908,35 @@ static cudaLaunchConfig_t engine_config(int csize, int threads, unsigned blocks,
   return cfg;
 }
 
-static cudaError_t engine_attrs(size_t smem) {
-  cudaError_t e = cudaFuncSetAttribute(engine_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+using EngineKernel = void (*)(const JobDev *, uint32_t, const SlotDev *, uint32_t *, StatsDev *, unsigned long long,
+                              const uint32_t *, uint32_t);
+static EngineKernel engine_for(int arith, bool group) {
+  if (arith == kArithRef) return group ? engine_kernel<kArithRef, true> : engine_kernel<kArithRef, false>;
+  if (arith == kArithPortable)
+    return group ? engine_kernel<kArithPortable, true> : engine_kernel<kArithPortable, false>;
+  return group ? engine_kernel<kArithMixed, true> : engine_kernel<kArithMixed, false>;
+}
+
+static cudaError_t engine_attrs(EngineKernel kernel, size_t smem) {
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(engine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
 int engine_threads() { return kEngineThreads; }
 
-cudaError_t engine_max_clusters(int csize, int threads, size_t smem, int *n) {
-  cudaError_t e = engine_attrs(smem);
+// Clusters of csize CTAs resident at once, of the kernel that launch_engine
+// runs for this arithmetic and kind of team.
+cudaError_t engine_max_clusters(int csize, int threads, size_t smem, int arith, bool group, int *n) {
+  const EngineKernel kernel = engine_for(arith, group);
+  cudaError_t e = engine_attrs(kernel, smem);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = engine_config(csize, threads, (unsigned)csize, smem, attr, 0);
-  return cudaOccupancyMaxActiveClusters(n, engine_kernel, &cfg);
+  return cudaOccupancyMaxActiveClusters(n, kernel, &cfg);
 }
 
+// arith: the jobs' common arithmetic (their JobDev::refm), or kArithMixed (2).
 // group == 0: n_slots clusters of csize CTAs.  group > 1: n_slots teams of
 // `group` CTAs in one cooperative launch (all CTAs co-resident, which the
 // teams' barriers need; the launch fails rather than run otherwise).
@@ -1893,8 +1945,9 @@ cudaError_t engine_max_clusters(int csize, int threads, size_t smem, int *n) {
 cudaError_t launch_engine(const JobDev *jobs, uint32_t n_jobs, const SlotDev *slots,
                           uint32_t n_slots, int csize, int threads, size_t smem, uint32_t *queue,
                           StatsDev *stats, unsigned long long max_sweeps, const uint32_t *order,
-                          uint32_t group, uint32_t phantom, cudaStream_t stream) {
-  cudaError_t e = engine_attrs(smem);
+                          uint32_t group, uint32_t phantom, int arith, cudaStream_t stream) {
+  const EngineKernel kernel = engine_for(arith, group > 1);
+  cudaError_t e = engine_attrs(kernel, smem);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr[1];
   if (group > 1) {
@@ -1908,11 +1961,11 @@ cudaError_t launch_engine(const JobDev *jobs, uint32_t n_jobs, const SlotDev *sl
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (phantom && n_slots != 1) return cudaErrorInvalidValue;
-    return cudaLaunchKernelEx(&cfg, engine_kernel, jobs, n_jobs, slots, queue, stats, max_sweeps,
+    return cudaLaunchKernelEx(&cfg, kernel, jobs, n_jobs, slots, queue, stats, max_sweeps,
                               order, group + phantom);
   }
   cudaLaunchConfig_t cfg = engine_config(csize, threads, n_slots * (unsigned)csize, smem, attr, stream);
-  return cudaLaunchKernelEx(&cfg, engine_kernel, jobs, n_jobs, slots, queue, stats, max_sweeps, order,
+  return cudaLaunchKernelEx(&cfg, kernel, jobs, n_jobs, slots, queue, stats, max_sweeps, order,
                             0u);
 }
 
