@@ -44,7 +44,9 @@ cudaError_t launch_rasterize_winner(const RasterPlanDev &p, int64_t W, int64_t H
     segment_kernel<<<grid_for((p.samples + kRasterThreads - 1) / kRasterThreads, sm_count, 8),
                      kRasterThreads, 0, stream>>>(p.segs, p.nseg, p.samples, W, H, win);
   if (p.rows)
-    polygon_kernel<<<grid_for(p.rows, sm_count, 4), kRasterThreads, 0, stream>>>(
+    polygon_kernel<<<grid_for(W <= 32 * (int64_t)kWarpRowWords ? (p.rows + kRasterWarps - 1) / kRasterWarps : p.rows,
+                             sm_count, 8),
+                     kRasterThreads, 0, stream>>>(
         p.polys, p.npoly, p.rows, p.edges, W, win);
   return cudaGetLastError();
 }

@@ -57,13 +57,15 @@ struct RasterEdge {
   double ax, ay, bx, by;
 };
 
-// A polygon: edges [first, first + count) and grid rows [row0, row1].
+// A polygon: edges [first, first + count), grid rows [row0, row1], and the
+// columns that can lie inside it, [col0, col1] before clipping to the grid.
 struct RasterPoly {
   uint64_t first;
   uint64_t before;  // rows of the polygons ahead of this one in the plan
   uint32_t count;
   int32_t feature;
   int32_t row0, row1;
+  int32_t col0, col1;
 };
 
 // Segments and polygons that reach a W x H grid, in burn order.
@@ -176,11 +178,15 @@ inline void plan_polygon(RasterPlan &plan, const std::vector<std::vector<Pt>> &r
   RasterPoly p{};
   p.first = plan.edges.size();
   p.feature = feature;
-  double rmin = 1e300, rmax = -1e300;
+  double rmin = 1e300, rmax = -1e300, cmin = 1e300, cmax = -1e300;
+  bool plain = true;  // finite vertices of ordinary size: crossings lie between them
   for (const auto &ring : rings) {
     for (const Pt &q : ring) {
       rmin = std::min(rmin, q.y);
       rmax = std::max(rmax, q.y);
+      cmin = std::min(cmin, q.x);
+      cmax = std::max(cmax, q.x);
+      plain = plain && std::fabs(q.x) < 1e9 && std::fabs(q.y) < 1e9;
     }
     for (size_t k = 0; k + 1 < ring.size(); ++k)
       plan.edges.push_back({ring[k].x, ring[k].y, ring[k + 1].x, ring[k + 1].y});
@@ -196,6 +202,11 @@ inline void plan_polygon(RasterPlan &plan, const std::vector<std::vector<Pt>> &r
   p.count = (uint32_t)count;
   p.row0 = (int32_t)r0;
   p.row1 = (int32_t)r1;
+  // a crossing rounds to within a small fraction of a cell of its edge, and an
+  // even number of them leaves every column outside [col0, col1] outside the
+  // polygon; vertices for which that does not hold take every column
+  p.col0 = plain ? (int32_t)std::floor(cmin) - 2 : 0;
+  p.col1 = plain ? (int32_t)std::ceil(cmax) + 2 : 0x7FFFFFFF;
   p.before = plan.rows;
   plan.rows += (uint64_t)(p.row1 - p.row0 + 1);
   plan.polys.push_back(p);

@@ -15,6 +15,8 @@ namespace raster_dev {
 
 constexpr int kRasterThreads = 256;  // every kernel below assumes 8 warps
 constexpr int kRowWords = 2048;      // row mask words: 65536 columns
+constexpr int kRasterWarps = kRasterThreads / 32;
+constexpr int kWarpRowWords = kRowWords / kRasterWarps;  // one warp's share of the mask: 8192 columns
 
 __global__ void __launch_bounds__(kRasterThreads) fill_winner_kernel(int32_t *win, int64_t n) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -47,40 +49,80 @@ __global__ void __launch_bounds__(kRasterThreads)
   }
 }
 
-// One polygon row per CTA iteration.  W <= 32 * kRowWords.
+// Polygon rows a CTA takes per iteration: one per warp while a row's mask fits
+// a warp's share of shared memory (grids up to 8192 columns), else one row
+// for the whole CTA.  Most polygons of a fuel map are narrow, and a CTA spent
+// its time on five barriers per row: 1200 polygons of 20 to 480 cells on a
+// 3001 x 2003 grid took 1005 us with a CTA and every column of the grid per
+// row, 145 us with a warp and the polygon's own columns.
+__device__ __forceinline__ int polygon_rows_per_cta(int64_t W) {
+  return W <= 32 * kWarpRowWords ? kRasterWarps : 1;
+}
+
+// A barrier of the threads that share a row.  (The CPU emulation has block
+// barriers only; its blocks meet all of them together.)
+#if defined(__CUDACC__)
+#define PG_ROW_SYNC(warp_row) \
+  do {                        \
+    if (warp_row)             \
+      __syncwarp();           \
+    else                      \
+      __syncthreads();        \
+  } while (0)
+#else
+#define PG_ROW_SYNC(warp_row) __syncthreads()
+#endif
+
+// W <= 32 * kRowWords.
 __global__ void __launch_bounds__(kRasterThreads)
     polygon_kernel(const RasterPoly *__restrict__ polys, uint64_t npoly, uint64_t rows,
                    const RasterEdge *__restrict__ edges, int64_t W, int32_t *__restrict__ win) {
-  __shared__ uint32_t mask[kRowWords];
-  __shared__ uint32_t warp_parity[kRasterThreads / 32];
+  __shared__ uint32_t masks[kRowWords];
+  __shared__ uint32_t warp_parity[kRasterWarps];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int nw = (int)((W + 31) / 32);
-  const int per = (nw + kRasterThreads - 1) / kRasterThreads;  // words per thread
-  const int w0 = min(nw, tid * per), w1 = min(nw, w0 + per);
-  for (uint64_t item = blockIdx.x; item < rows; item += gridDim.x) {
-    const RasterPoly p = polys[find_part(polys, npoly, item)];
-    const int64_t r = (int64_t)p.row0 + (int64_t)(item - p.before);
-    for (int w = tid; w < nw; w += kRasterThreads) mask[w] = 0u;
-    __syncthreads();
+  const int at_once = polygon_rows_per_cta(W);
+  const bool warp_row = at_once > 1;
+  const int gt = warp_row ? lane : tid, gn = warp_row ? 32 : kRasterThreads;  // this row's threads
+  uint32_t *const mask = masks + (warp_row ? wid * kWarpRowWords : 0);
+  for (uint64_t base = (uint64_t)blockIdx.x * at_once; base < rows; base += (uint64_t)gridDim.x * at_once) {
+    const uint64_t item = base + (warp_row ? (uint64_t)wid : 0);
+    RasterPoly p{};
+    int64_t r = 0;
+    int64_t c0 = 0, c1 = -1;  // the columns looked at: c0 a multiple of 32
+    if (item < rows) {
+      p = polys[find_part(polys, npoly, item)];
+      r = (int64_t)p.row0 + (int64_t)(item - p.before);
+      c0 = p.col0 > 0 ? (int64_t)p.col0 / 32 * 32 : 0;
+      c1 = p.col1 < W - 1 ? (int64_t)p.col1 : W - 1;
+    }
+    const int nw = c1 >= c0 ? (int)((c1 - c0) / 32 + 1) : 0;  // mask words in use
+    for (int w = gt; w < nw; w += gn) mask[w] = 0u;
+    PG_ROW_SYNC(warp_row);
     // a crossing toggles the first column whose centre is at or right of it
     const double yc = (double)r + 0.5;
-    for (uint64_t k = tid; k < p.count; k += kRasterThreads) {
+    for (uint64_t k = gt; nw > 0 && k < p.count; k += gn) {
       double x;
       if (!edge_crossing(edges[p.first + k], yc, x)) continue;
-      const int64_t c = crossing_cell(x, W);
-      if (c < W) atomicXor(&mask[c >> 5], 1u << (c & 31));
+      int64_t c = crossing_cell(x, W);
+      if (c > c1) continue;
+      c = c > c0 ? c - c0 : 0;
+      atomicXor(&mask[c >> 5], 1u << (c & 31));
     }
-    __syncthreads();
+    PG_ROW_SYNC(warp_row);
     // inside = odd number of toggles at or left of the column: an inclusive
     // prefix XOR along the row (within a word by shifts, across words and
     // threads by the parity of everything ahead)
+    const int per = (nw + gn - 1) / gn;  // words per thread
+    const int w0 = min(nw, gt * per), w1 = min(nw, w0 + per);
     uint32_t par = 0;
     for (int w = w0; w < w1; ++w) par ^= (uint32_t)__popc(mask[w]) & 1u;
     const uint32_t vote = __ballot_sync(0xFFFFFFFFu, par != 0u);
     uint32_t carry = (uint32_t)__popc(vote & ((1u << lane) - 1u)) & 1u;
-    if (lane == 0) warp_parity[wid] = (uint32_t)__popc(vote) & 1u;
-    __syncthreads();
-    for (int k = 0; k < wid; ++k) carry ^= warp_parity[k];
+    if (!warp_row) {
+      if (lane == 0) warp_parity[wid] = (uint32_t)__popc(vote) & 1u;
+      __syncthreads();
+      for (int k = 0; k < wid; ++k) carry ^= warp_parity[k];
+    }
     for (int w = w0; w < w1; ++w) {
       const uint32_t b = mask[w];
       uint32_t m = b;
@@ -92,11 +134,12 @@ __global__ void __launch_bounds__(kRasterThreads)
       mask[w] = carry ? ~m : m;
       carry ^= (uint32_t)__popc(b) & 1u;
     }
-    __syncthreads();
-    int32_t *row = win + r * W;
-    for (int64_t c = tid; c < W; c += kRasterThreads)
+    PG_ROW_SYNC(warp_row);
+    int32_t *row = win + r * W + c0;
+    const int n = c1 >= c0 ? (int)(c1 - c0 + 1) : 0;
+    for (int c = gt; c < n; c += gn)
       if ((mask[c >> 5] >> (c & 31)) & 1u) atomicMax(row + c, p.feature);
-    __syncthreads();  // the mask is reused by the next row
+    PG_ROW_SYNC(warp_row);  // the mask is reused by the next row
   }
 }
 
