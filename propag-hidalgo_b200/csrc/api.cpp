@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -272,6 +273,40 @@ extern "C" void propag_engine_destroy(propag_engine *e) {
   cudaGetLastError();  // leave no error of the teardown to the caller's next CUDA call
 }
 
+// CTAs of a group-mode team for a batch on `ctas` co-resident CTAs.  Jobs go to
+// the teams largest first, each to the team that is free first, so the number
+// of teams decides between many jobs at once on few CTAs each and few at once
+// on many.  A job of s x s cells takes about 8.2 us x s on any team (its sweeps,
+// each a chain of latencies) plus 0.229 us x s^2 / R on R CTAs (measured on
+// 1024^2 members in teams of 2 to 74 CTAs: 8.4 ms + 240 ms / R); the number of
+// teams with the shortest batch by that estimate is taken.  Measured, 32 uneven
+// scenarios of 128^2 to 2048^2: 109 ms in 32 teams of 4, 44 ms in 8 of 18; 64
+// members of 1024^2: 168 in 37 teams of 4, 142 in 16 of 9; 256 members of 512^2
+// keep 37 teams of 4 (105; 123 in 16 of 9).
+static int team_size(const std::vector<JobDev> &jobs, int ctas) {
+  std::vector<double> side(jobs.size());
+  for (size_t i = 0; i < jobs.size(); ++i) side[i] = std::sqrt((double)jobs[i].W * (double)jobs[i].H);
+  std::sort(side.begin(), side.end(), std::greater<double>());
+  int best = ctas;
+  double best_us = 0.0;
+  for (int teams : {1, 2, 3, 4, 6, 8, 12, 16, 24, 37, 49, 74}) {
+    if (teams > 1 && ((size_t)teams > jobs.size() || ctas / teams < 2)) break;
+    const int R = ctas / teams;
+    std::vector<double> ends((size_t)teams, 0.0);  // a min-heap of the teams' finishing times
+    for (double s : side) {
+      std::pop_heap(ends.begin(), ends.end(), std::greater<double>());
+      ends.back() += 8.2 * s + 0.229 * s * s / R;
+      std::push_heap(ends.begin(), ends.end(), std::greater<double>());
+    }
+    const double us = *std::max_element(ends.begin(), ends.end());
+    if (teams == 1 || us < best_us) {
+      best_us = us;
+      best = R;
+    }
+  }
+  return std::max(best, 2);
+}
+
 static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, cudaStream_t stream,
                       PropagStats *stats) {
   if (!e) return fail(PROPAG_ERR_INVALID, "null engine");
@@ -342,16 +377,13 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
   auto fits = [&](uint32_t i, int c) { return smem_bytes(tw[i], th[i], c) <= budget; };
   int csize = e->csize;
   if (csize == 0 && e->auto_groups) {
-    // Group mode, one team per job of max(4, CTAs / jobs) CTAs.  A scenario
-    // runs on one cluster at most in cluster mode (its tiles go one after
-    // another), so few scenarios leave most SMs idle, while a group-mode team
-    // spreads each sweep over its CTAs with one barrier per sweep.  Measured
-    // on B200, 1024^2 ensemble members: 1 member 79 ms in group mode against
-    // 120 ms on a 16-CTA cluster; 64 members 408 ms (teams of 8) against
-    // 514 (8-CTA clusters); 256 members 1 082 ms (teams of 4) against 1 531.
+    // Group mode.  A scenario runs on one cluster at most in cluster mode (its
+    // tiles go one after another), so few scenarios leave most SMs idle, while
+    // a group-mode team spreads each sweep over its CTAs with one barrier per
+    // sweep.
     int ctas = 0;
     CK(engine_max_clusters(1, e->threads, global_tile_smem(e->threads), arith, true, &ctas));
-    if (ctas >= 8) csize = -std::max(4, ctas / (int)std::max<uint32_t>(n_jobs, 1));
+    if (ctas >= 8) csize = -team_size(jd, ctas);
   }
   if (csize == 0) {
     // among the cluster sizes that hold every job's tile, the one that runs
