@@ -198,7 +198,7 @@ void build_catalog64(FuelModel64 out[kMaxFuels]) {
   }
 }
 
-void build_catalog_table(FuelConst out[kMaxFuels]) {
+bool build_catalog_table(FuelConst out[kMaxFuels]) {
   FuelModel64 m[kMaxFuels];
   build_catalog64(m);
   for (int i = 0; i < kMaxFuels; ++i) {
@@ -209,18 +209,19 @@ void build_catalog_table(FuelConst out[kMaxFuels]) {
     c.has_fire = 1.0f;
     c.has_live = f.has_live ? 1.0f : 0.0f;
     c.R0 = (float)f.R0;
-    auto split = [](double v, float &hi, float &lo) {
-      hi = (float)v;
-      lo = (float)(v - (double)hi);
-    };
-    for (int k = 0; k < kMoistureClasses; ++k) {
-      c.R[k] = (float)f.R[k];
-      split(f.A[k], c.A[k], c.A_lo[k]);
-      split(f.B[k], c.B[k], c.B_lo[k]);
-      split(f.LM[k], c.LM[k], c.LM_lo[k]);
+    for (int k = 0; k < kMoistureClasses; ++k) c.R[k] = (float)f.R[k];
+    for (int k = kD1; k <= kD100; ++k) {
+      c.A[k] = f.A[k];
+      c.LM[k] = f.LM[k];
+      if (f.B[k] != 0.0) return false;
     }
-    split(f.LM0, c.LM0, c.LM0_lo);
-    split(f.mext, c.mext, c.mext_lo);
+    for (int k = kHerb; k <= kWood; ++k) {
+      c.B[k - kHerb] = f.B[k];
+      if (f.A[k] != 0.0 || f.LM[k] != 0.0) return false;
+    }
+    c.LM0 = f.LM0;
+    c.mext = f.mext;
+    c.inv_mext = (float)(1.0 / f.mext);
     c.rx_alive = (float)f.rx_alive;
     c.rx_dead = (float)f.rx_dead;
     c.flux_ratio = (float)f.flux_ratio;
@@ -231,6 +232,7 @@ void build_catalog_table(FuelConst out[kMaxFuels]) {
     c.wind_k = (float)f.wind_k;
     c.residence_time = (float)f.residence_time;
   }
+  return true;
 }
 
 }  // namespace propag

@@ -4,7 +4,7 @@
 // time (crates/firelib/src/firelib.rs:554-979 over the catalog in
 // crates/firelib/src/lib.rs:126-268).  Here they are evaluated once on the
 // host in double precision and folded into per-moisture-class linear
-// coefficients, then rounded to float for the device table.
+// coefficients for the device table.
 #pragma once
 
 #include <cstdint>
@@ -17,33 +17,26 @@ constexpr int kCatalogFuels = 14;  // NoFuel + NFFL01..13
 // Moisture inputs in the order the kernel reads them.
 enum MoistureClass { kD1 = 0, kD10 = 1, kD100 = 2, kHerb = 3, kWood = 4, kMoistureClasses = 5 };
 
-// Device table entry (float).  Per cell, with m = (d1, d10, d100, herb, wood):
+// Device table entry.  Per cell, with m = (d1, d10, d100, herb, wood):
 //   rbqig      = R0 + sum R[k] m[k]          (fuel_bed_bulk_dens folded in)
-//   dead_moist = sum A[k] m[k]
-//   live_moist = sum B[k] m[k]
-//   live_mext  = LM0 - sum LM[k] m[k]        (before max(., mext))
-struct FuelConst {
-  float has_fire;  // 1 when the model has particles (Catalog::get)
-  float has_live;
-  float R0;
-  float R[kMoistureClasses];
-  float A[kMoistureClasses];
-  float B[kMoistureClasses];
-  float LM0;
-  float LM[kMoistureClasses];
-  float mext;
+//   dead_moist = sum A[k] m[k]               over the dead classes d1, d10, d100
+//   live_moist = sum B[k] m[kHerb + k]       over the live classes
+//   live_mext  = LM0 - sum LM[k] m[k]        (before max(., mext)), dead classes
+// The moisture sums are subtracted from the moisture of extinction, where
+// float would cancel: their coefficients are double.  The order groups what is
+// read together into 16-byte loads.
+struct alignas(16) FuelConst {
+  double A[3], mext;
+  double B[2];
+  double LM[3], LM0;
+  float R0, R[kMoistureClasses], inv_mext, has_live;
   float rx_alive, rx_dead;  // life_rx_factor
-  float flux_ratio, slope_k, wind_b, wind_b_inv, wind_e, wind_k;
+  float flux_ratio, slope_k, wind_k, wind_b, wind_b_inv, wind_e;
   float residence_time;  // min
-  // low parts of the double-float pairs used where the kernel subtracts
-  // nearly equal quantities (moisture vs moisture of extinction)
-  float A_lo[kMoistureClasses];
-  float B_lo[kMoistureClasses];
-  float LM_lo[kMoistureClasses];
-  float LM0_lo, mext_lo;
-  float pad[13];
+  float has_fire;        // 1 when the model has particles (Catalog::get)
+  float pad[2];
 };
-static_assert(sizeof(FuelConst) == 64 * 4, "FuelConst layout");
+static_assert(sizeof(FuelConst) == 40 * 4, "FuelConst layout");
 
 // Double-precision constants of one fuel model (imperial internal units, as
 // the reference keeps them).
@@ -61,7 +54,9 @@ struct FuelModel64 {
 };
 
 // Builds the catalog (indices 0..19; 14..19 and 0 have no fire).
+// build_catalog_table returns false when a coefficient that the table leaves
+// out (a live class's dead coefficient and the like) is not zero.
 void build_catalog64(FuelModel64 out[kMaxFuels]);
-void build_catalog_table(FuelConst out[kMaxFuels]);
+bool build_catalog_table(FuelConst out[kMaxFuels]);
 
 }  // namespace propag

@@ -68,52 +68,9 @@ struct FireOut {
       residence_time, byrams, flame;
 };
 
-// Double-float value hi + lo (|lo| <= ulp(hi) / 2).
-struct DF {
-  float hi, lo;
-};
-
-// Error-free sum of two floats (Knuth's two-sum).
-__device__ __forceinline__ DF two_sum(float a, float b) {
-  const float s = __fadd_rn(a, b);
-  const float bb = __fsub_rn(s, a);
-  const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-  return DF{s, e};
-}
-
-// sum_{k in [K0, K1)} (chi[k] + clo[k]) * m[k] as a double-float: exact
-// products (fma) and sums (two-sum), so that moisture sums keep ~2^-44
-// relative accuracy.  The catalog's dead-moisture and live-extinction
-// coefficients are zero for the live classes (3, 4) and the live-moisture
-// coefficients for the dead classes (0-2); zero terms leave hi and lo
-// unchanged, so summing only [K0, K1) gives the same bits.
-template <int K0, int K1>
-__device__ __forceinline__ DF dot_df(const float *chi, const float *clo, const float m[5]) {
-  float hi = 0.0f, lo = 0.0f;
-#pragma unroll
-  for (int k = K0; k < K1; ++k) {
-    const float p = __fmul_rn(chi[k], m[k]);
-    const float pe = __fmaf_rn(chi[k], m[k], -p);
-    const DF s = two_sum(hi, p);
-    hi = s.hi;
-    lo = __fadd_rn(lo, __fadd_rn(s.lo, __fmaf_rn(clo[k], m[k], pe)));
-  }
-  return two_sum(hi, lo);
-}
-
-__device__ __forceinline__ DF df_sub(DF a, DF b) {
-  const DF s = two_sum(a.hi, -b.hi);
-  return two_sum(s.hi, __fadd_rn(s.lo, __fsub_rn(a.lo, b.lo)));
-}
-
 // eta_m (firelib.rs:1060-1076) with rt = moist / mext, as
 // u (2.93 - 5.45 u + 3.52 u^2), u = 1 - rt = (mext - moist) / mext.
-__device__ __forceinline__ float eta_m(DF moist, DF mext) {
-  const DF d = df_sub(mext, moist);
-  if (!(d.hi > 0.0f)) return 0.0f;  // life_moist >= life_mext
-  const float u = __fdividef(d.hi + d.lo, mext.hi + mext.lo);  // 2 ulp; operands in [2^-126, 2^126]
-  return u * fmaf(u, fmaf(u, 3.52f, -5.45f), 2.93f);
-}
+__device__ __forceinline__ float eta_of(float u) { return u * fmaf(u, fmaf(u, 3.52f, -5.45f), 2.93f); }
 
 // x^y for x >= 0 (0^y = 0 for y > 0) as 2^(y log2 x): about 1e-6 relative
 // (|y log2 x| < 30 here), well inside the fields' 1e-5 budget, at a fraction
@@ -132,17 +89,18 @@ template <bool kFull>
 __device__ __forceinline__ void burn_cell(const FuelConst &F, const float m[5], float ws,
                                           float waz, float slope, float aspect, FireOut &o) {
   // rx_int_rbqig
-  const DF dead = dot_df<0, 3>(F.A, F.A_lo, m);
-  const DF live = dot_df<3, 5>(F.B, F.B_lo, m);
   const float rbqig = F.R0 + dot5(F.R, m);
-  const DF mext{F.mext, F.mext_lo};
-  const float eta_dead = eta_m(dead, mext);
-  DF live_mext{0.0f, 0.0f};
+  const double m0 = (double)m[0], m1 = (double)m[1], m2 = (double)m[2];
+  // mext - dead_moist; not positive: life_moist >= life_mext
+  const double dead = __fma_rn(-F.A[2], m2, __fma_rn(-F.A[1], m1, __fma_rn(-F.A[0], m0, F.mext)));
+  const float eta_dead = dead > 0.0 ? eta_of((float)dead * F.inv_mext) : 0.0f;
+  float eta_live = 0.0f;
   if (F.has_live != 0.0f) {
-    live_mext = df_sub(DF{F.LM0, F.LM0_lo}, dot_df<0, 3>(F.LM, F.LM_lo, m));
-    if (!(df_sub(live_mext, mext).hi > 0.0f)) live_mext = mext;  // max(live_mext, mext)
+    double lmext = __fma_rn(-F.LM[2], m2, __fma_rn(-F.LM[1], m1, __fma_rn(-F.LM[0], m0, F.LM0)));
+    if (!(lmext > F.mext)) lmext = F.mext;  // max(live_mext, mext)
+    const double live = __fma_rn(-F.B[1], (double)m[4], __fma_rn(-F.B[0], (double)m[3], lmext));
+    if (live > 0.0) eta_live = eta_of(__fdividef((float)live, (float)lmext));  // 2 ulp; operands in [2^-126, 2^126]
   }
-  const float eta_live = eta_m(live, live_mext);
   const float rx = fmaf(F.rx_alive, eta_live, F.rx_dead * eta_dead);
   const float speed0 = __fdividef(rx * F.flux_ratio, rbqig);
 
@@ -235,9 +193,10 @@ __device__ __forceinline__ void store_cell(const Outputs &out, Index i, const Fi
     if ((kFull || (k >= 4 && k <= 6)) && out.f[k]) out.f[k][i] = v[k];
 }
 
-// Shared-memory copy of the fuel table, rows kCatStride words apart (odd:
-// the same field of different models lies in different banks).
-constexpr int kCatStride = 65;
+// Shared-memory copy of the fuel table, rows kCatStride words apart: a
+// multiple of four (16-byte loads) whose quads 11 f mod 8 lie in different
+// banks for any eight models in a row.
+constexpr int kCatStride = 44;
 static_assert(sizeof(FuelConst) / 4 <= kCatStride, "a FuelConst fits a table row");
 
 __device__ __forceinline__ void load_catalog(float *cat) {
@@ -274,7 +233,7 @@ __device__ __forceinline__ void one_cell(const float *cat, const Inputs &in, con
 // address arithmetic), else uint64_t.
 template <bool kFull, typename Index>
 __global__ void __launch_bounds__(256) fire_kernel(Inputs in, Outputs out, Index first, Index n) {
-  __shared__ float cat[kMaxFuels * kCatStride];
+  __shared__ __align__(16) float cat[kMaxFuels * kCatStride];
   load_catalog(cat);
   const Index stride = (Index)gridDim.x * blockDim.x;
   for (Index i = first + (Index)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
@@ -291,7 +250,7 @@ __global__ void __launch_bounds__(256) fire_kernel(Inputs in, Outputs out, Index
 template <typename Index>
 __global__ void __launch_bounds__(256) fire_weather_kernel(DmoistIn win, int hour, int month,
                                                            Inputs in, Outputs out, Index n) {
-  __shared__ float cat[kMaxFuels * kCatStride];
+  __shared__ __align__(16) float cat[kMaxFuels * kCatStride];
   __shared__ DmoistTables T;
   load_dmoist_tables(T);
   load_catalog(cat);
@@ -340,16 +299,7 @@ static cudaError_t launch_fire_t(const Inputs &in, const Outputs &out, uint64_t 
 // ---- host-side launchers (called from api.cpp) ------------------------------
 cudaError_t upload_catalog() {
   FuelConst table[kMaxFuels];
-  build_catalog_table(table);
-  // the kernel's moisture sums skip the classes whose coefficients are zero
-  for (int f = 0; f < kMaxFuels; ++f) {
-    for (int k = kHerb; k <= kWood; ++k)
-      if (table[f].A[k] != 0.0f || table[f].A_lo[k] != 0.0f || table[f].LM[k] != 0.0f ||
-          table[f].LM_lo[k] != 0.0f)
-        return cudaErrorInvalidValue;
-    for (int k = kD1; k <= kD100; ++k)
-      if (table[f].B[k] != 0.0f || table[f].B_lo[k] != 0.0f) return cudaErrorInvalidValue;
-  }
+  if (!build_catalog_table(table)) return cudaErrorInvalidValue;
   return cudaMemcpyToSymbol(c_catalog, table, sizeof(table));
 }
 
