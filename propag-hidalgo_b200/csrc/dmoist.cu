@@ -6,11 +6,9 @@
 // weather; the 10-h class interpolates the 1-h values of the requested hour
 // and of hours 6 and 15, and the 100-h class does the same on the 10-h
 // values (lib.rs:109-127) -- so a cell reads the weather of three hours, not
-// 24.  The model's look-up tables are copied to shared memory per block
-// (per-lane indices would serialise constant-memory reads).  Float
-// operations follow the reference's order; this file is compiled without
-// FMA contraction, explicit __fmaf_rn where the portable arctangent uses
-// fused multiply-adds, so results equal the CPU restatement bit for bit.
+// 24.  Float operations follow the reference's order (dmoist_device.cuh); this
+// file is compiled without FMA contraction, explicit __fmaf_rn where fused
+// multiply-adds are meant, so results equal the CPU restatement bit for bit.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -23,13 +21,13 @@ __global__ void __launch_bounds__(256) dmoist_kernel(DmoistIn in, uint64_t n, in
                                                      float scale, float *__restrict__ d1,
                                                      float *__restrict__ d10,
                                                      float *__restrict__ d100) {
-  __shared__ DmoistTables T;
+  __shared__ DmoistShared T;
   load_dmoist_tables(T);
+  const DmoistRows rows = dmoist_rows(in, n, hour, month);
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
     float m1, m10, m100;
-    dmoist_cell(T, in, n, i, hour, month, __ldg(in.fuel + i), __ldg(in.slope + i), __ldg(in.aspect + i),
-                m1, m10, m100);
+    dmoist_cell(T, rows, i, __ldg(in.fuel + i), __ldg(in.slope + i), __ldg(in.aspect + i), m1, m10, m100);
     d1[i] = m1 * scale;
     d10[i] = m10 * scale;
     d100[i] = m100 * scale;

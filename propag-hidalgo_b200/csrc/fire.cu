@@ -12,24 +12,24 @@
 //
 // Layout and mapping: one cell per thread, grid-stride, so that every load
 // and store of a warp is one coalesced run (4 bytes per lane, 1 for the fuel
-// codes); the grid holds as many CTAs as are resident at once (one wave),
-// and 32-bit indices serve every grid below 2^32 cells.  Four cells per thread
-// with 128-bit loads measured slower (0.298 against 0.277 ms at 4096^2): the
-// pass is bound by instruction issue, and four inlined copies of the cell
-// code overflow the instruction cache.  The fuel table sits in shared memory
-// with a row stride of 65 words (20 models), so that the lanes of a warp that
-// read the same field of different models hit different banks.  Double-float
-// moisture sums measured faster here than FP64 ones (0.33-0.35 ms against
-// 0.35-0.36 ms at 4096^2).  Compiled without automatic multiply-add
+// codes); 32-bit indices serve every grid below 2^32 cells.  The pass is bound
+// by instruction issue (325 instructions a cell, 66-71 % of issue slots used;
+// 516 with double-float moisture sums and single-word table reads: 280 us at
+// 4096^2, 200 now).  Four cells per thread with 128-bit loads measured slower
+// (0.298 against 0.277 ms: four inlined copies of the cell code overflow the
+// instruction cache), and so did loading a cell's inputs while the cell before
+// it is computed (0.247 against 0.235 ms: 48 registers instead of 32 leave 40
+// warps per SM instead of 64).  The fuel table sits in shared memory, a row's
+// fields in the order they are read.  Compiled without automatic multiply-add
 // contraction, so that the 3-field and 10-field instantiations round alike
 // (contraction measured no faster).
 //
 // FP32 formulation.  The arithmetic is the reference's, rearranged where the
 // float evaluation of the literal formula loses accuracy against double:
 //   * the moisture sums are pre-folded per moisture class; the dead and live
-//     sums and the live extinction moisture are double-float (error-free
-//     products and sums), because they are subtracted from the moisture of
-//     extinction, where float cancellation would dominate the error;
+//     sums and the live extinction moisture are double (eight multiply-adds),
+//     because they are subtracted from the moisture of extinction, where float
+//     cancellation would dominate the error;
 //   * eta_m = 1 - 2.59 rt + 5.11 rt^2 - 3.52 rt^3 is evaluated in
 //     u = 1 - rt = (mext - moist) / mext as u (2.93 - 5.45 u + 3.52 u^2),
 //     the same cubic expanded at rt = 1 where it vanishes;
@@ -61,7 +61,9 @@ constexpr float kHpuaToSI = 11348.8125851319f;    // BTU/ft^2 -> J/m^2
 constexpr float kByramsToSI = 3459.15354330709f;  // BTU/ft/s -> W/m
 constexpr float kFootToM = 0.3048f;
 
-__constant__ FuelConst c_catalog[kMaxFuels];
+// The fuel table in global memory: every block copies it to shared memory with
+// coalesced loads (per-lane indices would serialise constant-memory reads).
+__device__ FuelConst d_catalog[kMaxFuels];
 
 struct FireOut {
   float rx_int, speed0, hpua, phi_eff_wind, speed_max, azimuth_max, eccentricity,
@@ -200,7 +202,7 @@ constexpr int kCatStride = 44;
 static_assert(sizeof(FuelConst) / 4 <= kCatStride, "a FuelConst fits a table row");
 
 __device__ __forceinline__ void load_catalog(float *cat) {
-  const float *src = reinterpret_cast<const float *>(c_catalog);
+  const float *src = reinterpret_cast<const float *>(d_catalog);
   constexpr int kWords = (int)(sizeof(FuelConst) / 4);
   for (int t = threadIdx.x; t < kMaxFuels * kWords; t += blockDim.x)
     cat[(t / kWords) * kCatStride + t % kWords] = src[t];
@@ -251,9 +253,10 @@ template <typename Index>
 __global__ void __launch_bounds__(256) fire_weather_kernel(DmoistIn win, int hour, int month,
                                                            Inputs in, Outputs out, Index n) {
   __shared__ __align__(16) float cat[kMaxFuels * kCatStride];
-  __shared__ DmoistTables T;
+  __shared__ DmoistShared T;
   load_dmoist_tables(T);
   load_catalog(cat);
+  const DmoistRows rows = dmoist_rows(win, (uint64_t)n, hour, month);
   const Index stride = (Index)gridDim.x * blockDim.x;
   for (Index i = (Index)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     const uint8_t code = __ldg(in.fuel + i);
@@ -261,7 +264,7 @@ __global__ void __launch_bounds__(256) fire_weather_kernel(DmoistIn win, int hou
     if (code < kMaxFuels && fuel_row(cat, code).has_fire != 0.0f) {
       const float slope = __ldg(in.slope + i), aspect = __ldg(in.aspect + i);
       float m1, m10, m100;
-      dmoist_cell(T, win, (uint64_t)n, (uint64_t)i, hour, month, code, slope, aspect, m1, m10, m100);
+      dmoist_cell(T, rows, i, code, slope, aspect, m1, m10, m100);
       const float m[5] = {m1 * 0.01f, m10 * 0.01f, m100 * 0.01f, __ldg(in.m[3] + i), __ldg(in.m[4] + i)};
       burn_cell<false>(fuel_row(cat, code), m, __ldg(in.ws + i), __ldg(in.waz + i), slope, aspect, o);
     }
@@ -278,11 +281,18 @@ static int ctas_per_sm(K kernel, int threads) {
   return n;
 }
 
-// one wave: as many CTAs as are resident at once, each striding over an
-// equal share (a second, partial wave would leave SMs idle at the end)
-static unsigned one_wave(uint64_t items, int threads, int sm_count, int per_sm) {
+// As many CTAs as are resident at once, each striding over an equal share: a
+// small grid's table copies and partial last wave would cost more than they
+// balance.  Up to four times as many when a thread still has eight cells to
+// compute: equal shares take unequal time (patches that do not burn, divergent
+// cells), and 4096^2 cells ran 229 us in one wave, with the SMs' warps active
+// 80 % of the time, 209 in four, 214 in sixteen; 1.9 M cells 45 us in one, 46 in
+// four, 52 in sixteen.
+static unsigned grid_for(uint64_t items, int threads, int sm_count, int per_sm) {
+  const uint64_t wave = (uint64_t)sm_count * (uint64_t)per_sm;
+  const uint64_t waves = items / (wave * (uint64_t)threads * 8);
+  const uint64_t cap = wave * (waves < 1 ? 1 : waves > 4 ? 4 : waves);
   uint64_t blocks = (items + threads - 1) / threads;
-  const uint64_t cap = (uint64_t)sm_count * (uint64_t)per_sm;
   if (blocks > cap) blocks = cap;
   return blocks ? (unsigned)blocks : 1u;
 }
@@ -291,7 +301,7 @@ template <bool kFull, typename Index>
 static cudaError_t launch_fire_t(const Inputs &in, const Outputs &out, uint64_t n, int sm_count,
                                  int threads, cudaStream_t stream) {
   auto k1 = fire_kernel<kFull, Index>;
-  k1<<<one_wave(n, threads, sm_count, ctas_per_sm(k1, threads)), threads, 0, stream>>>(in, out, (Index)0,
+  k1<<<grid_for(n, threads, sm_count, ctas_per_sm(k1, threads)), threads, 0, stream>>>(in, out, (Index)0,
                                                                                     (Index)n);
   return cudaGetLastError();
 }
@@ -300,7 +310,7 @@ static cudaError_t launch_fire_t(const Inputs &in, const Outputs &out, uint64_t 
 cudaError_t upload_catalog() {
   FuelConst table[kMaxFuels];
   if (!build_catalog_table(table)) return cudaErrorInvalidValue;
-  return cudaMemcpyToSymbol(c_catalog, table, sizeof(table));
+  return cudaMemcpyToSymbol(d_catalog, table, sizeof(table));
 }
 
 cudaError_t launch_fire(bool full, uint64_t n, const uint8_t *fuel, const float *const m[5],
@@ -312,8 +322,8 @@ cudaError_t launch_fire(bool full, uint64_t n, const uint8_t *fuel, const float 
   for (int k = 0; k < 10; ++k) out.f[k] = outs[k];
   if (n == 0) return cudaSuccess;
   const int threads = 256;
-  // 32-bit indices while the last index plus one grid stride stays below 2^32
-  const bool narrow = n + (uint64_t)sm_count * 8 * threads < (1ull << 32);
+  // 32-bit indices while the last index plus one grid stride (four waves) stays below 2^32
+  const bool narrow = n + 4 * (uint64_t)sm_count * 8 * threads < (1ull << 32);
   if (full)
     return narrow ? launch_fire_t<true, uint32_t>(in, out, n, sm_count, threads, stream)
                   : launch_fire_t<true, uint64_t>(in, out, n, sm_count, threads, stream);
@@ -335,14 +345,14 @@ cudaError_t launch_fire_weather(uint64_t n, int hour, int month, const float *t,
   out.f[5] = azimuth_max;
   out.f[6] = eccentricity;
   const int threads = 256;
-  const bool narrow = n + (uint64_t)sm_count * 8 * threads < (1ull << 32);
+  const bool narrow = n + 4 * (uint64_t)sm_count * 8 * threads < (1ull << 32);
   if (narrow) {
     auto k = fire_weather_kernel<uint32_t>;
-    k<<<one_wave(n, threads, sm_count, ctas_per_sm(k, threads)), threads, 0, stream>>>(
+    k<<<grid_for(n, threads, sm_count, ctas_per_sm(k, threads)), threads, 0, stream>>>(
         win, hour, month, in, out, (uint32_t)n);
   } else {
     auto k = fire_weather_kernel<uint64_t>;
-    k<<<one_wave(n, threads, sm_count, ctas_per_sm(k, threads)), threads, 0, stream>>>(
+    k<<<grid_for(n, threads, sm_count, ctas_per_sm(k, threads)), threads, 0, stream>>>(
         win, hour, month, in, out, (uint64_t)n);
   }
   return cudaGetLastError();
