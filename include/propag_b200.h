@@ -455,7 +455,7 @@ int64_t propag_rasterize_ignitions(const GeoReference *geo_ref, const FFITimeFea
  * to pixel space; the burning runs on the GPU with the same rules as the
  * host rasteriser above, and the rasters are bit-identical to its result.
  * All three are stream-ordered on `stream`; the device scratch they need is
- * allocated and released on that stream (cudaMallocAsync / cudaFreeAsync).
+ * allocated and released on that stream, from a pool that keeps up to 128 MiB.
  *
  * propag_rasterize_times_device writes the initial time raster of the
  * reference's rasterize_times (crates/propag/src/propag.rs:837-890):

@@ -30,11 +30,12 @@ struct Reader {
   }
   double f64(bool le) {
     if (!need(8)) return 0;
-    uint8_t b[8];
-    for (int i = 0; i < 8; ++i) b[i] = le ? p[at + i] : p[at + 7 - i];
+    uint64_t b;
+    std::memcpy(&b, p + at, 8);
+    if (!le) b = __builtin_bswap64(b);  // the host is little-endian
     at += 8;
     double v;
-    std::memcpy(&v, b, 8);
+    std::memcpy(&v, &b, 8);
     return v;
   }
 };
