@@ -12,6 +12,7 @@
 //   NFFL catalog                                        crates/firelib/src/lib.rs:126-268
 #include "catalog.hpp"
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -221,7 +222,15 @@ bool build_catalog_table(FuelConst out[kMaxFuels]) {
     }
     c.LM0 = f.LM0;
     c.mext = f.mext;
-    c.inv_mext = (float)(1.0 / f.mext);
+    c.mext_f = (float)f.mext;
+    // the sums' magnitudes, at most 2 mext and 2 (LM0 + mext), over 8 and 32; and
+    // for the choice of the larger of live_mext and mext far more than their error
+    const double live_size = std::fabs(f.LM0) + f.mext, differ = live_size * 0x1p-16;
+    c.dead_min = (float)(f.mext / 4.0);
+    c.dead_exact = f.A[kD1] == 1.0 && f.A[kD10] == 0.0 && f.A[kD100] == 0.0 && (double)(float)f.mext == f.mext ? 1.0f : 0.0f;
+    c.live_min = (float)(live_size / 16.0);
+    c.live_above = (float)std::max(f.mext + differ, live_size / 16.0);
+    c.live_below = (float)(f.mext - differ);
     c.rx_alive = (float)f.rx_alive;
     c.rx_dead = (float)f.rx_dead;
     c.flux_ratio = (float)f.flux_ratio;

@@ -29,14 +29,19 @@ struct alignas(16) FuelConst {
   double A[3], mext;
   double B[2];
   double LM[3], LM0;
-  float R0, R[kMoistureClasses], inv_mext, has_live;
+  float R0, R[kMoistureClasses], mext_f, has_live;
   float rx_alive, rx_dead;  // life_rx_factor
   float flux_ratio, slope_k, wind_k, wind_b, wind_b_inv, wind_e;
   float residence_time;  // min
   float has_fire;        // 1 when the model has particles (Catalog::get)
-  float pad[2];
+  // sizes below which a double moisture sum is not trusted to round as the
+  // double-float one does, and the range in which live_mext before max(., mext)
+  // is not (fire.cu)
+  float dead_min, live_min, live_above, live_below;
+  float mext_rcp;    // set by the kernels
+  float dead_exact;  // 1: the dead sum is exact in both
 };
-static_assert(sizeof(FuelConst) == 40 * 4, "FuelConst layout");
+static_assert(sizeof(FuelConst) == 44 * 4, "FuelConst layout");
 
 // Double-precision constants of one fuel model (imperial internal units, as
 // the reference keeps them).

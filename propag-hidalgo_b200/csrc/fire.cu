@@ -13,9 +13,9 @@
 // Layout and mapping: one cell per thread, grid-stride, so that every load
 // and store of a warp is one coalesced run (4 bytes per lane, 1 for the fuel
 // codes); 32-bit indices serve every grid below 2^32 cells.  The pass is bound
-// by instruction issue (325 instructions a cell, 66-71 % of issue slots used;
-// 516 with double-float moisture sums and single-word table reads: 280 us at
-// 4096^2, 200 now).  Four cells per thread with 128-bit loads measured slower
+// by instruction issue and the warps in flight (360 instructions a cell; 516
+// with double-float moisture sums for every cell and single-word table reads:
+// 280 us at 4096^2, 213 now).  Four cells per thread with 128-bit loads measured slower
 // (0.298 against 0.277 ms: four inlined copies of the cell code overflow the
 // instruction cache), and so did loading a cell's inputs while the cell before
 // it is computed (0.247 against 0.235 ms: 48 registers instead of 32 leave 40
@@ -27,9 +27,9 @@
 // FP32 formulation.  The arithmetic is the reference's, rearranged where the
 // float evaluation of the literal formula loses accuracy against double:
 //   * the moisture sums are pre-folded per moisture class; the dead and live
-//     sums and the live extinction moisture are double (eight multiply-adds),
-//     because they are subtracted from the moisture of extinction, where float
-//     cancellation would dominate the error;
+//     sums and the live extinction moisture have more than float precision
+//     (moist_sums), because they are subtracted from the moisture of
+//     extinction, where float cancellation would dominate the error;
 //   * eta_m = 1 - 2.59 rt + 5.11 rt^2 - 3.52 rt^3 is evaluated in
 //     u = 1 - rt = (mext - moist) / mext as u (2.93 - 5.45 u + 3.52 u^2),
 //     the same cubic expanded at rt = 1 where it vanishes;
@@ -46,6 +46,7 @@
 
 #include "catalog.hpp"
 #include "dmoist_device.cuh"
+#include "moist_sums.cuh"
 
 namespace propag {
 
@@ -92,17 +93,10 @@ __device__ __forceinline__ void burn_cell(const FuelConst &F, const float m[5], 
                                           float waz, float slope, float aspect, FireOut &o) {
   // rx_int_rbqig
   const float rbqig = F.R0 + dot5(F.R, m);
-  const double m0 = (double)m[0], m1 = (double)m[1], m2 = (double)m[2];
-  // mext - dead_moist; not positive: life_moist >= life_mext
-  const double dead = __fma_rn(-F.A[2], m2, __fma_rn(-F.A[1], m1, __fma_rn(-F.A[0], m0, F.mext)));
-  const float eta_dead = dead > 0.0 ? eta_of((float)dead * F.inv_mext) : 0.0f;
-  float eta_live = 0.0f;
-  if (F.has_live != 0.0f) {
-    double lmext = __fma_rn(-F.LM[2], m2, __fma_rn(-F.LM[1], m1, __fma_rn(-F.LM[0], m0, F.LM0)));
-    if (!(lmext > F.mext)) lmext = F.mext;  // max(live_mext, mext)
-    const double live = __fma_rn(-F.B[1], (double)m[4], __fma_rn(-F.B[0], (double)m[3], lmext));
-    if (live > 0.0) eta_live = eta_of(__fdividef((float)live, (float)lmext));  // 2 ulp; operands in [2^-126, 2^126]
-  }
+  const Moist w = moist_sums(F, m);
+  // not positive: life_moist >= life_mext.  2 ulp; operands in [2^-126, 2^126]
+  const float eta_dead = w.dead > 0.0f ? eta_of(w.dead * F.mext_rcp) : 0.0f;  // __fdividef(w.dead, mext), as below
+  const float eta_live = w.live > 0.0f ? eta_of(__fdividef(w.live, w.lmext)) : 0.0f;
   const float rx = fmaf(F.rx_alive, eta_live, F.rx_dead * eta_dead);
   const float speed0 = __fdividef(rx * F.flux_ratio, rbqig);
 
@@ -207,6 +201,12 @@ __device__ __forceinline__ void load_catalog(float *cat) {
   for (int t = threadIdx.x; t < kMaxFuels * kWords; t += blockDim.x)
     cat[(t / kWords) * kCatStride + t % kWords] = src[t];
   __syncthreads();
+  // the reciprocal that the fast division by mext multiplies with
+  if (threadIdx.x < kMaxFuels) {
+    FuelConst *const f = reinterpret_cast<FuelConst *>(cat + threadIdx.x * kCatStride);
+    f->mext_rcp = __fdividef(1.0f, f->mext_f);
+  }
+  __syncthreads();
 }
 
 __device__ __forceinline__ const FuelConst &fuel_row(const float *cat, uint32_t code) {
@@ -232,9 +232,10 @@ __device__ __forceinline__ void one_cell(const float *cat, const Inputs &in, con
 // the three the propagation needs (the shared fields are the same
 // operations, so both give the same values for them).
 // Index: uint32_t when n + the grid's threads fit in 32 bits (cheaper
-// address arithmetic), else uint64_t.
+// address arithmetic), else uint64_t.  Six CTAs an SM: 40 registers (44 to 47
+// without the bound: 240 us against 225 at 4096^2; 32 for eight CTAs: 230).
 template <bool kFull, typename Index>
-__global__ void __launch_bounds__(256) fire_kernel(Inputs in, Outputs out, Index first, Index n) {
+__global__ void __launch_bounds__(256, 6) fire_kernel(Inputs in, Outputs out, Index first, Index n) {
   __shared__ __align__(16) float cat[kMaxFuels * kCatStride];
   load_catalog(cat);
   const Index stride = (Index)gridDim.x * blockDim.x;
