@@ -33,8 +33,13 @@ cudaError_t launch_fire(bool full, uint64_t n, const uint8_t *fuel, const float 
                         const float *aspect, float *const outs[10], int sm_count,
                         cudaStream_t stream);
 cudaError_t launch_prep(const JobDev *jobs, uint32_t n_jobs, uint64_t max_cells, int sms,
-                        cudaStream_t stream);
-cudaError_t launch_ignite(const JobDev *jobs, uint32_t n_jobs, cudaStream_t stream);
+                        const uint32_t *only_if, cudaStream_t stream);
+cudaError_t launch_ignite(const JobDev *jobs, uint32_t n_jobs, const uint32_t *only_if,
+                          cudaStream_t stream);
+cudaError_t waves_max_ctas(int threads, size_t smem, int arith, int *n);
+cudaError_t launch_waves(const JobDev *job, const SlotDev *slots, uint32_t teams, uint32_t group, int threads,
+                         size_t smem, uint32_t *err, StatsDev *stats, const WaveDev &w, uint32_t *redo, int arith,
+                         cudaStream_t stream);
 cudaError_t launch_engine(const JobDev *jobs, uint32_t n_jobs, const SlotDev *slots,
                           uint32_t n_slots, int csize, int threads, size_t smem, uint32_t *queue,
                           StatsDev *stats, unsigned long long max_sweeps, const uint32_t *order,
@@ -188,13 +193,14 @@ size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 // Sweeps a job may take before it stops with the sweep-limit status: 2^40
 // (no real scenario comes near), or PROPAG_MAX_SWEEPS from the environment
 // (used by the tests to make the limit run out).
+constexpr unsigned long long kMaxSweeps = 1ull << 40;
 unsigned long long max_sweeps() {
   const char *v = std::getenv("PROPAG_MAX_SWEEPS");
   if (v && *v) {
     const unsigned long long n = std::strtoull(v, nullptr, 10);
     if (n > 0) return n;
   }
-  return 1ull << 40;
+  return kMaxSweeps;
 }
 
 bool valid_size(uint32_t w, uint32_t h) { return w >= 1 && h >= 1 && w <= 65534 && h <= 65534; }
@@ -355,6 +361,32 @@ static int team_size(const std::vector<JobDev> &jobs, int ctas) {
   return std::max(best, 2);
 }
 
+// Several teams on one job (WaveDev in engine.cuh): how many, and the window
+// within which launches keep their sequence; no teams when the job has too few
+// tiles to run any of them at once.  A window of one tile of at least 257
+// cells, two of 129, three of 86 holds every reference of up to 256 cells'
+// offset: the longest lines of sight of the hilly and ridged scenarios are 160
+// to 218 steps, and a job with a longer one is run twice.  The number of teams
+// is what a simulation of the schedule with measured sweep times favours (in
+// sequence / 2 / 3 / 4 / 6 teams; 4096^2 with 20 ignitions: 478 / 265 / 208 / 186 /
+// 212 ms; 2048^2 with 20: 103 / 58 / 53 / 59 / 71, with one: 49 / 33 / 35 / 37 /
+// 45).
+struct WavePlan {
+  uint32_t teams = 0;
+  int window = 0;
+};
+static WavePlan wave_plan(const JobDev &j) {
+  WavePlan p;
+  const uint64_t tiles = (uint64_t)j.TX * (uint64_t)j.TY;
+  const int window = j.T >= 257 ? 1 : j.T >= 129 ? 2 : 3;
+  if (j.T < 86 || tiles > kWaveTiles || std::max(j.TX, j.TY) < 2 * window + 2 ||
+      (uint64_t)j.W * (uint64_t)j.H >= (1ull << 27))
+    return p;
+  p.window = window;
+  p.teams = j.n_ignitions < 2 ? 2 : tiles >= 100 ? 4 : 3;
+  return p;
+}
+
 static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, cudaStream_t stream,
                       PropagStats *stats) {
   if (!e) return fail(PROPAG_ERR_INVALID, "null engine");
@@ -464,7 +496,8 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
     }
   }
   size_t smem = 0, tn_max = 1, ovf_cap = 0;
-  uint32_t n_slots = 0, group = 0;
+  uint32_t n_slots = 0, group = 0, wave_group = 0;
+  WavePlan waves;
   if (csize <= PROPAG_CLUSTER_GROUPS) {
     // group mode: the co-resident CTAs split into teams of at least 32 CTAs
     // (or of -csize CTAs when given), one team per job up to that, tiles in
@@ -479,6 +512,13 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
     for (uint32_t i = 0; i < n_jobs; ++i) {
       jd[i].smem_tile = kSmemTileGlobal;
       tn_max = std::max<size_t>(tn_max, (size_t)tw[i] * (size_t)th[i]);
+    }
+    if (n_jobs == 1 && e->csize == 0 && !e->phantom && max_sweeps() == kMaxSweeps) {
+      waves = wave_plan(jd[0]);
+      int wave_ctas = 0;
+      if (waves.teams) CK(waves_max_ctas(e->threads, smem, arith, &wave_ctas));
+      wave_group = waves.teams ? (uint32_t)wave_ctas / waves.teams : 0;
+      if (wave_group < 8) waves = WavePlan{};
     }
     csize = 1;
   } else {
@@ -538,20 +578,26 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
   // global-memory tiles: each CTA of a team has its own words of the dirty
   // bitmap and its own update region
   const size_t team_ctas = group ? group : (size_t)csize;
-  const size_t words_max = (size_t)owner_words((uint32_t)tn_max, (uint32_t)team_ctas) * team_ctas;
+  size_t words_max = (size_t)owner_words((uint32_t)tn_max, (uint32_t)team_ctas) * team_ctas;
+  // waves: a slot per team, then the slot of a second start in sequence
+  const uint32_t first_slot = waves.teams, all_slots = waves.teams + n_slots;
+  if (waves.teams)
+    words_max = std::max(words_max, (size_t)owner_words((uint32_t)tn_max, wave_group) * wave_group);
   const size_t upd_max = words_max * 32;
   const size_t ovf_list_bytes = align_up((size_t)csize * ovf_cap * 2, 256);
   const size_t ovf_upd_bytes = align_up((size_t)csize * ovf_cap * sizeof(Update), 256);
   // two dirty bitmaps (alternating) and two update arrays (by sweep parity)
   const size_t slot_bytes = 2 * align_up(words_max * 4, 256) + 2 * align_up(upd_max * sizeof(TileUpdate), 256) +
                             256 + ovf_list_bytes + ovf_upd_bytes;
-  CK(e->slot_scratch.reserve(slot_bytes * n_slots, stream));
+  CK(e->slot_scratch.reserve(slot_bytes * all_slots, stream));
   // meta: jobs, slots, stats, queue
   const size_t meta_jobs = align_up(sizeof(JobDev) * n_jobs, 256);
-  const size_t meta_slots = align_up(sizeof(SlotDev) * n_slots, 256);
+  const size_t meta_slots = align_up(sizeof(SlotDev) * all_slots, 256);
   const size_t meta_stats = align_up(sizeof(StatsDev) * n_jobs, 256);
   const size_t meta_order = align_up(sizeof(uint32_t) * n_jobs, 256);
-  CK(e->meta.reserve(meta_jobs + meta_slots + meta_stats + 256 + meta_order, stream));
+  const uint64_t tiles = (uint64_t)jd[0].TX * (uint64_t)jd[0].TY;
+  const size_t wave_words = waves.teams ? 64 + 2 * align_up(tiles, 64) + 2 * align_up(kWaveRounds, 64) : 0;
+  CK(e->meta.reserve(meta_jobs + meta_slots + meta_stats + 256 + meta_order + wave_words * 4, stream));
   // staging buffers (pinned) may still be read by the previous run's copies
   // (a run being captured into a graph follows a completed uncaptured run)
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
@@ -563,10 +609,10 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
     CK(cudaMallocHost(&e->jobs_pinned, sizeof(JobDev) * n_jobs + sizeof(uint32_t) * n_jobs));
     e->pinned_jobs = n_jobs;
   }
-  if (e->pinned_slots < n_slots) {
+  if (e->pinned_slots < all_slots) {
     if (e->slots_pinned) cudaFreeHost(e->slots_pinned);
-    CK(cudaMallocHost(&e->slots_pinned, sizeof(SlotDev) * n_slots));
-    e->pinned_slots = n_slots;
+    CK(cudaMallocHost(&e->slots_pinned, sizeof(SlotDev) * all_slots));
+    e->pinned_slots = all_slots;
   }
   std::copy(jd.begin(), jd.end(), e->jobs_pinned);
   // queue order: largest grids first, so that the longest jobs start first
@@ -576,7 +622,7 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
   std::stable_sort(order_pinned, order_pinned + n_jobs, [&](uint32_t a, uint32_t b) {
     return (uint64_t)jd[a].W * jd[a].H > (uint64_t)jd[b].W * jd[b].H;
   });
-  for (uint32_t s = 0; s < n_slots; ++s) {
+  for (uint32_t s = 0; s < all_slots; ++s) {
     size_t o = slot_bytes * s;
     SlotDev &sd = e->slots_pinned[s];
     sd.dirty = e->slot_scratch.at<uint32_t>(o);
@@ -604,20 +650,39 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
   e->last_stats = d_stats;
   CK(cudaMemcpyAsync(d_jobs, e->jobs_pinned, sizeof(JobDev) * n_jobs, cudaMemcpyHostToDevice, stream));
   CK(cudaMemcpyAsync(d_order, order_pinned, sizeof(uint32_t) * n_jobs, cudaMemcpyHostToDevice, stream));
-  CK(cudaMemcpyAsync(d_slots, e->slots_pinned, sizeof(SlotDev) * n_slots, cudaMemcpyHostToDevice, stream));
+  CK(cudaMemcpyAsync(d_slots, e->slots_pinned, sizeof(SlotDev) * all_slots, cudaMemcpyHostToDevice, stream));
   // the engine's events time uncaptured runs only (an event recorded into a
   // graph cannot be waited on or timed from the host)
   const bool live = capturing == cudaStreamCaptureStatusNone;
   if (live) CK(cudaEventRecord(e->staged, stream));
   CK(cudaMemsetAsync(d_stats, 0, sizeof(StatsDev) * n_jobs, stream));
-  CK(cudaMemsetAsync(d_queue, 0, 8, stream));  // queue position, group error flag
+  CK(cudaMemsetAsync(d_queue, 0, 16, stream));  // queue position, group error flag (two launches of a waves run)
+  WaveDev wave{};
+  if (waves.teams) {
+    uint32_t *words = e->meta.at<uint32_t>(meta_jobs + meta_slots + meta_stats + 256 + meta_order);
+    CK(cudaMemsetAsync(words, 0, wave_words * 4, stream));
+    wave.far = words;
+    wave.done = words + 64;
+    wave.claim = wave.done + align_up(tiles, 64);
+    wave.worked = wave.claim + align_up(tiles, 64);
+    wave.sweeps = wave.worked + align_up(kWaveRounds, 64);
+    wave.tiles = (uint32_t)tiles;
+    wave.window = waves.window;
+  }
   // ---- kernels ----
   if (live) CK(cudaEventRecord(e->ev[0], stream));
-  CK(launch_prep(d_jobs, n_jobs, max_cells, e->sms, stream));
-  CK(launch_ignite(d_jobs, n_jobs, stream));
+  CK(launch_prep(d_jobs, n_jobs, max_cells, e->sms, nullptr, stream));
+  CK(launch_ignite(d_jobs, n_jobs, nullptr, stream));
   if (live) CK(cudaEventRecord(e->ev[1], stream));
-  CK(launch_engine(d_jobs, n_jobs, d_slots, n_slots, csize, e->threads, smem, d_queue, d_stats,
-                   max_sweeps(), d_order, group, group ? e->phantom : 0u, arith, stream));
+  if (waves.teams) {
+    CK(launch_waves(d_jobs, d_slots, waves.teams, wave_group, e->threads, smem, d_queue + 1, d_stats, wave,
+                    d_queue + 2, arith, stream));
+    // these do nothing unless the waves found the job's launches dependent
+    CK(launch_prep(d_jobs, n_jobs, max_cells, e->sms, wave.far, stream));
+    CK(launch_ignite(d_jobs, n_jobs, wave.far, stream));
+  }
+  CK(launch_engine(d_jobs, n_jobs, d_slots + first_slot, n_slots, csize, e->threads, smem,
+                   waves.teams ? d_queue + 2 : d_queue, d_stats, max_sweeps(), d_order, group, group ? e->phantom : 0u, arith, stream));
   if (live) CK(cudaEventRecord(e->ev[2], stream));
   CK(launch_post(d_jobs, n_jobs, max_cells, e->sms, d_stats, stream));
   if (live) CK(cudaEventRecord(e->ev[3], stream));
@@ -1036,8 +1101,8 @@ extern "C" int propag_run_device_static(const PropagJob *job, void *stream_ptr, 
   uint32_t *d_queue = reinterpret_cast<uint32_t *>(base + kStaticQueueOff);
   cudaStream_t stream = (cudaStream_t)stream_ptr;
   CK(launch_stage_static(d_job, d, d_slot, s, d_stats, d_queue, stream));
-  CK(launch_prep(d_job, 1, N, sms, stream));
-  CK(launch_ignite(d_job, 1, stream));
+  CK(launch_prep(d_job, 1, N, sms, nullptr, stream));
+  CK(launch_ignite(d_job, 1, nullptr, stream));
   CK(launch_engine(d_job, 1, d_slot, 1, csize, engine_threads(), smem, d_queue, d_stats, max_sweeps(),
                    nullptr, 0u, 0u, d.refm, stream));
   CK(launch_post(d_job, 1, N, sms, d_stats, stream));

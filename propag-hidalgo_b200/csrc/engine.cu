@@ -95,7 +95,11 @@ __device__ __forceinline__ float dir_inv_speed(const DirConst &dc, int k, const 
 // Boundary bits (find_boundaries) packed with a warp ballot, plus the initial
 // state: time = FLT_MAX, no reference, empty referrer boxes; and the
 // reciprocal direct-spread speeds toward the 8 neighbours (when the job has them).
-__global__ void __launch_bounds__(256) prep_kernel(const JobDev *__restrict__ jobs) {
+// only_if: when given and zero, nothing is done (a second start of a job that
+// turned out not to need one).
+__global__ void __launch_bounds__(256) prep_kernel(const JobDev *__restrict__ jobs,
+                                                   const uint32_t *__restrict__ only_if) {
+  if (only_if && *only_if == 0u) return;
   const JobDev j = jobs[blockIdx.y];
   __shared__ DirConst dc;
   if (threadIdx.x == 0) dir_consts(j, dc);
@@ -153,7 +157,8 @@ __global__ void __launch_bounds__(256) prep_kernel(const JobDev *__restrict__ jo
 // Later ignitions overwrite earlier ones in the same cell (GDAL burn order);
 // every cell whose time is not f32::MAX references itself
 // (crates/propag/src/propag.rs:441-449).
-__global__ void ignite_kernel(const JobDev *__restrict__ jobs) {
+__global__ void ignite_kernel(const JobDev *__restrict__ jobs, const uint32_t *__restrict__ only_if) {
+  if (only_if && *only_if == 0u) return;
   const JobDev j = jobs[blockIdx.x];
   if (threadIdx.x != 0) return;
   struct Ign {
@@ -1056,10 +1061,15 @@ __device__ __forceinline__ uint32_t walk_los(const uint32_t *__restrict__ bnd, c
 // scans read referrers outside the launching tile too, from X[p]: a launch
 // writes only its tile's cells, and both copies agree everywhere when a
 // launch ends, so outside the tile X[0] and X[1] hold the same state.
-template <int kArith, bool kGroup>
+// kWaves: other teams run launches of other tiles of the job at the same time;
+// reach is the largest offset (in cells, per axis) of a reference for which
+// their launches and this one are independent, and *far is set when a cell
+// adopts one further away.
+template <int kArith, bool kGroup, bool kWaves>
 __device__ __forceinline__ bool tile_global(const JobDev &j, const DirConst &dc, const SlotDev &s, const TileDesc &td,
                             uint32_t *list, TileUpdate *sm_upd, uint32_t *cta_ctr, ScanItem *queue, const float *cross,
-                            uint32_t rank, uint32_t R, SweepCtx &cx, Team<kGroup> &team) {
+                            uint32_t rank, uint32_t R, SweepCtx &cx, Team<kGroup> &team, int reach,
+                            uint32_t *far) {
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const uint32_t k8 = lane & 7u, g0 = lane & 24u;
   const int x0 = td.x0, y0 = td.y0, TW = td.TW, TH = td.TH;
@@ -1217,6 +1227,7 @@ __device__ __forceinline__ bool tile_global(const JobDev &j, const DirConst &dc,
           if (k8 == 0) {
             st_state(ws + c, CellState{b.time, b.ref, los, 0u});
             const CellState e{b.time, b.ref, los, k};
+            if (kWaves && max(abs(ref_x(b.ref) - x), abs(ref_y(b.ref) - y)) > reach) *far = 1u;
             if (ai < (uint32_t)kTileUpdSmem)
               supd[ai] = e;
             else
@@ -1710,6 +1721,36 @@ __device__ bool tile_smem(const JobDev &j, const DirConst &dc, char *smem, const
 }
 
 // ================================================================ engine ====
+// Accumulated crossing times of the line-of-sight walks (dda_columns.cuh).
+__device__ __forceinline__ void fill_cross(float *cross) {
+  for (int n = 1 + (int)threadIdx.x; n <= kColumnsMax; n += blockDim.x) {
+    const float step = __frcp_rn((float)n);
+    float t = step;
+    for (int i = 1; i <= n; ++i, t = __fadd_rn(t, step)) cross[cross_at(n, i)] = t;
+  }
+}
+
+// A warp's counters into the job's statistics.  Called by all 32 lanes.
+__device__ __forceinline__ void add_counters(Counters &cnt, StatsDev *st, uint32_t lane) {
+  unsigned long long evals = cnt.evals, scans = cnt.scans, scan_cells = cnt.scan_cells;
+  for (int o = 16; o > 0; o >>= 1) {
+    cnt.dda += __shfl_xor_sync(kFull, cnt.dda, o);
+    cnt.gat += __shfl_xor_sync(kFull, cnt.gat, o);
+    cnt.walk_max = max(cnt.walk_max, __shfl_xor_sync(kFull, cnt.walk_max, o));
+    scans += __shfl_xor_sync(kFull, scans, o);
+    scan_cells += __shfl_xor_sync(kFull, scan_cells, o);
+    evals += __shfl_xor_sync(kFull, evals, o);
+  }
+  if (lane == 0) {
+    if (cnt.dda) atomicAdd(&st->dda_steps, (unsigned long long)cnt.dda);
+    if (cnt.gat) atomicAdd(&st->gathers, (unsigned long long)cnt.gat);
+    if (scans) atomicAdd(&st->refbox_scans, scans);
+    if (scan_cells) atomicAdd(&st->scan_cells, scan_cells);
+    if (evals) atomicAdd(&st->evaluations, evals);
+    if (cnt.walk_max) atomicMax(&st->max_walk, cnt.walk_max);
+  }
+}
+
 // Cluster mode (group == 0): every cluster is one team.  Group mode
 // (group = G > 1, launched cooperatively without clusters): CTAs
 // [g * G, (g + 1) * G) form team g, which keeps its tiles in global memory
@@ -1758,12 +1799,7 @@ __global__ void __launch_bounds__(kEngineThreads, 1)
     const JobDev &j = js;  // shared-memory copy: frees registers
     // accumulated crossing times of the line-of-sight walks (a shared-memory
     // tile of another job may have used the space since the last time)
-    if (j.smem_tile == kSmemTileGlobal)
-      for (int n = 1 + (int)threadIdx.x; n <= kColumnsMax; n += blockDim.x) {
-        const float step = __frcp_rn((float)n);
-        float t = step;
-        for (int i = 1; i <= n; ++i, t = __fadd_rn(t, step)) cross[cross_at(n, i)] = t;
-      }
+    if (j.smem_tile == kSmemTileGlobal) fill_cross(cross);
     StatsDev *st = stats + jid;
     if (tid == 0) st->t_start_ns = globaltimer_ns();
     SweepCtx cx;
@@ -1789,33 +1825,16 @@ __global__ void __launch_bounds__(kEngineThreads, 1)
             w = tile_smem<BoxCoarse, kArith>(j, dc, dyn_smem, s, td, scan_boxes, cx, team);
         }
         if (kGroup || j.smem_tile == kSmemTileGlobal)
-          w = tile_global<kArith, kGroup>(
+          w = tile_global<kArith, kGroup, false>(
               j, dc, s, td, reinterpret_cast<uint32_t *>(dyn_smem),
               reinterpret_cast<TileUpdate *>(dyn_smem + global_tile_list_bytes(blockDim.x)), cta_ctr,
-              reinterpret_cast<ScanItem *>(scan_boxes), cross, rank, csize, cx, team);
+              reinterpret_cast<ScanItem *>(scan_boxes), cross, rank, csize, cx, team, 0, nullptr);
         round_worked |= w;
       }
       if (!round_worked || cx.abort) break;
     }
     // per-job statistics
-    Counters &cnt = cx.cnt;
-    unsigned long long evals = cnt.evals, scans = cnt.scans, scan_cells = cnt.scan_cells;
-    for (int o = 16; o > 0; o >>= 1) {
-      cnt.dda += __shfl_xor_sync(kFull, cnt.dda, o);
-      cnt.gat += __shfl_xor_sync(kFull, cnt.gat, o);
-      cnt.walk_max = max(cnt.walk_max, __shfl_xor_sync(kFull, cnt.walk_max, o));
-      scans += __shfl_xor_sync(kFull, scans, o);
-      scan_cells += __shfl_xor_sync(kFull, scan_cells, o);
-      evals += __shfl_xor_sync(kFull, evals, o);
-    }
-    if (lane == 0) {
-      if (cnt.dda) atomicAdd(&st->dda_steps, (unsigned long long)cnt.dda);
-      if (cnt.gat) atomicAdd(&st->gathers, (unsigned long long)cnt.gat);
-      if (scans) atomicAdd(&st->refbox_scans, scans);
-      if (scan_cells) atomicAdd(&st->scan_cells, scan_cells);
-      if (evals) atomicAdd(&st->evaluations, evals);
-      if (cnt.walk_max) atomicMax(&st->max_walk, cnt.walk_max);
-    }
+    add_counters(cx.cnt, st, lane);
     // every CTA's own improvements (global-memory tiles), or the cluster's
     // total counted by its leader (shared-memory tiles)
     if (threadIdx.x == 0 && cx.improvements) atomicAdd(&st->improvements, cx.improvements);
@@ -1839,6 +1858,194 @@ __global__ void __launch_bounds__(kEngineThreads, 1)
     for (uint32_t q = taken; q < n_jobs; q = atomicAdd(queue, 1u))
       stats[order ? __ldg(order + q) : q].status = kStatusGroupTimeout;
   }
+}
+
+// ================================================================= waves ====
+// One job by several teams.  The reference runs the launches one after
+// another: rounds of all tiles in row-major order.  Launches of tiles more than
+// `window` tiles apart are independent as long as no reference lies more than
+// window * T - 1 cells from its cell (per axis): a launch reads and marks cells
+// within that many cells of its own tile's border, plus one, and the tiles in
+// between are window * T cells wide.  So a launch (round r, tile t) may run as
+// soon as, within the window, the tiles ahead of t have finished round r and
+// those behind it round r - 1, and round r is known to take place (a launch of
+// round r - 1 improved a cell).  Every launch then reads what it reads in
+// sequence: times, references and all work counts are the same.  A cell that
+// adopts a reference further away than that sets *far: the teams stop, and the
+// job is started again, its launches in sequence (wave_end_kernel).
+//
+// Why: a sweep is a chain of latencies whose length hardly depends on the CTAs
+// that share it, and one tile's front is too small for 148 of them.  4096^2, 20
+// ignitions: 381 ms in sequence, 168 ms with four teams of 37 CTAs; 777 x 1283
+// in tiles of 190, 5 ignitions: 63 and 44 ms.
+constexpr uint32_t kWaveStop = 0xFFFFFFFFu, kWaveIdle = 0xFFFFFFFEu;
+constexpr unsigned long long kWavePickNs = 1000000ull;       // 1 ms: a team's members wait that long at their barrier
+constexpr unsigned long long kWaveStallNs = 20000000000ull;  // 20 s without a launch done anywhere
+
+// The first launch in sequence that may run and no team has taken: round << 12
+// | tile; kWaveStop when the job is finished (or cannot go on), kWaveIdle when
+// nothing was to be had for kWavePickNs.  By one warp; `done` is shared memory
+// for w.tiles words.
+__device__ __noinline__ uint32_t wave_pick(const WaveDev &w, int TX, int TY, const uint32_t *err,
+                                           uint32_t *done, uint32_t lane) {
+  const unsigned long long start = globaltimer_ns();
+  for (;;) {
+    if (ld_relaxed_u32(err) != 0u || ld_relaxed_u32(w.far) != 0u) return kWaveStop;
+    uint32_t low = 0xFFFFFFFFu;
+    for (uint32_t t = lane; t < w.tiles; t += 32) {
+      const uint32_t d = ld_relaxed_u32(w.done + t);
+      done[t] = d;
+      low = min(low, d);
+    }
+    low = __reduce_min_sync(kFull, low);
+    __threadfence();  // what those launches wrote is read after their `done`
+    __syncwarp();
+    // all tiles have finished round `low`, and it improved nothing
+    if (low >= 1 && ld_relaxed_u32(w.worked + low) == 0u) return kWaveStop;
+    uint32_t best = 0xFFFFFFFFu;
+    for (uint32_t t = lane; t < w.tiles; t += 32) {
+      const uint32_t d = done[t], r = d + 1;
+      if (ld_relaxed_u32(w.claim + t) != d) continue;
+      if (r >= kWaveRounds) {
+        *w.far = 1u;
+        continue;
+      }
+      if (r > 1 && ld_relaxed_u32(w.worked + d) == 0u) continue;
+      const int x = (int)t % TX, y = (int)t / TX;
+      bool ready = true;
+      for (int v = max(y - w.window, 0); v <= min(y + w.window, TY - 1) && ready; ++v)
+        for (int u = max(x - w.window, 0); u <= min(x + w.window, TX - 1); ++u) {
+          const uint32_t o = (uint32_t)(u + v * TX);
+          ready = ready && done[o] >= (o < t ? r : d);
+        }
+      if (ready) best = min(best, r << 12 | t);
+    }
+    best = __reduce_min_sync(kFull, best);
+    if (best != 0xFFFFFFFFu) {
+      uint32_t got = 0;
+      if (lane == 0) {
+        const uint32_t r = best >> 12;
+        got = atomicCAS(w.claim + (best & 0xFFFu), r - 1, r) == r - 1;
+      }
+      if (__shfl_sync(kFull, got, 0)) {
+        __threadfence();
+        return best;
+      }
+    } else {
+      if (globaltimer_ns() - start > kWavePickNs) return kWaveIdle;
+      __nanosleep(200);
+    }
+    __syncwarp();
+  }
+}
+
+template <int kArith>
+__global__ void __launch_bounds__(kEngineThreads, 1)
+    waves_kernel(const JobDev *__restrict__ jobs, const SlotDev *__restrict__ slots, uint32_t *__restrict__ err,
+                 StatsDev *__restrict__ st, WaveDev w, uint32_t group) {
+  extern __shared__ __align__(16) char dyn_smem[];
+  const SlotDev s = slots[blockIdx.x / group];
+  const uint32_t rank = blockIdx.x % group;
+  const uint32_t tid = rank * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  __shared__ DirConst dc;
+  __shared__ JobDev js;
+  __shared__ ScanItem queue[kScanQueue];
+  __shared__ int team_ok[2];
+  __shared__ uint32_t cta_ctr[5];
+  Team<true> team{reinterpret_cast<unsigned long long *>(s.ctr + 8), err, team_ok, group};
+  float *const cross = reinterpret_cast<float *>(dyn_smem + global_tile_cross_off(blockDim.x));
+  uint32_t *const list = reinterpret_cast<uint32_t *>(dyn_smem);  // between launches: the leader's copy of w.done
+  if (threadIdx.x == 0) {
+    js = jobs[0];
+    dir_consts(js, dc);
+  }
+  __syncthreads();
+  const JobDev &j = js;
+  fill_cross(cross);
+  if (blockIdx.x == 0 && threadIdx.x == 0) st->t_start_ns = globaltimer_ns();
+  SweepCtx cx;
+  cx.leader = tid == 0;
+  cx.max_sweeps = ~0ull;
+  cx.t_phase = clock64();
+  uint32_t turn = 0, seen = 0;
+  unsigned long long idle_since = 0;
+  for (;;) {
+    // the leader's warp picks; its word alternates, so that it is not
+    // overwritten before every CTA has read it
+    if (rank == 0 && threadIdx.x < 32) {
+      uint32_t pick = wave_pick(w, j.TX, j.TY, err, list, lane);
+      if (lane == 0) {
+        const uint32_t done = ld_relaxed_u32(w.far + 1);
+        if (pick != kWaveIdle || done != seen || idle_since == 0) {
+          seen = done;
+          idle_since = globaltimer_ns();
+        } else if (globaltimer_ns() - idle_since > kWaveStallNs) {
+          atomicOr(err, 1u);
+          pick = kWaveStop;
+        }
+        s.ctr[turn & 1u] = pick;
+      }
+    }
+    if (!team.sync()) {
+      cx.failed = true;
+      break;
+    }
+    const uint32_t pick = __ldcg(s.ctr + (turn & 1u));
+    ++turn;
+    if (pick == kWaveIdle) continue;
+    if (pick == kWaveStop) break;
+    const uint32_t r = pick >> 12, t = pick & 0xFFFu;
+    TileDesc td;
+    td.x0 = ((int)t % j.TX) * j.T;
+    td.y0 = ((int)t / j.TX) * j.T;
+    td.TW = min(j.T, j.W - td.x0);
+    td.TH = min(j.T, j.H - td.y0);
+    const unsigned long long before = cx.sweeps;
+    const bool worked = tile_global<kArith, true, true>(
+        j, dc, s, td, list, reinterpret_cast<TileUpdate *>(dyn_smem + global_tile_list_bytes(blockDim.x)), cta_ctr,
+        queue, cross, rank, group, cx, team, w.window * j.T - 1, w.far);
+    if (cx.abort) break;
+    if (tid == 0) {
+      atomicAdd(w.sweeps + r, (uint32_t)(cx.sweeps - before));
+      if (worked) atomicOr(w.worked + r, 1u);
+      __threadfence();  // the team's writes (its last barrier made them visible here), then `done`
+      atomicExch(w.done + t, r);
+      atomicAdd(w.far + 1, 1u);
+    }
+  }
+  add_counters(cx.cnt, st, lane);
+  if (threadIdx.x == 0 && cx.improvements) atomicAdd(&st->improvements, cx.improvements);
+  if (tid == 0) {
+    atomicAdd(&st->cyc_first, cx.cyc[0]);
+    atomicAdd(&st->cyc_eval, cx.cyc[1]);
+    atomicAdd(&st->cyc_wait, team.waited);
+    atomicMax(&st->t_done_ns, globaltimer_ns());
+    if (cx.failed || ld_relaxed_u32(err) != 0u) atomicMax(&st->status, kStatusGroupTimeout);
+  }
+}
+
+// After the waves: the schedule's counts, or a second start.  redo: the queue
+// (position, error flag) of the engine launch that follows, which takes the job
+// only when *w.far is set.
+__global__ void wave_end_kernel(WaveDev w, StatsDev *__restrict__ st, uint32_t *__restrict__ redo) {
+  if (threadIdx.x != 0) return;
+  redo[1] = 0u;
+  if (st->status != 0u) *w.far = 0u;  // a wait gave up: reported, not repeated
+  if (*w.far != 0u) {
+    *st = StatsDev{};
+    redo[0] = 0u;
+    return;
+  }
+  redo[0] = 1u;  // past the last job
+  unsigned long long sweeps = 0;
+  uint32_t r = 1;
+  for (; r < kWaveRounds; ++r) {
+    sweeps += w.sweeps[r];
+    if (w.worked[r] == 0u) break;
+  }
+  st->rounds = r;
+  st->launches = (unsigned long long)r * w.tiles;
+  st->sweeps = sweeps;
 }
 
 // ---------------------------------------------------------------- post ----
@@ -1881,14 +2088,15 @@ static unsigned grid_for(uint64_t cells, int sms) {
 }
 
 cudaError_t launch_prep(const JobDev *jobs, uint32_t n_jobs, uint64_t max_cells, int sms,
-                        cudaStream_t stream) {
+                        const uint32_t *only_if, cudaStream_t stream) {
   dim3 grid(grid_for(max_cells, sms), n_jobs);
-  prep_kernel<<<grid, 256, 0, stream>>>(jobs);
+  prep_kernel<<<grid, 256, 0, stream>>>(jobs, only_if);
   return cudaGetLastError();
 }
 
-cudaError_t launch_ignite(const JobDev *jobs, uint32_t n_jobs, cudaStream_t stream) {
-  ignite_kernel<<<n_jobs, 32, 0, stream>>>(jobs);
+cudaError_t launch_ignite(const JobDev *jobs, uint32_t n_jobs, const uint32_t *only_if,
+                          cudaStream_t stream) {
+  ignite_kernel<<<n_jobs, 32, 0, stream>>>(jobs, only_if);
   return cudaGetLastError();
 }
 
@@ -1917,7 +2125,8 @@ static EngineKernel engine_for(int arith, bool group) {
   return group ? engine_kernel<kArithMixed, true> : engine_kernel<kArithMixed, false>;
 }
 
-static cudaError_t engine_attrs(EngineKernel kernel, size_t smem) {
+template <typename K>
+static cudaError_t engine_attrs(K kernel, size_t smem) {
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1967,6 +2176,44 @@ cudaError_t launch_engine(const JobDev *jobs, uint32_t n_jobs, const SlotDev *sl
   cudaLaunchConfig_t cfg = engine_config(csize, threads, n_slots * (unsigned)csize, smem, attr, stream);
   return cudaLaunchKernelEx(&cfg, kernel, jobs, n_jobs, slots, queue, stats, max_sweeps, order,
                             0u);
+}
+
+using WavesKernel = void (*)(const JobDev *, const SlotDev *, uint32_t *, StatsDev *, WaveDev, uint32_t);
+static WavesKernel waves_for(int arith) {
+  return arith == kArithRef ? waves_kernel<kArithRef> : waves_kernel<kArithPortable>;
+}
+
+// CTAs of the waves kernel resident at once.
+cudaError_t waves_max_ctas(int threads, size_t smem, int arith, int *n) {
+  cudaError_t e = engine_attrs(waves_for(arith), smem);
+  if (e != cudaSuccess) return e;
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t cfg = engine_config(1, threads, 1, smem, attr, 0);
+  return cudaOccupancyMaxActiveClusters(n, waves_for(arith), &cfg);
+}
+
+// One job by `teams` teams of `group` CTAs (a cooperative launch), then the
+// counts or the order to start again; err: the launch's error flag.
+cudaError_t launch_waves(const JobDev *job, const SlotDev *slots, uint32_t teams, uint32_t group, int threads,
+                         size_t smem, uint32_t *err, StatsDev *stats, const WaveDev &w, uint32_t *redo, int arith,
+                         cudaStream_t stream) {
+  const WavesKernel kernel = waves_for(arith);
+  cudaError_t e = engine_attrs(kernel, smem);
+  if (e != cudaSuccess) return e;
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(teams * group, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, kernel, job, slots, err, stats, w, group);
+  if (e != cudaSuccess) return e;
+  wave_end_kernel<<<1, 32, 0, stream>>>(w, stats, redo);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_post(const JobDev *jobs, uint32_t n_jobs, uint64_t max_cells, int sms,

@@ -114,6 +114,21 @@ constexpr uint32_t kOwnGroup = 4;
 __host__ __device__ inline uint32_t owner_words(uint32_t TN, uint32_t R) {
   return (((TN + kOwnGroup - 1) / kOwnGroup + R - 1) / R + 7) / 8;
 }
+// Several teams on one job (waves): the tile launches of the reference's
+// sequence (rounds of all tiles in row-major order) run as soon as the launches
+// they depend on are done.  Words, zeroed before the run:
+struct WaveDev {
+  uint32_t *done;    // per tile: rounds finished
+  uint32_t *claim;   // per tile: rounds taken by a team
+  uint32_t *worked;  // per round: a launch of it improved a cell
+  uint32_t *sweeps;  // per round: sweeps of its launches
+  uint32_t *far;     // [0] a reference lies too far away for `window`; [1] launches done
+  uint32_t tiles;
+  int32_t window;    // launches of tiles up to this many tiles apart keep their order
+};
+constexpr uint32_t kWaveRounds = 1024;  // rounds the words hold
+constexpr uint32_t kWaveTiles = 4096;   // tiles a team's leader looks through
+
 // Update-array entries a CTA of an R-CTA team may need in one sweep of a
 // global-memory tile of TN cells: the cells it owns.
 __host__ __device__ inline uint32_t global_tile_upd_cap(uint32_t TN, uint32_t R) {
