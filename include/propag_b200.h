@@ -381,7 +381,7 @@ int propag_autotune(const PropagJob *jobs, const PropagTerrainPtrs *terrains, ui
  *
  * Same kernels, schedule and results as propag_engine_run with one job, but
  * its scratch (references, referrer boxes, boundary bits, job descriptor,
- * counters, statistics, list overflow) lives in one fixed device array of about 25 MiB,
+ * counters, statistics, list overflow) lives in one fixed device array of about 29 MiB,
  * reserved by the CUDA driver when the library's module holding it is loaded.
  * The call makes no cudaMalloc, cudaFree or cudaMallocHost, creates no events
  * and uses no caching allocator.  It is meant for callers that cannot

@@ -28,6 +28,7 @@ namespace propag {
 
 // launchers (fire.cu, engine_launch.cu)
 cudaError_t upload_catalog();
+cudaError_t upload_cross_table();
 cudaError_t launch_fire(bool full, uint64_t n, const uint8_t *fuel, const float *const m[5],
                         const float *ws, const float *waz, const float *slope,
                         const float *aspect, float *const outs[10], int sm_count,
@@ -105,6 +106,7 @@ int ensure_device(int want, int *sms_out) {
   if (!d.ready) {
     CK(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
     CK(upload_catalog());
+    CK(upload_cross_table());
     d.ready = true;
   }
   if (sms_out) *sms_out = d.sms;
@@ -440,8 +442,8 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
     off[i] = job_bytes;
     // fifteen words a cell, the boundary bits and the pending bitmap: packed
     // records (fire and box_x0, two state copies, the other box corners) for
-    // global-memory tiles, or references, referrer boxes and travel-time
-    // planes for shared-memory ones
+    // global-memory tiles, or references, lines of sight, referrer boxes and
+    // travel-time planes for shared-memory ones
     job_bytes += align_up(N * 4, 256) * 15 + (j.boundaries ? 0 : align_up(words * 4, 256)) +
                  align_up(words * 4, 256);
     max_cells = std::max<uint64_t>(max_cells, N);
@@ -562,6 +564,7 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
       d.tt = reinterpret_cast<float *>(take(8 * plane));
       d.tt_plane = (int64_t)(plane / 4);
       d.refs = reinterpret_cast<uint32_t *>(take(plane));
+      d.los = reinterpret_cast<uint32_t *>(take(plane));
       d.box_x0 = reinterpret_cast<uint32_t *>(take(plane));
       d.box_x0_step = 1;
     }
@@ -1089,6 +1092,7 @@ extern "C" int propag_run_device_static(const PropagJob *job, void *stream_ptr, 
   d.box_y0 = cells + 2 * kStaticMaxCells;
   d.box_x1 = cells + 3 * kStaticMaxCells;
   d.box_y1 = cells + 4 * kStaticMaxCells;
+  d.los = cells + 5 * kStaticMaxCells;
   d.bnd = j.boundaries ? j.boundaries : reinterpret_cast<uint32_t *>(base + kStaticBndOff);
   SlotDev s{};  // shared-memory tiles use the counters and the list overflow
   s.ctr = reinterpret_cast<uint32_t *>(base + kStaticCtrOff);

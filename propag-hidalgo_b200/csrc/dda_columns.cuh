@@ -21,6 +21,11 @@
 #define __device__
 #define __forceinline__ inline
 #endif
+#if defined(__CUDACC__)
+#define PG_HOST_DEVICE __host__ __device__
+#else
+#define PG_HOST_DEVICE
+#endif
 
 namespace propag {
 
@@ -28,7 +33,7 @@ constexpr int kColumnsMax = 127;
 // Accumulated crossing times: T(n, i) (i steps of 1 / n) at n (n - 1) / 2 + i - 1.
 constexpr int kCrossTableLen = kColumnsMax * (kColumnsMax + 1) / 2;
 
-__device__ __forceinline__ int cross_at(int n, int i) { return n * (n - 1) / 2 + i - 1; }
+PG_HOST_DEVICE inline int cross_at(int n, int i) { return n * (n - 1) / 2 + i - 1; }
 
 // Rows crossed strictly before the c-th crossing of the longer axis, and
 // whether a row crossing coincides with it.  inv_p is 1 / P rounded to float:

@@ -44,6 +44,7 @@
 
 #include <cfloat>
 #include <cstdint>
+#include <vector>
 
 #include "dda_columns.cuh"
 #include "engine.cuh"
@@ -181,13 +182,13 @@ __global__ void ignite_kernel(const JobDev *__restrict__ jobs, const uint32_t *_
     const float t = packed ? j.st0[c].time : j.time[c];
     if (t != FLT_MAX) {
       const uint32_t r = pack_ref(ign[k].x, ign[k].y);
+      const uint32_t los = los_of_self((j.bnd[c >> 5] >> (c & 31)) & 1u);
       if (packed) {
-        // a cell that references itself visits itself twice, or is blocked at once
-        const bool b = (j.bnd[c >> 5] >> (c & 31)) & 1u;
         j.st0[c].ref = r;
-        j.st0[c].los = b ? kLosBlocked | 1u : 2u;
+        j.st0[c].los = los;
       } else {
         j.refs[c] = r;
+        j.los[c] = los;
       }
       j.box_x0[c * j.box_x0_step] = j.box_x1[c] = ign[k].x;
       j.box_y0[c] = j.box_y1[c] = ign[k].y;
@@ -229,11 +230,6 @@ struct Best {
   uint32_t ref;
 };
 
-__device__ __forceinline__ bool line_blocked_call(const uint32_t *__restrict__ bnd, int W, int fx,
-                                               int fy, int tx, int ty, uint32_t &steps) {
-  return line_blocked(bnd, W, fx, fy, tx, ty, steps);
-}
-
 struct Counters {
   uint32_t dda = 0, gat = 0, walk_max = 0;
   unsigned long long evals = 0, scans = 0, scan_cells = 0;
@@ -246,11 +242,11 @@ struct Counters {
 // direct time when the line of sight is blocked or the candidate is not
 // faster -- and the sequential loop keeps the first strictly smaller offer;
 // so the result is the first minimum of the offers when it beats the cell's
-// own time.  A lane walks its line of sight whenever the sequential loop
-// could (candidate faster than the neighbour's direct time and than the
-// cell's own time); only the walks the sequential loop performs (candidate
-// also faster than every earlier offer) are counted, so the counters match
-// the reference's order exactly.  Called by all 32 lanes.
+// own time.  The line of sight from the neighbour to its reference was walked
+// when it adopted the reference, and is read; only the walks the sequential
+// loop performs (candidate also faster than every earlier offer) are counted,
+// so the counters match the reference's order exactly.  Called by all 32
+// lanes.
 template <int kArith, typename Acc>
 __device__ __forceinline__ Best evaluate_coop(const JobDev &j, const DirConst &dc, const Acc &acc,
                                               int x, int y, Best own, bool valid, uint32_t lane,
@@ -259,26 +255,34 @@ __device__ __forceinline__ Best evaluate_coop(const JobDev &j, const DirConst &d
   const int k = (int)(lane & 7u);
   const int kk = k < 4 ? k : k + 1;
   const int nx = x + kk % 3 - 1, ny = y + kk / 3 - 1;
-  bool act = false;
   float nt = FLT_MAX, rt = FLT_MAX;
   uint32_t nr = kNoRef;
+  bool act = false;
+  if (valid && nx >= 0 && ny >= 0 && nx < j.W && ny < j.H) {
+    acc.cell(nx, ny, nt, nr);
+    act = nt < j.max_time && nr != pack_ref(x, y);
+  }
+  // far from the fire (most cells of a whole tile's first sweep) nothing else
+  // is read
+  if (!__any_sync(kFull, act)) return own;
   Fire f{0.0f, 0.0f, 0.0f};
   float tt = 0.0f;
-  if (valid && nx >= 0 && ny >= 0 && nx < j.W && ny < j.H) {
-    // the fire loads go out together with the state load (one memory
-    // round trip), whether or not the neighbour turns out to burn
+  uint32_t los = 0;
+  if (act) {
+    // one memory round trip for all of these
     const int64_t n = nx + (int64_t)ny * j.W;
     f.speed_max = __ldg(j.speed + n);
     f.azimuth_max = __ldg(j.az + n);
     f.eccentricity = __ldg(j.ecc + n);
     if (j.tt) tt = __ldg(j.tt + k * j.tt_plane + n);
-    acc.cell(nx, ny, nt, nr);
-    act = nt < j.max_time && f.speed_max != 0.0f && !(ref_x(nr) == x && ref_y(nr) == y);
-    if (act) rt = acc.time_of(nr);
+    los = __ldcg(j.los + n);
+    rt = acc.time_of(nr);
+    act = f.speed_max != 0.0f;
   }
   cnt.gat += act ? 1u : 0u;
   float offer = kInf, cand = kInf;
-  uint32_t oref = 0, steps = 0;
+  uint32_t oref = 0;
+  const uint32_t steps = los & ~kLosBlocked;
   bool walked = false;
   if (act) {
     const bool refm = arith_of<kArith>(j);
@@ -288,12 +292,8 @@ __device__ __forceinline__ Best evaluate_coop(const JobDev &j, const DirConst &d
     offer = ntime;
     oref = pack_ref(nx, ny);
     if (cand < ntime) {
-      bool blocked = false;
-      if (cand < own.time) {
-        walked = true;
-        blocked = line_blocked_call(j.bnd, j.W, nx, ny, ref_x(nr), ref_y(nr), steps);
-      }
-      if (!blocked) {
+      walked = cand < own.time;
+      if (!(walked && (los & kLosBlocked))) {
         offer = cand;
         oref = nr;
       }
@@ -903,9 +903,13 @@ __device__ __forceinline__ Best evaluate_packed(const JobDev &j, const Hot &h,
   return bv < own.time ? Best{bv, br} : own;
 }
 
-// The line of sight from cell (fx, fy) to (tx, ty) (line_blocked's walk, same
-// cells, same count) by the eight lanes of a cell; the result is a CellState's
-// los.  Called by all 32 lanes; `on` is uniform in each group of eight.
+// The line of sight from cell (fx, fy) to (tx, ty) by the eight lanes of a
+// cell; the result is a CellState's los.  The walk (propag.h:91-135) visits the
+// cells from one to the other inclusive; its t-max accumulators are the
+// reference's float arithmetic: start 1/|d|, step +1/|d|, a diagonal step when
+// |tmax.x - tmax.y| < 1e-9 (a double comparison in the reference: for a float v,
+// (double)v < 1e-9 exactly when v is at most the largest float below 1e-9).
+// Called by all 32 lanes; `on` is uniform in each group of eight.
 //
 // Step by step, for offsets beyond kColumnsMax: every lane generates the walk,
 // lane i of the eight looks up the visited cells i, i + 8, ... of each run of
@@ -970,6 +974,10 @@ __device__ __noinline__ uint32_t walk_los_steps(const uint32_t *__restrict__ bnd
   }
   return los ? los : steps;
 }
+
+// Accumulated crossing times for tiles whose CTAs have no shared memory left
+// for them (uploaded once per device).
+__device__ float d_cross[kCrossTableLen];
 
 // In closed form (dda_columns.cuh), lane i of the eight taking columns i, i +
 // 8, ..., four at a time (kColumnRun columns a group): all bitmap words of a
@@ -1504,7 +1512,7 @@ struct SmemAcc {
 // One tile launch resident in the cluster's shared memory; B is the staged
 // referrer-box codec.
 template <class B, int kArith>
-__device__ bool tile_smem(const JobDev &j, const DirConst &dc, char *smem, const SlotDev &slot,
+__device__ bool tile_smem(const JobDev &j, const DirConst &dc, char *smem, const float *cross, const SlotDev &slot,
                           const TileDesc &td, ScanBox *scan_boxes, SweepCtx &cx, Team<false> &team) {
   using BoxT = typename B::T;
   cg::cluster_group cluster = cg::this_cluster();
@@ -1628,12 +1636,13 @@ __device__ bool tile_smem(const JobDev &j, const DirConst &dc, char *smem, const
     for (uint32_t base = (threadIdx.x >> 5) * per; base < nupd; base += nwarps * per) {
       const uint32_t u = base + lane;
       const bool valid = lane < per && u < nupd;
-      uint32_t want = 0;
+      uint32_t want = 0, adopted = 0;
       Box box{1, 1, 0, 0};
       if (valid) {
         uint32_t s, r;
         float t;
         upd_get(sm, u, s, t, r);
+        adopted = r;
         const int lr = g.div_p((int)s), hx = (int)s - lr * g.P, hy = g.rank + lr * g.C;
         const int x = g.x0 - 1 + hx, y = g.y0 - 1 + hy;
         sm.time[s] = t;
@@ -1667,6 +1676,15 @@ __device__ bool tile_smem(const JobDev &j, const DirConst &dc, char *smem, const
           box = clip_box(g.x0 - 1 + bx0, g.y0 - 1 + by0, g.x0 - 1 + bx1, g.y0 - 1 + by1, g.x0, g.y0,
                          g.TW, g.TH, j.W, j.H);
         }
+      }
+      // the lines of sight to the adopted references, four cells at a time
+      // (eight lanes each; read by other CTAs after the barrier below)
+      for (uint32_t i = 0; i < per; i += 4) {
+        const uint32_t from = i + (lane >> 3);
+        const uint32_t c = __shfl_sync(kFull, want, (int)(from & 31u)), r = __shfl_sync(kFull, adopted, (int)(from & 31u));
+        const bool on = from < per && base + from < nupd;
+        const uint32_t los = walk_los(j.bnd, cross, j.W, ref_x(c), ref_y(c), ref_x(r), ref_y(r), on, lane);
+        if (on && (lane & 7u) == 0) __stcg(j.los + (uint32_t)ref_x(c) + (uint32_t)ref_y(c) * (uint32_t)j.W, los);
       }
       warp_scan_boxes(
           scan_boxes + (threadIdx.x & ~31u), box, want, j, lane, cnt,
@@ -1820,9 +1838,9 @@ __global__ void __launch_bounds__(kEngineThreads, 1)
         bool w = false;
         if constexpr (!kGroup) {
           if (j.smem_tile == kSmemTileExact)
-            w = tile_smem<BoxExact, kArith>(j, dc, dyn_smem, s, td, scan_boxes, cx, team);
+            w = tile_smem<BoxExact, kArith>(j, dc, dyn_smem, d_cross, s, td, scan_boxes, cx, team);
           else if (j.smem_tile == kSmemTileCoarse)
-            w = tile_smem<BoxCoarse, kArith>(j, dc, dyn_smem, s, td, scan_boxes, cx, team);
+            w = tile_smem<BoxCoarse, kArith>(j, dc, dyn_smem, d_cross, s, td, scan_boxes, cx, team);
         }
         if (kGroup || j.smem_tile == kSmemTileGlobal)
           w = tile_global<kArith, kGroup, false>(
@@ -2133,6 +2151,17 @@ static cudaError_t engine_attrs(K kernel, size_t smem) {
 }
 
 int engine_threads() { return kEngineThreads; }
+
+// The walks' crossing times on the current device.
+cudaError_t upload_cross_table() {
+  std::vector<float> t(kCrossTableLen);
+  for (int n = 1; n <= kColumnsMax; ++n) {
+    const float step = 1.0f / (float)n;
+    float v = step;
+    for (int i = 1; i <= n; ++i, v += step) t[(size_t)cross_at(n, i)] = v;
+  }
+  return cudaMemcpyToSymbol(d_cross, t.data(), t.size() * sizeof(float));
+}
 
 // Clusters of csize CTAs resident at once, of the kernel that launch_engine
 // runs for this arithmetic and kind of team.

@@ -20,6 +20,9 @@ struct alignas(16) CellState {
   uint32_t pad;
 };
 constexpr uint32_t kLosBlocked = 0x80000000u;
+// The line of sight of a cell that references itself (an ignition): its walk
+// visits it twice, or meets a boundary at once.
+__host__ __device__ inline uint32_t los_of_self(bool boundary) { return boundary ? kLosBlocked | 1u : 2u; }
 
 // One scenario as the device sees it.
 struct JobDev {
@@ -33,6 +36,7 @@ struct JobDev {
   const float *speed, *az, *ecc;
   float *time;         // the output; shared-memory tiles also keep their state here
   uint32_t *refs;      // state of shared-memory tiles: packed x | y << 16
+  uint32_t *los;       // and every cell's line of sight to its reference (CellState::los)
   uint32_t *bnd;       // boundary bits (written by the prep pass)
   // referrer box of every cell (the cells that ever adopted it as their
   // reference): min and max corner, 0xFFFFFFFF in box_x0 = empty

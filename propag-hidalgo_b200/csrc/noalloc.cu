@@ -9,8 +9,8 @@
 //   [512, 768)      StatsDev
 //   [768, 1024)     job queue counter
 //   [1024, 1280)    slot counters
-//   [2048, ...)     five per-cell arrays of kStaticMaxCells uint32 (references
-//                   and the four referrer-box corners), then the boundary
+//   [2048, ...)     six per-cell arrays of kStaticMaxCells uint32 (references,
+//                   the four referrer-box corners and lines of sight), then the boundary
 //                   bitmap (kStaticMaxCells / 32 words), then the overflow of
 //                   the shared-memory work and update lists
 //                   (kStaticOvfSlots u16 entries, then kStaticOvfSlots Updates)

@@ -13,8 +13,8 @@ struct JobDev;
 struct SlotDev;
 struct StatsDev;
 
-// Largest grid the fixed scratch holds: 1024 x 1024 cells (20 B per cell of
-// references and referrer boxes, plus one boundary bit).
+// Largest grid the fixed scratch holds: 1024 x 1024 cells (24 B per cell of
+// references, referrer boxes and lines of sight, plus one boundary bit).
 constexpr uint64_t kStaticMaxCells = 1ull << 20;
 constexpr size_t kStaticJobOff = 0;
 constexpr size_t kStaticSlotOff = 256;
@@ -24,7 +24,7 @@ constexpr size_t kStaticCtrOff = 1024;
 constexpr int kStaticCtrWords = 16;
 constexpr size_t kStaticCellsOff = 2048;
 constexpr size_t kStaticArrayBytes = kStaticMaxCells * 4;
-constexpr size_t kStaticBndOff = kStaticCellsOff + 5 * kStaticArrayBytes;
+constexpr size_t kStaticBndOff = kStaticCellsOff + 6 * kStaticArrayBytes;
 // Overflow of the shared-memory work and update lists: cluster size x cell
 // slots per CTA entries (16 CTAs x 17 408 slots covers every tile whose
 // shared-memory footprint fits the 200 KB budget).

@@ -10,7 +10,6 @@
 // Semantics follow the reference kernel (paths relative to the reference
 // project):
 //   time_from                          crates/propag/src/propag.cu:269-294
-//   DDA line walk                      crates/propag/src/propag.h:91-135
 //   find_neighbor_which_reaches_first  crates/propag/src/propag.cu:124-190
 //   similar_fires / find_boundaries    crates/propag/src/propag.cu:296-302,345-375
 #pragma once
@@ -155,85 +154,6 @@ __device__ __forceinline__ float time_from(int fx, int fy, float ftime, int tx, 
                                            bool refm) {
   const float inv = inv_speed(bearing(fx, fy, tx, ty, north_up, refm), f, refm);
   return step_time(ftime, cell_distance(fx - tx, fy - ty, gdx, gdy, refm), inv, refm);
-}
-
-// ---- DDA line-of-sight walk (propag.h:91-135) ------------------------------
-// Visits the cells from `from` to `to` inclusive in the reference's order and
-// reports whether one of them is a boundary; `steps` counts the cells
-// visited up to and including the first boundary.  The t-max accumulators
-// are the reference's float arithmetic: start 1/|d| (formed in double), step
-// +1/|d|, diagonal step when |tmax.x - tmax.y| < 1e-9 (a double comparison
-// in the reference: for a float v, (double)v < 1e-9 exactly when v is at most
-// the largest float below 1e-9).  The walk is bounded by |dx| + |dy| + 2
-// visits, more than any walk takes.
-//
-// The cells are generated kWalkBatch at a time by the (load-free) DDA
-// arithmetic, their bitmap words are loaded together, and then checked in
-// visiting order: one load latency per batch instead of one per cell.
-constexpr int kWalkBatch = 8;
-
-__device__ __forceinline__ bool is_boundary(const uint32_t *__restrict__ bnd, int64_t ix) {
-  return (__ldg(bnd + (ix >> 5)) >> (ix & 31)) & 1u;
-}
-
-__device__ __forceinline__ bool line_blocked(const uint32_t *__restrict__ bnd, int W, int fx,
-                                             int fy, int tx, int ty, uint32_t &steps) {
-  const int sx = (tx > fx) - (tx < fx), sy = (ty > fy) - (ty < fy);
-  const int adx = abs(tx - fx), ady = abs(ty - fy);
-  float tmx = __double2float_rn(1.0 / (double)(float)adx);
-  float tmy = __double2float_rn(1.0 / (double)(float)ady);
-  const float ddx = tmx, ddy = tmy;
-  const float kTie = __int_as_float(0x3089705F);  // the largest float below 1e-9
-  int cx = fx, cy = fy;
-  int left = adx + ady + 2;  // visits the bound still allows
-  for (;;) {
-    uint32_t ix[kWalkBatch];  // cell index x + y W (grids below 2^32 cells)
-    int nv = 0;               // cells of this batch
-    bool ended = left <= 0;
-#pragma unroll
-    for (int i = 0; i < kWalkBatch; ++i) {
-      if (!ended && i < left) {
-        const int px = cx, py = cy;
-        if (px == tx && py == ty) {
-          cx += sx;
-          cy += sy;
-        } else {
-          const bool vx = sx > 0 ? cx <= tx : cx >= tx;
-          const bool vy = sy > 0 ? cy <= ty : cy >= ty;
-          if (!(vx && vy)) {
-            ended = true;
-          } else if (fabsf(__fsub_rn(tmx, tmy)) <= kTie) {
-            cx += sx;
-            cy += sy;
-            tmx = __fadd_rn(tmx, ddx);
-            tmy = __fadd_rn(tmy, ddy);
-          } else if (tmx < tmy) {
-            cx += sx;
-            tmx = __fadd_rn(tmx, ddx);
-          } else {
-            cy += sy;
-            tmy = __fadd_rn(tmy, ddy);
-          }
-        }
-        if (!ended) {
-          ix[i] = (uint32_t)px + (uint32_t)py * (uint32_t)W;
-          nv = i + 1;
-        }
-      }
-    }
-    uint32_t word[kWalkBatch];
-#pragma unroll
-    for (int i = 0; i < kWalkBatch; ++i) word[i] = i < nv ? __ldg(bnd + (ix[i] >> 5)) : 0u;
-#pragma unroll
-    for (int i = 0; i < kWalkBatch; ++i) {
-      if (i < nv) {
-        ++steps;
-        if ((word[i] >> (ix[i] & 31)) & 1u) return true;
-      }
-    }
-    if (nv < kWalkBatch) return false;  // the walk ended in this batch
-    left -= kWalkBatch;
-  }
 }
 
 // similar_fires (propag.cu:296-302): float differences compared against the
