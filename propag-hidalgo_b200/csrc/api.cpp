@@ -231,9 +231,8 @@ struct propag_engine {
   size_t last_smem = 0;
   cudaStream_t stream = nullptr;  // the stream of the last run
   DevBuf job_scratch, slot_scratch, meta;
-  JobDev *jobs_pinned = nullptr;
-  SlotDev *slots_pinned = nullptr;
-  size_t pinned_jobs = 0, pinned_slots = 0;
+  char *pinned = nullptr;  // staging of the job and slot descriptors and the queue order
+  size_t pinned_bytes = 0;
   cudaEvent_t staged = nullptr;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // around prep, engine, post
   StatsDev *last_stats = nullptr;  // device statistics of the last run's jobs
@@ -246,6 +245,31 @@ namespace propag {
 void engine_keep_to_clusters(propag_engine *e) { e->auto_groups = false; }
 
 
+// Layout of an engine's descriptors in device memory (and, up to `zeros`, in
+// the pinned staging): jobs, slots and queue order, copied in one piece, then
+// the statistics, the queue words and a waves run's words, cleared in one piece.
+struct MetaLayout {
+  size_t slots, order, zeros, queue, wave, bytes;
+  MetaLayout(size_t n_jobs, size_t n_slots, size_t wave_words) {
+    slots = align_up(sizeof(JobDev) * n_jobs, 256);
+    order = slots + align_up(sizeof(SlotDev) * n_slots, 256);
+    zeros = order + align_up(sizeof(uint32_t) * n_jobs, 256);
+    queue = zeros + align_up(sizeof(StatsDev) * n_jobs, 256);
+    wave = queue + 256;
+    bytes = wave + wave_words * 4;
+  }
+};
+
+static int reserve_pinned(propag_engine *e, size_t bytes) {
+  if (e->pinned_bytes >= bytes) return PROPAG_OK;
+  if (e->pinned) cudaFreeHost(e->pinned);
+  e->pinned = nullptr;
+  e->pinned_bytes = 0;
+  CK(cudaMallocHost(&e->pinned, bytes));
+  e->pinned_bytes = bytes;
+  return PROPAG_OK;
+}
+
 // Reserves the engine's device scratch and pinned staging for batches of up
 // to max_jobs jobs whose job scratch sums to at most job_bytes, with slot
 // scratch of slot_bytes, so that such batches allocate nothing (a later
@@ -255,22 +279,10 @@ int engine_reserve(propag_engine *e, size_t job_bytes, uint32_t max_jobs, size_t
   CK(cudaSetDevice(e->device));
   CK(e->job_scratch.reserve(job_bytes, stream, true));
   CK(e->slot_scratch.reserve(slot_bytes, stream, true));
-  CK(e->meta.reserve(align_up(sizeof(JobDev) * max_jobs, 256) + align_up(sizeof(SlotDev) * max_jobs, 256) +
-                         align_up(sizeof(StatsDev) * max_jobs, 256) + 256 +
-                         align_up(sizeof(uint32_t) * max_jobs, 256),
-                     stream));
-  if (e->pinned_jobs < max_jobs) {
-    if (e->jobs_pinned) cudaFreeHost(e->jobs_pinned);
-    e->jobs_pinned = nullptr;
-    CK(cudaMallocHost(&e->jobs_pinned, sizeof(JobDev) * max_jobs + sizeof(uint32_t) * max_jobs));
-    e->pinned_jobs = max_jobs;
-  }
-  if (e->pinned_slots < max_jobs) {
-    if (e->slots_pinned) cudaFreeHost(e->slots_pinned);
-    e->slots_pinned = nullptr;
-    CK(cudaMallocHost(&e->slots_pinned, sizeof(SlotDev) * max_jobs));
-    e->pinned_slots = max_jobs;
-  }
+  const MetaLayout meta(max_jobs, max_jobs, 0);
+  CK(e->meta.reserve(meta.bytes, stream));
+  const int rc = reserve_pinned(e, meta.zeros);
+  if (rc) return rc;
   return PROPAG_OK;
 }
 }  // namespace propag
@@ -323,8 +335,7 @@ extern "C" void propag_engine_destroy(propag_engine *e) {
   }
   for (int i = 0; i < 4; ++i)
     if (e->ev[i]) cudaEventDestroy(e->ev[i]);
-  if (e->jobs_pinned) cudaFreeHost(e->jobs_pinned);
-  if (e->slots_pinned) cudaFreeHost(e->slots_pinned);
+  if (e->pinned) cudaFreeHost(e->pinned);
   delete e;
   cudaGetLastError();  // leave no error of the teardown to the caller's next CUDA call
 }
@@ -589,81 +600,68 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
   const size_t upd_max = words_max * 32;
   const size_t ovf_list_bytes = align_up((size_t)csize * ovf_cap * 2, 256);
   const size_t ovf_upd_bytes = align_up((size_t)csize * ovf_cap * sizeof(Update), 256);
-  // two dirty bitmaps (alternating) and two update arrays (by sweep parity)
-  const size_t slot_bytes = 2 * align_up(words_max * 4, 256) + 2 * align_up(upd_max * sizeof(TileUpdate), 256) +
-                            256 + ovf_list_bytes + ovf_upd_bytes;
+  // per slot two dirty bitmaps (alternating) and the counters, the slots' side
+  // by side (cleared in one piece), then two update arrays (by sweep parity)
+  // and the overflow lists
+  const size_t clear_bytes = 2 * align_up(words_max * 4, 256) + 256;
+  const size_t rest_bytes = 2 * align_up(upd_max * sizeof(TileUpdate), 256) + ovf_list_bytes + ovf_upd_bytes;
+  const size_t slot_bytes = clear_bytes + rest_bytes;
   CK(e->slot_scratch.reserve(slot_bytes * all_slots, stream));
-  // meta: jobs, slots, stats, queue
-  const size_t meta_jobs = align_up(sizeof(JobDev) * n_jobs, 256);
-  const size_t meta_slots = align_up(sizeof(SlotDev) * all_slots, 256);
-  const size_t meta_stats = align_up(sizeof(StatsDev) * n_jobs, 256);
-  const size_t meta_order = align_up(sizeof(uint32_t) * n_jobs, 256);
   const uint64_t tiles = (uint64_t)jd[0].TX * (uint64_t)jd[0].TY;
   const size_t wave_words = waves.teams ? 64 + 2 * align_up(tiles, 64) + 2 * align_up(kWaveRounds, 64) : 0;
-  CK(e->meta.reserve(meta_jobs + meta_slots + meta_stats + 256 + meta_order + wave_words * 4, stream));
+  const MetaLayout meta(n_jobs, all_slots, wave_words);
+  CK(e->meta.reserve(meta.bytes, stream));
   // staging buffers (pinned) may still be read by the previous run's copies
   // (a run being captured into a graph follows a completed uncaptured run)
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   CK(cudaStreamIsCapturing(stream, &capturing));
   if (capturing == cudaStreamCaptureStatusNone) CK(cudaEventSynchronize(e->staged));
-  if (e->pinned_jobs < n_jobs) {
-    if (e->jobs_pinned) cudaFreeHost(e->jobs_pinned);
-    // the job descriptors, then the queue order
-    CK(cudaMallocHost(&e->jobs_pinned, sizeof(JobDev) * n_jobs + sizeof(uint32_t) * n_jobs));
-    e->pinned_jobs = n_jobs;
-  }
-  if (e->pinned_slots < all_slots) {
-    if (e->slots_pinned) cudaFreeHost(e->slots_pinned);
-    CK(cudaMallocHost(&e->slots_pinned, sizeof(SlotDev) * all_slots));
-    e->pinned_slots = all_slots;
-  }
-  std::copy(jd.begin(), jd.end(), e->jobs_pinned);
+  const int pinned_rc = reserve_pinned(e, meta.zeros);
+  if (pinned_rc) return pinned_rc;
+  std::copy(jd.begin(), jd.end(), reinterpret_cast<JobDev *>(e->pinned));
+  SlotDev *slots_pinned = reinterpret_cast<SlotDev *>(e->pinned + meta.slots);
   // queue order: largest grids first, so that the longest jobs start first
   // and the batch ends close to its longest job (results do not depend on it)
-  uint32_t *order_pinned = reinterpret_cast<uint32_t *>(e->jobs_pinned + n_jobs);
+  uint32_t *order_pinned = reinterpret_cast<uint32_t *>(e->pinned + meta.order);
   for (uint32_t i = 0; i < n_jobs; ++i) order_pinned[i] = i;
   std::stable_sort(order_pinned, order_pinned + n_jobs, [&](uint32_t a, uint32_t b) {
     return (uint64_t)jd[a].W * jd[a].H > (uint64_t)jd[b].W * jd[b].H;
   });
   for (uint32_t s = 0; s < all_slots; ++s) {
-    size_t o = slot_bytes * s;
-    SlotDev &sd = e->slots_pinned[s];
+    size_t o = clear_bytes * s;
+    SlotDev &sd = slots_pinned[s];
     sd.dirty = e->slot_scratch.at<uint32_t>(o);
     sd.dirty_words = (uint32_t)(align_up(words_max * 4, 256) / 4);
     sd.pad0 = 0;
-    o += 2 * align_up(words_max * 4, 256);
+    sd.ctr = e->slot_scratch.at<uint32_t>(o + 2 * align_up(words_max * 4, 256));
+    o = clear_bytes * all_slots + rest_bytes * s;
     sd.upd = e->slot_scratch.at<TileUpdate>(o);
     o += 2 * align_up(upd_max * sizeof(TileUpdate), 256);
-    sd.ctr = e->slot_scratch.at<uint32_t>(o);
-    o += 256;
     sd.ovf_list = e->slot_scratch.at<uint16_t>(o);
     o += ovf_list_bytes;
     sd.ovf_upd = e->slot_scratch.at<Update>(o);
     sd.ovf_cap = (uint32_t)ovf_cap;
     sd.pad = 0;
-    // the dirty bitmap and counters must start cleared
-    CK(cudaMemsetAsync(sd.dirty, 0, 2 * align_up(words_max * 4, 256), stream));
-    CK(cudaMemsetAsync(sd.ctr, 0, 64, stream));  // counters and barrier arrivals
   }
+  // the dirty bitmaps, counters and barrier arrivals must start cleared
+  CK(cudaMemsetAsync(e->slot_scratch.p, 0, clear_bytes * all_slots, stream));
   JobDev *d_jobs = e->meta.at<JobDev>(0);
-  SlotDev *d_slots = e->meta.at<SlotDev>(meta_jobs);
-  StatsDev *d_stats = e->meta.at<StatsDev>(meta_jobs + meta_slots);
-  uint32_t *d_queue = e->meta.at<uint32_t>(meta_jobs + meta_slots + meta_stats);
-  uint32_t *d_order = e->meta.at<uint32_t>(meta_jobs + meta_slots + meta_stats + 256);
+  SlotDev *d_slots = e->meta.at<SlotDev>(meta.slots);
+  uint32_t *d_order = e->meta.at<uint32_t>(meta.order);
+  StatsDev *d_stats = e->meta.at<StatsDev>(meta.zeros);
+  uint32_t *d_queue = e->meta.at<uint32_t>(meta.queue);
   e->last_stats = d_stats;
-  CK(cudaMemcpyAsync(d_jobs, e->jobs_pinned, sizeof(JobDev) * n_jobs, cudaMemcpyHostToDevice, stream));
-  CK(cudaMemcpyAsync(d_order, order_pinned, sizeof(uint32_t) * n_jobs, cudaMemcpyHostToDevice, stream));
-  CK(cudaMemcpyAsync(d_slots, e->slots_pinned, sizeof(SlotDev) * all_slots, cudaMemcpyHostToDevice, stream));
+  CK(cudaMemcpyAsync(e->meta.p, e->pinned, meta.zeros, cudaMemcpyHostToDevice, stream));
   // the engine's events time uncaptured runs only (an event recorded into a
   // graph cannot be waited on or timed from the host)
   const bool live = capturing == cudaStreamCaptureStatusNone;
   if (live) CK(cudaEventRecord(e->staged, stream));
-  CK(cudaMemsetAsync(d_stats, 0, sizeof(StatsDev) * n_jobs, stream));
-  CK(cudaMemsetAsync(d_queue, 0, 16, stream));  // queue position, group error flag (two launches of a waves run)
+  // statistics, queue position and group error flag (of two launches in a
+  // waves run), a waves run's words
+  CK(cudaMemsetAsync(e->meta.at<char>(meta.zeros), 0, meta.bytes - meta.zeros, stream));
   WaveDev wave{};
   if (waves.teams) {
-    uint32_t *words = e->meta.at<uint32_t>(meta_jobs + meta_slots + meta_stats + 256 + meta_order);
-    CK(cudaMemsetAsync(words, 0, wave_words * 4, stream));
+    uint32_t *words = e->meta.at<uint32_t>(meta.wave);
     wave.far = words;
     wave.done = words + 64;
     wave.claim = wave.done + align_up(tiles, 64);
