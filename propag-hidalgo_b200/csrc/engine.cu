@@ -486,6 +486,7 @@ __device__ __forceinline__ void warp_scan_boxes4(const Box &box, uint32_t want, 
     cnt.scans += area ? 1 : 0;
     cnt.scan_cells += area;
   }
+  if (!__any_sync(kFull, area != 0u)) return;
   if (area > kScanInline) {
     uint32_t at = 0;
     if ((lane & 7u) == 0) {
@@ -991,16 +992,14 @@ __device__ __noinline__ uint32_t walk_los_steps(const uint32_t *__restrict__ bnd
 __device__ float d_cross[kCrossTableLen];
 
 // In closed form (dda_columns.cuh), lane i of the eight taking columns i, i +
-// 8, ..., four at a time (kColumnRun columns a group): all bitmap words of a
-// run are loaded together, and no step waits for the one before.
-constexpr int kColumnRun = 32;
-__device__ __forceinline__ uint32_t walk_los(const uint32_t *__restrict__ bnd, const float *cross, int W,
-                                             int fx, int fy, int tx, int ty, bool on, uint32_t lane) {
+// 8, ..., kRuns at a time: all bitmap words of a run of 8 kRuns columns are
+// loaded together, and no step waits for the one before.
+template <int kRuns>
+__device__ __forceinline__ uint32_t walk_los_runs(const uint32_t *__restrict__ bnd, const float *cross, int W,
+                                                  int fx, int fy, int tx, int ty, bool on, uint32_t lane) {
   const int dx = tx - fx, dy = ty - fy;
   const int adx = abs(dx), ady = abs(dy);
   const int P = max(adx, ady), Q = min(adx, ady);
-  if (__any_sync(kFull, on && (P > kColumnsMax || P == 0)))
-    return walk_los_steps(bnd, W, fx, fy, tx, ty, on, lane);
   const int sx = dx < 0 ? -1 : 1, sy = dy < 0 ? -W : W;
   const int step_p = adx >= ady ? sx : sy, step_q = adx >= ady ? sy : sx;
   const uint32_t start = (uint32_t)fx + (uint32_t)fy * (uint32_t)W;  // grids below 2^32 cells
@@ -1008,12 +1007,12 @@ __device__ __forceinline__ uint32_t walk_los(const uint32_t *__restrict__ bnd, c
   const uint32_t k = lane & 7u, g0 = lane & 24u;
   const int last = on ? P : -1;
   uint32_t D = 0, los = 0;  // diagonal steps so far; the result once blocked
-  for (int c0 = 0; __any_sync(kFull, c0 <= last && !los); c0 += kColumnRun) {
+  for (int c0 = 0; kRuns == 1 ? c0 == 0 : __any_sync(kFull, c0 <= last && !los); c0 += 8 * kRuns) {
     uint32_t hit_in = 0, hit_out = 0, diags = 0;  // bit b: column c0 + 8 b + k
-    uint32_t ia[4], wa[4], wb[4];
-    int two[4];
+    uint32_t ia[kRuns], wa[kRuns], wb[kRuns];
+    int two[kRuns];
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
+    for (int b = 0; b < kRuns; ++b) {
       const int c = c0 + 8 * b + (int)k;
       wa[b] = wb[b] = 0u;
       ia[b] = 0u;
@@ -1029,8 +1028,11 @@ __device__ __forceinline__ uint32_t walk_los(const uint32_t *__restrict__ bnd, c
         wb[b] = __ldg(bnd + ((ia[b] + (uint32_t)two[b]) >> 5));
       }
     }
+    uint32_t dm[kRuns];  // the cell's diagonal steps, a byte per eight columns
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
+    for (int b = 0; b < kRuns; ++b) dm[b] = (__ballot_sync(kFull, (diags >> b) & 1u) >> g0) & 0xFFu;
+#pragma unroll
+    for (int b = 0; b < kRuns; ++b) {
       hit_in |= ((wa[b] >> (ia[b] & 31u)) & 1u) << b;
       hit_out |= ((wb[b] >> ((ia[b] + (uint32_t)two[b]) & 31u)) & 1u) << b;
     }
@@ -1043,10 +1045,9 @@ __device__ __forceinline__ uint32_t walk_los(const uint32_t *__restrict__ bnd, c
       for (int o = 1; o < 8; o <<= 1) first = min(first, __shfl_xor_sync(kFull, first, o));
       uint32_t before = 0;  // diagonal steps up to and including that column
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const uint32_t m = (__ballot_sync(kFull, (diags >> b) & 1u) >> g0) & 0xFFu;
+      for (int b = 0; b < kRuns; ++b) {
         const int upto = (int)first - 8 * b;  // bits 0 .. upto count
-        before += (uint32_t)__popc(upto >= 7 ? m : upto >= 0 ? m & ((2u << upto) - 1u) : 0u);
+        before += (uint32_t)__popc(upto >= 7 ? dm[b] : upto >= 0 ? dm[b] & ((2u << upto) - 1u) : 0u);
       }
       const uint32_t in_hits = __shfl_sync(kFull, hit_in, g0 + (first & 7u));
       if (first != 0xFFFFu && !los) {
@@ -1058,9 +1059,21 @@ __device__ __forceinline__ uint32_t walk_los(const uint32_t *__restrict__ bnd, c
       }
     }
 #pragma unroll
-    for (int b = 0; b < 4; ++b) D += (uint32_t)__popc((__ballot_sync(kFull, (diags >> b) & 1u) >> g0) & 0xFFu);
+    for (int b = 0; b < kRuns; ++b) D += (uint32_t)__popc(dm[b]);
   }
   return los ? los : (uint32_t)(P + Q + 1) - D;
+}
+
+// Walks of up to eight columns (the usual ones on rough ground) take the
+// single-run code: a third of the instructions.
+__device__ __forceinline__ uint32_t walk_los(const uint32_t *__restrict__ bnd, const float *cross, int W,
+                                             int fx, int fy, int tx, int ty, bool on, uint32_t lane) {
+  const int P = max(abs(tx - fx), abs(ty - fy));
+  if (!__any_sync(kFull, on && (uint32_t)(P - 1) > 6u))
+    return walk_los_runs<1>(bnd, cross, W, fx, fy, tx, ty, on, lane);
+  if (__any_sync(kFull, on && (uint32_t)(P - 1) >= (uint32_t)kColumnsMax))
+    return walk_los_steps(bnd, W, fx, fy, tx, ty, on, lane);
+  return walk_los_runs<4>(bnd, cross, W, fx, fy, tx, ty, on, lane);
 }
 
 // One tile launch with the state in global memory, by a team of R CTAs
@@ -1176,7 +1189,7 @@ __device__ __forceinline__ bool tile_global(const JobDev &j, const DirConst &dc,
       // improvements of the same cells (ordered by the barrier below)
       if (c0 == 0)
         for (uint32_t u = threadIdx.x; u < prev_upd; u += blockDim.x) {
-          CellState e = get_update(sm_upd + (p ^ 1) * kTileUpdSmem, s.upd + ((size_t)(p ^ 1) * R + rank) * cap, u);
+          const CellState e = get_update(sm_upd + (p ^ 1) * kTileUpdSmem, s.upd + ((size_t)(p ^ 1) * R + rank) * cap, u);
           uint32_t col;
           const uint32_t row = tb.by_tw.div(e.pad, col);
           st_state(ws + ((uint32_t)x0 + col + ((uint32_t)y0 + row) * (uint32_t)h.W), e);
@@ -1226,17 +1239,19 @@ __device__ __forceinline__ bool tile_global(const JobDev &j, const DirConst &dc,
         if (!__any_sync(kFull, improved)) continue;
         // referrer box (whole with a pending bitmap: referrers anywhere mark
         // pending cells; else clipped to the tile grown by one cell)
-        Box box;
-        box.x0 = (int)__shfl_sync(kFull, corner, g0);
-        box.y0 = (int)__shfl_sync(kFull, corner, g0 + 1);
-        box.x1 = (int)__shfl_sync(kFull, corner, g0 + 2);
-        box.y1 = (int)__shfl_sync(kFull, corner, g0 + 3);
-        if (!improved || (uint32_t)box.x0 == kEmptyBox)
-          box = Box{1, 1, 0, 0};
-        else if (pending)
-          box = Box{max(box.x0, 0), max(box.y0, 0), min(box.x1, j.W - 1), min(box.y1, j.H - 1)};
-        else
-          box = clip_box(box.x0, box.y0, box.x1, box.y1, x0, y0, TW, TH, j.W, j.H);
+        Box box{1, 1, 0, 0};
+        if (__any_sync(kFull, improved && k8 == 0 && corner != kEmptyBox)) {
+          box.x0 = (int)__shfl_sync(kFull, corner, g0);
+          box.y0 = (int)__shfl_sync(kFull, corner, g0 + 1);
+          box.x1 = (int)__shfl_sync(kFull, corner, g0 + 2);
+          box.y1 = (int)__shfl_sync(kFull, corner, g0 + 3);
+          if (!improved || (uint32_t)box.x0 == kEmptyBox)
+            box = Box{1, 1, 0, 0};
+          else if (pending)
+            box = Box{max(box.x0, 0), max(box.y0, 0), min(box.x1, h.W - 1), min(box.y1, h.H - 1)};
+          else
+            box = clip_box(box.x0, box.y0, box.x1, box.y1, x0, y0, TW, TH, h.W, h.H);
+        }
         const uint32_t los = walk_los(bnd, cross, h.W, x, y, ref_x(b.ref), ref_y(b.ref), improved, lane);
         const uint32_t adds = __ballot_sync(kFull, improved && k8 == 0);
         uint32_t ai = 0;
@@ -1254,10 +1269,11 @@ __device__ __forceinline__ bool tile_global(const JobDev &j, const DirConst &dc,
           }
           // the reference's box grows to hold (x, y), a corner a lane
           const uint32_t rc = (uint32_t)ref_x(b.ref) + (uint32_t)ref_y(b.ref) * (uint32_t)h.W;
-          if (k8 == 0) atomicMin(j.box_x0 + 4 * (size_t)rc, (uint32_t)x);
-          if (k8 == 1) atomicMin(j.box_y0 + rc, (uint32_t)y);
-          if (k8 == 2) atomicMax(j.box_x1 + rc, (uint32_t)x);
-          if (k8 == 3) atomicMax(j.box_y1 + rc, (uint32_t)y);
+          const uint32_t at = k8 & 1u ? (uint32_t)y : (uint32_t)x;
+          if (k8 < 2)
+            atomicMin(k8 == 0 ? j.box_x0 + 4 * (size_t)rc : j.box_y0 + rc, at);
+          else if (k8 < 4)
+            atomicMax(k8 == 2 ? j.box_x1 + rc : j.box_y1 + rc, at);
           // only a burning cell is read by its neighbours
           if (b.time < h.max_time && own_speed != 0.0f) {
             if (k8 < 6) tb.mark_half(dirty_next, lx, ly, (int)(k8 >> 1), (int)(k8 & 1u));
