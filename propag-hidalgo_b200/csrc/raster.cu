@@ -7,9 +7,10 @@
 // only parses the WKB and turns it into a pixel-space plan (raster.hpp); the
 // work that grows with the grid runs on the device in three passes:
 //   1. every cell of a winner raster (int32) is set to -1;
-//   2. segment samples (one thread each) and polygon rows (one CTA each: the
-//      row's edge crossings toggle bits of a shared-memory row mask, a prefix
-//      XOR over the mask gives the even-odd inside test) raise the cells they
+//   2. segment samples (one thread each) and polygon rows (eight threads to
+//      a CTA each, by the grid's width: the row's edge crossings toggle bits of
+//      a shared-memory row mask, a prefix XOR over the mask gives the even-odd
+//      inside test) raise the cells they
 //      burn to their feature's index with atomicMax -- the largest index is
 //      the last feature in burn order, whatever order the threads run in;
 //   3. each cell takes its winner's value (a time, or a fuel code) or nodata.
@@ -44,10 +45,8 @@ cudaError_t launch_rasterize_winner(const RasterPlanDev &p, int64_t W, int64_t H
     segment_kernel<<<grid_for((p.samples + kRasterThreads - 1) / kRasterThreads, sm_count, 8),
                      kRasterThreads, 0, stream>>>(p.segs, p.nseg, p.samples, W, H, win);
   if (p.rows)
-    polygon_kernel<<<grid_for(W <= 32 * (int64_t)kWarpRowWords ? (p.rows + kRasterWarps - 1) / kRasterWarps : p.rows,
-                             sm_count, 8),
-                     kRasterThreads, 0, stream>>>(
-        p.polys, p.npoly, p.rows, p.edges, W, win);
+    polygon_kernel<<<grid_for((p.rows * polygon_row_threads(W) + kRasterThreads - 1) / kRasterThreads, sm_count, 8),
+                     kRasterThreads, 0, stream>>>(p.polys, p.npoly, p.rows, p.edges, W, win);
   return cudaGetLastError();
 }
 

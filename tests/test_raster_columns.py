@@ -1,7 +1,7 @@
 """Polygon rows over the polygon's own columns (csrc/raster_kernels.cuh), at the
 forms where the columns could be cut wrongly: polygons left and right of the
 grid and across its edges, vertices far away, infinite and NaN vertices, on
-grids with a warp and with a CTA to a row (8192 and 8193 columns).  The emulated
+grids with eight threads, a warp and a CTA to a row (up to 4096, up to 16384, more).  The emulated
 kernels' rasters equal the host rasteriser's, which looks at every column."""
 import ctypes as C
 
@@ -30,7 +30,7 @@ def _rings(w, h, rng):
     return rings
 
 
-@pytest.mark.parametrize("w", [70, 8192, 8193])
+@pytest.mark.parametrize("w", [70, 4096, 4097, 8192, 8193, 16384, 16385])
 def test_polygon_columns(L, emul, w):  # noqa: F811
     h = 5
     g = georef(L, w, h, (0.0, 1.0, 0.0, 0.0, 0.0, 1.0))
