@@ -1078,7 +1078,7 @@ __device__ __forceinline__ uint32_t walk_los(const uint32_t *__restrict__ bnd, c
 
 // One tile launch with the state in global memory, by a team of R CTAs
 // (this one is `rank`).  `list` is shared memory for blockDim.x * 32 entries,
-// `sm_upd` for two sweeps' kTileUpdSmem update entries, `cta_ctr` five shared
+// `sm_upd` for two sweeps' kTileUpdSmem update entries, `cta_ctr` six shared
 // counters, `queue` kScanQueue boxes, `cross` the crossing times of the line-of-sight walks.  Returns
 // whether any sweep improved a cell.
 //
@@ -1135,7 +1135,7 @@ __device__ __forceinline__ bool tile_global(const JobDev &j, const DirConst &dc,
   uint32_t q = 0;  // list counter of this chunk: cta_ctr[q]
   int p = 0;       // sweep parity: read X[p], write X[p ^ 1]
   if (threadIdx.x < 1)
-    for (int i = 0; i < 5; ++i) cta_ctr[i] = 0u;
+    for (int i = 0; i < 6; ++i) cta_ctr[i] = 0u;
   __syncthreads();
   for (;;) {
     ++cx.sweeps;  // every thread counts, so the abort below is uniform
@@ -1158,6 +1158,7 @@ __device__ __forceinline__ bool tile_global(const JobDev &j, const DirConst &dc,
     };
     for (uint32_t c0 = 0; c0 < tb.wpo; c0 += chunk) {
       if (c0) __syncthreads();  // the previous chunk's list is consumed
+      if (threadIdx.x == 0) cta_ctr[5] = 0u;
       const uint32_t c1 = min(tb.wpo, c0 + chunk);
       // ---- 1: this CTA's marked cells into the list ----
       if (!first) {
@@ -1206,7 +1207,17 @@ __device__ __forceinline__ bool tile_global(const JobDev &j, const DirConst &dc,
       // ---- 2: evaluate and commit, up to four cells a warp, spread over the
       // CTA's warps (a warp's walks and scans take as long as its longest) ----
       const uint32_t per = min(4u, (nlist + nwarps - 1) / nwarps);
-      for (uint32_t base = warp * per; base < nlist; base += nwarps * per) {
+      // Longer lists go on with whichever warp is done first: fours differ by
+      // their walks and scans, and the CTA waits for its last warp (teams of a
+      // few CTAs: 64 scenarios 132/159/260 -> 129/156/253 ms; 4096 x 4096
+      // 160/171/179 -> 155/165/179 ms; short lists are not touched).
+      auto next_four = [&]() -> uint32_t {
+        if (nlist <= 4u * nwarps) return nlist;
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(cta_ctr + 5, 4u);
+        return 4u * nwarps + __shfl_sync(kFull, at, 0);
+      };
+      for (uint32_t base = warp * per; base < nlist; base = next_four()) {
         const uint32_t ci = base + (lane >> 3);
         const bool valid = (lane >> 3) < per && ci < nlist;
         uint32_t k = 0;
@@ -1817,7 +1828,7 @@ __global__ void __launch_bounds__(kEngineThreads, 1)
   __shared__ ScanBox scan_boxes[kEngineThreads];  // or the scan queue of global-memory tiles
   static_assert(sizeof(ScanItem) * kScanQueue <= sizeof(ScanBox) * kEngineThreads, "the scan queue fits");
   __shared__ int team_ok[2];
-  __shared__ uint32_t cta_ctr[5];  // global-memory tiles: work-list and update counts (two each), scan queue
+  __shared__ uint32_t cta_ctr[6];  // global-memory tiles: work-list and update counts (two each), scan queue, cells taken
   Team<kGroup> team{reinterpret_cast<unsigned long long *>(s.ctr + 8), queue + 1, team_ok, csize};
   team.cnt3 = s.ctr + 5;  // cluster mode: slot counters 5..7
   team.cnt_leader = rank == 0;
@@ -1996,7 +2007,7 @@ __global__ void __launch_bounds__(kEngineThreads, 1)
   __shared__ JobDev js;
   __shared__ ScanItem queue[kScanQueue];
   __shared__ int team_ok[2];
-  __shared__ uint32_t cta_ctr[5];
+  __shared__ uint32_t cta_ctr[6];
   Team<true> team{reinterpret_cast<unsigned long long *>(s.ctr + 8), err, team_ok, group};
   float *const cross = reinterpret_cast<float *>(dyn_smem + global_tile_cross_off(blockDim.x));
   uint32_t *const list = reinterpret_cast<uint32_t *>(dyn_smem);  // between launches: the leader's copy of w.done
