@@ -164,8 +164,10 @@ typedef struct PropagIgnition {
  * team keeps its tiles in global memory and meets at a counter barrier in
  * global memory whose waits are bounded (a wait that gives up fails the run
  * with PROPAG_ERR_TIMEOUT).  One scenario then runs on the whole device
- * instead of one cluster.  cluster = 0 chooses group mode with teams of
- * max(4, CTAs / scenarios).  Results are identical in every mode. */
+ * instead of one cluster.  cluster = 0 chooses group mode with the
+ * team size that an estimate of the batch's length favours, and runs a lone
+ * scenario of at least four tiles a side with several teams on independent
+ * tiles.  Results are identical in every mode. */
 #define PROPAG_CLUSTER_GROUPS (-1)
 
 /* Self-test of group mode's bounded wait (no reference counterpart): runs an
@@ -275,8 +277,8 @@ typedef struct propag_engine propag_engine;
 propag_engine *propag_engine_create(const PropagOptions *opt);
 
 /* Device scratch the engine holds for one job of width x height cells
- * (references, referrer boxes, travel-time planes, second state copy,
- * boundary and pending bitmaps: about 60 bytes per cell), as a run lays it
+ * (fire and state records in two copies or travel-time planes, referrer
+ * boxes, boundary and pending bitmaps: about 60 bytes per cell), as a run lays it
  * out; the server admits requests by it.  No counterpart in the reference. */
 uint64_t propag_engine_job_bytes(uint32_t width, uint32_t height);
 void propag_engine_destroy(propag_engine *engine);

@@ -20,7 +20,9 @@
 //     propag.cu:221-224).  Each cell keeps the bounding box of the cells that
 //     ever adopted it as their reference, so those referrers are found by
 //     scanning that box only.
-// The first sweep of each tile launch evaluates the whole tile.
+// The first sweep of a tile launch evaluates the whole tile (shared-memory
+// tiles) or its pending cells, those whose inputs changed since their last
+// evaluation (global-memory tiles).
 //
 // Mapping.  The engine is one persistent launch whose CTAs form teams; a
 // team works on one scenario at a time and pulls scenarios from a queue
@@ -38,7 +40,10 @@
 //     teams of any size (the whole device for one scenario).  The tile state
 //     stays in global memory in two copies, so that a sweep is one phase; the
 //     team meets at a counter barrier in global memory whose wait is bounded
-//     (the engine's only spin-wait; see Team).
+//     (see Team).  A lone scenario of enough tiles is run by several teams
+//     (waves_kernel): tile launches that cannot read each other's cells run at
+//     the same time, and a team's wait for the launches it depends on is
+//     bounded too.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
