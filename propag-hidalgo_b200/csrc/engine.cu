@@ -1673,21 +1673,42 @@ __device__ bool tile_smem(const JobDev &j, const DirConst &dc, char *smem, const
       cx.improvements += total;
     }
     const uint32_t nupd = sm.ctr[1];
-    // updates dealt `per` to a warp (see tile_global)
-    const uint32_t nwarps = blockDim.x >> 5;
-    const uint32_t per = min(32u, (nupd + nwarps - 1) / nwarps);
-    for (uint32_t base = (threadIdx.x >> 5) * per; base < nupd; base += nwarps * per) {
+    // Some of the warps commit, the others walk the lines of sight to the
+    // adopted references (read by other CTAs after the barrier below): both are
+    // chains of latencies, a few dozen updates a CTA, and need nothing of each
+    // other.  Six and ten of 16: a warp commits up to 32 updates at once, but
+    // walks four.  512 x 512 on 16 CTAs, three seeds: 13.1 / 18.3 / 8.9 ms with
+    // every warp doing both in turn, 12.1 / 16.6 / 7.8 so (12.2 / 17.0 / 7.8 with
+    // eight and eight, 12.2 / 16.3 / 7.8 with four and twelve).
+    const uint32_t nwarps = blockDim.x >> 5, warp = threadIdx.x >> 5;
+    const uint32_t committers = max(nwarps * 3 / 8, 1u), walkers = max(nwarps - committers, 1u);
+    const uint32_t walker = nwarps == 1 ? 0u : warp - committers;  // past `walkers` for the others
+    if (walker < walkers) {
+      const uint32_t four = min(4u, (nupd + walkers - 1) / walkers);
+      for (uint32_t base = walker * four; base < nupd; base += walkers * four) {
+        const uint32_t u = base + (lane >> 3);
+        const bool on = (lane >> 3) < four && u < nupd;
+        uint32_t s = 0, r = 0;
+        float t;
+        if (on) upd_get(sm, u, s, t, r);
+        const int lr = g.div_p((int)s), x = g.x0 - 1 + (int)s - lr * g.P, y = g.y0 - 1 + g.rank + lr * g.C;
+        const uint32_t los = walk_los(j.bnd, cross, j.W, x, y, ref_x(r), ref_y(r), on, lane);
+        if (on && (lane & 7u) == 0) __stcg(j.los + (uint32_t)x + (uint32_t)y * (uint32_t)j.W, los);
+      }
+    }
+    const uint32_t per = min(32u, (nupd + committers - 1) / committers);
+    for (uint32_t base = warp * per; warp < committers && base < nupd; base += committers * per) {
       const uint32_t u = base + lane;
       const bool valid = lane < per && u < nupd;
-      uint32_t want = 0, adopted = 0;
+      uint32_t want = 0;
       Box box{1, 1, 0, 0};
       if (valid) {
         uint32_t s, r;
         float t;
         upd_get(sm, u, s, t, r);
-        adopted = r;
         const int lr = g.div_p((int)s), hx = (int)s - lr * g.P, hy = g.rank + lr * g.C;
         const int x = g.x0 - 1 + hx, y = g.y0 - 1 + hy;
+        const float own_speed = __ldg(j.speed + x + (int64_t)y * j.W);  // on its way during the rest
         sm.time[s] = t;
         sm.ref[s] = r;
         // referrer box of r: the staged box inside the staged region (merged
@@ -1707,8 +1728,7 @@ __device__ bool tile_smem(const JobDev &j, const DirConst &dc, char *smem, const
           box_expand_global(j, r, x, y);
         }
         // only a burning cell is read by its neighbours
-        if (t < j.max_time && __ldg(j.speed + x + (int64_t)y * j.W) != 0.0f)
-          mark3x3_smem(sm, g, hx, hy);
+        if (t < j.max_time && own_speed != 0.0f) mark3x3_smem(sm, g, hx, hy);
         want = pack_ref(x, y);
         const BoxT pb = sbox[s];
         if (pb != B::kEmpty) {
@@ -1719,15 +1739,6 @@ __device__ bool tile_smem(const JobDev &j, const DirConst &dc, char *smem, const
           box = clip_box(g.x0 - 1 + bx0, g.y0 - 1 + by0, g.x0 - 1 + bx1, g.y0 - 1 + by1, g.x0, g.y0,
                          g.TW, g.TH, j.W, j.H);
         }
-      }
-      // the lines of sight to the adopted references, four cells at a time
-      // (eight lanes each; read by other CTAs after the barrier below)
-      for (uint32_t i = 0; i < per; i += 4) {
-        const uint32_t from = i + (lane >> 3);
-        const uint32_t c = __shfl_sync(kFull, want, (int)(from & 31u)), r = __shfl_sync(kFull, adopted, (int)(from & 31u));
-        const bool on = from < per && base + from < nupd;
-        const uint32_t los = walk_los(j.bnd, cross, j.W, ref_x(c), ref_y(c), ref_x(r), ref_y(r), on, lane);
-        if (on && (lane & 7u) == 0) __stcg(j.los + (uint32_t)ref_x(c) + (uint32_t)ref_y(c) * (uint32_t)j.W, los);
       }
       warp_scan_boxes(
           scan_boxes + (threadIdx.x & ~31u), box, want, j, lane, cnt,
