@@ -1948,8 +1948,7 @@ __global__ void __launch_bounds__(kEngineThreads, 1)
 //
 // Why: a sweep is a chain of latencies whose length hardly depends on the CTAs
 // that share it, and one tile's front is too small for 148 of them.  4096^2, 20
-// ignitions: 381 ms in sequence, 168 ms with four teams of 37 CTAs; 777 x 1283
-// in tiles of 190, 5 ignitions: 63 and 44 ms.
+// ignitions: 445 ms in sequence, 199 ms with four teams of 37 CTAs.
 constexpr uint32_t kWaveStop = 0xFFFFFFFFu, kWaveIdle = 0xFFFFFFFEu;
 constexpr unsigned long long kWavePickNs = 1000000ull;       // 1 ms: a team's members wait that long at their barrier
 constexpr unsigned long long kWaveStallNs = 20000000000ull;  // 20 s without a launch done anywhere
