@@ -162,7 +162,8 @@ __device__ __forceinline__ int dm_prob(const DmoistTables &T, float t, float s, 
 }
 
 // What the shading correction takes from the hour and month alone: the
-// table's season and hour columns, and whether the cloud cover counts.
+// table's season and hour columns, and whether the cloud cover counts.  (A
+// month outside 1..12 has no season: DmoistRows::shaded.)
 struct DmoistHour {
   int mi, hi;
   bool dark;  // fully shaded whatever the clouds
@@ -266,6 +267,7 @@ struct DmoistRows {
   const float *pp[6];
   DmoistHour h[3];
   int hour, season;  // season: row of the precipitation table
+  bool shaded;       // the month has a shading correction (1..12)
 };
 __device__ __forceinline__ DmoistRows dmoist_rows(const DmoistIn &in, uint64_t n, int hour, int month) {
   DmoistRows r;
@@ -282,6 +284,7 @@ __device__ __forceinline__ DmoistRows dmoist_rows(const DmoistIn &in, uint64_t n
   for (int d = 0; d < 6; ++d) r.pp[d] = in.pp + (uint64_t)d * n;
   r.hour = hour;
   r.season = (month >= 4 && month <= 10) ? 0 : 1;
+  r.shaded = month >= 1 && month <= 12;
   return r;
 }
 
@@ -312,15 +315,16 @@ __device__ __forceinline__ void dmoist_cell(const DmoistShared &T, const DmoistR
 #pragma unroll
   for (int d = 0; d < 6; ++d) ppmax = fmaxf(ppmax, dm_pp_effect(T.t, in.season, pp[d], d));
   const float *const ratio = T.ratio[dm_precip_class(ppmax)];
-  const int oi = dm_exposure(slope, aspect);
+  const int oi = in.shaded ? dm_exposure(slope, aspect) : -1;
   float m1[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     const DmoistHour &h = in.h[k];
     const float s = dm_shading(cc[k], fuel);
     const int shi = h.dark || !(s < 50.0f) ? 1 : 0;
-    // a cell without an exposure row has no corrected class (NaN in the
-    // reference): it takes neither a probability nor the 30 % of a positive one
+    // a cell without an exposure row, or in a month the correction does not
+    // know, has no corrected class (NaN in the reference): it takes neither a
+    // probability nor the 30 % of a positive one
     float hcs = 0.0f;
     if (fuel != 0 && oi >= 0) hcs = (float)(dm_hcb(T.t, t[k], rh[k]) + T.t.shade[h.mi][shi][oi][h.hi]);
     const int p = dm_prob(T.t, t[k], s, hcs, fuel);
