@@ -54,6 +54,7 @@
 #include "dda_columns.cuh"
 #include "engine.cuh"
 #include "propag_device.cuh"
+#include "tile_index.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -1478,12 +1479,10 @@ struct SmemGeom {
   int x0, y0, TW, TH, P, HR, C, rank, rows_mine;
   int sh;    // box_shift: 0 when the halo side fits a byte, else 1
   int lc;    // log2 C (cluster sizes are powers of two): row hy -> CTA hy & (C-1), local row hy >> lc
-  uint32_t pm;  // ceil(2^32 / P): s / P = umulhi(s, pm), exact for s < 2^16 and P < 2^12
+  uint32_t pm, tm;  // recip_of(P), recip_of(TW)
   __device__ __forceinline__ int owner(int hy) const { return hy & (C - 1); }
   __device__ __forceinline__ int lrow(int hy) const { return hy >> lc; }
-  uint32_t tm;  // the same for TW
-  __device__ __forceinline__ int div_p(int s) const { return (int)__umulhi((uint32_t)s, pm); }
-  __device__ __forceinline__ int div_tw(int s) const { return (int)__umulhi((uint32_t)s, tm); }
+  __device__ __forceinline__ int div_p(int s) const { return (int)div_wide((uint32_t)s, pm); }
 };
 
 template <typename T>
@@ -1568,8 +1567,8 @@ __device__ bool tile_smem(const JobDev &j, const DirConst &dc, char *smem, const
   g.HR = td.TH + 2;
   g.C = (int)cluster.num_blocks();
   g.lc = __ffs(g.C) - 1;
-  g.pm = (uint32_t)(0xFFFFFFFFu / (uint32_t)g.P) + 1u;
-  g.tm = (uint32_t)(0xFFFFFFFFu / (uint32_t)g.TW) + 1u;
+  g.pm = recip_of((uint32_t)g.P);
+  g.tm = recip_of((uint32_t)g.TW);
   g.rank = (int)cluster.block_rank();
   g.rows_mine = g.HR > g.rank ? (g.HR - g.rank + g.C - 1) / g.C : 0;
   g.sh = (sizeof(BoxT) == 4 && (g.P > 256 || g.HR > 256)) ? 1 : 0;
@@ -1620,10 +1619,8 @@ __device__ bool tile_smem(const JobDev &j, const DirConst &dc, char *smem, const
   for (;;) {
     ++cx.sweeps;
     // ---- evaluate: this CTA's list (all its tile cells, or its marks) ----
-    // The first sweep's list is implicit: the in-tile rows of this CTA
-    // (local rows lr_first ..), TW cells each.
-    const int lr_first = g.rank == 0 ? 1 : 0;
-    const int in_rows = g.TH >= g.rank ? max((g.TH - g.rank) / g.C - lr_first + 1, 0) : 0;
+    // The first sweep's list is implicit: the in-tile rows of this CTA, TW
+    // cells each.
     if (!first) {
       for (int w0 = (int)(threadIdx.x & ~31u); w0 < nwords; w0 += blockDim.x) {
         const int w = w0 + (int)lane;
@@ -1637,7 +1634,7 @@ __device__ bool tile_smem(const JobDev &j, const DirConst &dc, char *smem, const
       }
     }
     __syncthreads();
-    const uint32_t nlist = first ? (uint32_t)(in_rows * g.TW) : sm.ctr[0];
+    const uint32_t nlist = first ? (uint32_t)(own_rows(g.TH, g.rank, g.C) * g.TW) : sm.ctr[0];
     if (threadIdx.x == 0) cnt.evals += nlist;
     // four cells per warp, eight lanes per cell
     for (uint32_t base = (threadIdx.x >> 5) * 4; base < nlist; base += (blockDim.x >> 5) * 4) {
@@ -1647,8 +1644,7 @@ __device__ bool tile_smem(const JobDev &j, const DirConst &dc, char *smem, const
       int x = 0, y = 0;
       Best own{FLT_MAX, kNoRef};
       if (valid) {
-        s = first ? (uint32_t)((lr_first + g.div_tw((int)ci)) * g.P + 1 + ((int)ci - g.div_tw((int)ci) * g.TW))
-                  : list_get(sm, ci);
+        s = first ? (uint32_t)own_slot((int)ci, g.rank, g.P, g.tm) : list_get(sm, ci);
         const int lr = g.div_p((int)s), hx = (int)s - lr * g.P, hy = g.rank + lr * g.C;
         x = g.x0 - 1 + hx;
         y = g.y0 - 1 + hy;
