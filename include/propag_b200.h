@@ -256,7 +256,7 @@ typedef struct PropagJob {
   uint32_t height;
   float dx;
   float dy;
-  float max_time;
+  float max_time; /* s; infinity: no limit */
   int32_t tile; /* 0 = the engine's default */
   const float *speed_max;
   const float *azimuth_max;

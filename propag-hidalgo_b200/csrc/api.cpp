@@ -441,7 +441,7 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
     d.H = (int)j.height;
     d.gdx = j.dx;
     d.gdy = j.dy;
-    d.max_time = j.max_time;
+    d.max_time = time_limit(j.max_time);
     d.T = T;
     d.TX = (int)((j.width + T - 1) / T);
     d.TY = (int)((j.height + T - 1) / T);
@@ -1075,7 +1075,7 @@ extern "C" int propag_run_device_static(const PropagJob *job, void *stream_ptr, 
   d.H = (int)j.height;
   d.gdx = j.dx;
   d.gdy = j.dy;
-  d.max_time = j.max_time;
+  d.max_time = time_limit(j.max_time);
   d.T = T;
   d.TX = (int)((j.width + T - 1) / T);
   d.TY = (int)((j.height + T - 1) / T);

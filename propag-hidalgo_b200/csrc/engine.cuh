@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cfloat>
 #include <cstdint>
 
 #include "dda_columns.cuh"
@@ -24,10 +25,17 @@ constexpr uint32_t kLosBlocked = 0x80000000u;
 // visits it twice, or meets a boundary at once.
 __host__ __device__ inline uint32_t los_of_self(bool boundary) { return boundary ? kLosBlocked | 1u : 2u; }
 
+// JobDev::max_time of a caller's limit.  A cell that has not burned has the time
+// FLT_MAX and no reference, and the kernels follow the reference of every cell
+// whose time is below the limit: infinity (no limit) becomes FLT_MAX, below
+// which every time of a burned cell lies.
+inline float time_limit(float max_time) { return max_time > FLT_MAX ? FLT_MAX : max_time; }
+
 // One scenario as the device sees it.
 struct JobDev {
   int32_t W, H;
-  float gdx, gdy, max_time;
+  float gdx, gdy;
+  float max_time;  // time_limit: at most FLT_MAX
   int32_t T;       // tile side in cells (>= max(W, H) means one tile)
   int32_t TX, TY;  // tiles per axis
   int32_t north_up;
