@@ -223,11 +223,14 @@ struct propag_engine {
   int csize = 0;    // 0 = auto, PROPAG_CLUSTER_GROUPS = teams of CTAs without clusters
   bool auto_groups = true;  // auto may choose group mode (needs the whole device)
   uint32_t phantom = 0;     // self-test only: CTAs a group-mode team waits for in vain
+  int64_t wave_hold = -1;   // self-test only: a tile that no team of a waves run may take
+  uint64_t wave_stall_ns = kWaveStallNs;
   int threads = 512;  // the engine kernel's launch bound
   int default_tile = PROPAG_DEFAULT_TILE;
   size_t smem_budget = 200 * 1024;  // dynamic shared memory per CTA for resident tiles
   int last_cluster = 0;             // cluster size and shared memory of the last run
   uint32_t last_group = 0;          // CTAs per team of the last run (group mode), else 0
+  uint32_t last_teams = 0;          // teams that shared the last run's lone job (waves), else 0
   size_t last_smem = 0;
   cudaStream_t stream = nullptr;  // the stream of the last run
   DevBuf job_scratch, slot_scratch, meta;
@@ -597,6 +600,7 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
   e->last_cluster = group ? PROPAG_CLUSTER_GROUPS : csize;
   e->last_group = group;
   e->last_smem = smem;
+  e->last_teams = waves.teams;
   // global-memory tiles: each CTA of a team has its own words of the dirty
   // bitmap and its own update region
   const size_t team_ctas = group ? group : (size_t)csize;
@@ -677,6 +681,8 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
     wave.sweeps = wave.worked + align_up(kWaveRounds, 64);
     wave.tiles = (uint32_t)tiles;
     wave.window = waves.window;
+    wave.stall_ns = e->wave_stall_ns;
+    if (e->wave_hold >= 0) CK(cudaMemsetAsync(wave.claim + e->wave_hold, 0xFF, sizeof(uint32_t), stream));
   }
   // ---- kernels ----
   if (live) CK(cudaEventRecord(e->ev[0], stream));
@@ -765,6 +771,34 @@ extern "C" int propag_selftest_group_wait(uint32_t *status) {
     PropagStats st{};
     rc = engine_run(e, &j, 1, nullptr, &st);
     *status = st.status;
+  }
+  propag_engine_destroy(e);
+  return rc;
+}
+
+extern "C" int propag_selftest_wave_wait(const PropagJob *job, int64_t hold, uint32_t limit_ms, PropagStats stats[2]) {
+  if (!job || !stats) return fail(PROPAG_ERR_INVALID, "null job or stats");
+  stats[0] = stats[1] = PropagStats{};
+  const int rc0 = ensure_device(-1, nullptr);  // no device: PROPAG_ERR_NO_DEVICE
+  if (rc0) return rc0;
+  // both runs' grid and tiles, checked before a tile is held
+  const uint32_t T = job->tile > 0 ? (uint32_t)job->tile : PROPAG_DEFAULT_TILE;
+  const uint64_t tiles = (uint64_t)((job->width + T - 1) / T) * (uint64_t)((job->height + T - 1) / T);
+  if (hold >= 0 && (uint64_t)hold >= tiles) return fail(PROPAG_ERR_INVALID, "no such tile");
+  propag_engine *e = propag_engine_create(nullptr);
+  if (!e) return PROPAG_ERR_CUDA;  // message set by propag_engine_create
+  e->wave_hold = hold;
+  e->wave_stall_ns = (uint64_t)limit_ms * 1000000ull;
+  int rc = engine_run(e, job, 1, nullptr, &stats[0]);
+  const std::string msg = rc ? g_error : std::string();
+  if (e->last_teams == 0) {
+    if (!rc) rc = fail(PROPAG_ERR_INVALID, "the job is not run by several teams");
+  } else {
+    e->wave_hold = -1;
+    e->wave_stall_ns = kWaveStallNs;
+    const int rc2 = engine_run(e, job, 1, nullptr, &stats[1]);
+    if (rc2) rc = rc2;
+    else if (rc) g_error = msg;
   }
   propag_engine_destroy(e);
   return rc;

@@ -1946,8 +1946,7 @@ __global__ void __launch_bounds__(kEngineThreads, 1)
 // that share it, and one tile's front is too small for 148 of them.  4096^2, 20
 // ignitions: 445 ms in sequence, 199 ms with four teams of 37 CTAs.
 constexpr uint32_t kWaveStop = 0xFFFFFFFFu, kWaveIdle = 0xFFFFFFFEu;
-constexpr unsigned long long kWavePickNs = 1000000ull;       // 1 ms: a team's members wait that long at their barrier
-constexpr unsigned long long kWaveStallNs = 20000000000ull;  // 20 s without a launch done anywhere
+constexpr unsigned long long kWavePickNs = 1000000ull;  // 1 ms: a team's members wait that long at their barrier
 
 // The first launch in sequence that may run and no team has taken: round << 12
 // | tile; kWaveStop when the job is finished (or cannot go on), kWaveIdle when
@@ -2046,7 +2045,7 @@ __global__ void __launch_bounds__(kEngineThreads, 1)
         if (pick != kWaveIdle || done != seen || idle_since == 0) {
           seen = done;
           idle_since = globaltimer_ns();
-        } else if (globaltimer_ns() - idle_since > kWaveStallNs) {
+        } else if (globaltimer_ns() - idle_since > w.stall_ns) {
           atomicOr(err, 1u);
           pick = kWaveStop;
         }

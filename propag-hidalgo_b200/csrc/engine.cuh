@@ -137,7 +137,9 @@ struct WaveDev {
   uint32_t *far;     // [0] a reference lies too far away for `window`; [1] launches done
   uint32_t tiles;
   int32_t window;    // launches of tiles up to this many tiles apart keep their order
+  unsigned long long stall_ns;  // a team that waits this long for other teams' launches gives the run up
 };
+constexpr unsigned long long kWaveStallNs = 20000000000ull;
 constexpr uint32_t kWaveRounds = 1024;  // rounds the words hold
 constexpr uint32_t kWaveTiles = 4096;   // tiles a team's leader looks through
 

@@ -188,6 +188,7 @@ SIGNATURES = {
                                     C.POINTER(PropagStats)]),
     "propag_engine_last_times": (C.c_int, [C.c_void_p, C.POINTER(C.c_float * 3)]),
     "propag_selftest_group_wait": (C.c_int, [C.POINTER(C.c_uint32)]),
+    "propag_selftest_wave_wait": (C.c_int, [C.POINTER(PropagJob), C.c_int64, C.c_uint32, C.POINTER(PropagStats)]),
     "propag_selftest_time_from": (C.c_int, [C.c_int, C.c_uint64] + [C.c_void_p] * 8 +
                                   [C.c_float, C.c_float, C.c_void_p]),
     "propag_selftest_cosf_table": (C.c_int, [C.c_uint32, C.c_uint64, C.c_void_p]),
