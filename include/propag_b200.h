@@ -297,9 +297,9 @@ int propag_engine_last_times(propag_engine *engine, float ms[3]);
 
 /* Self-test of the bounded waits of several teams on one job (no reference
  * counterpart): runs the job twice on one engine, first with the teams' limit
- * of waiting for one another's launches at limit_ms (else 20 s) and, for hold >=
- * 0, with tile `hold` (row-major) kept from every team, so that the launches
- * that depend on it are never ready; then as usual.  stats[0] and stats[1] are
+ * of waiting for one another while no team ends a sweep at limit_ms (else 20 s)
+ * and, for hold >= 0, with tile `hold` (row-major) kept from every team, so that
+ * the launches that depend on it are never ready; then as usual.  stats[0] and stats[1] are
  * the two runs'.  Returns the first run's code when the second succeeds:
  * PROPAG_ERR_TIMEOUT with stats[0].status = 2 when the teams gave up.  The job
  * must be one that cluster = 0 gives several teams (PROPAG_ERR_INVALID). */

@@ -1101,8 +1101,8 @@ __device__ __forceinline__ uint32_t walk_los(const uint32_t *__restrict__ bnd, c
 // launch ends, so outside the tile X[0] and X[1] hold the same state.
 // kWaves: other teams run launches of other tiles of the job at the same time;
 // reach is the largest offset (in cells, per axis) of a reference for which
-// their launches and this one are independent, and *far is set when a cell
-// adopts one further away.
+// their launches and this one are independent, *far is set when a cell
+// adopts one further away, and far[1] counts the sweeps of all teams.
 template <int kArith, bool kGroup, bool kWaves>
 __device__ __forceinline__ bool tile_global(const JobDev &j, const DirConst &dc, const SlotDev &s, const TileDesc &td,
                             uint32_t *list, TileUpdate *sm_upd, uint32_t *cta_ctr, ScanItem *queue, const float *cross,
@@ -1312,6 +1312,8 @@ __device__ __forceinline__ bool tile_global(const JobDev &j, const DirConst &dc,
     uint32_t improving = 0;
     const bool met = team.sync(true, upd_ctr, &improving);
     cx.tick(first ? 0 : 1);
+    // a sweep's beat: teams that wait for this launch see that it goes on
+    if (kWaves && cx.leader) atomicAdd(far + 1, 1u);
     if (!met) {
       cx.failed = cx.abort = true;
       break;
@@ -2033,7 +2035,7 @@ __global__ void __launch_bounds__(kEngineThreads, 1)
   cx.leader = tid == 0;
   cx.max_sweeps = ~0ull;
   cx.t_phase = clock64();
-  uint32_t turn = 0, seen = 0;
+  uint32_t turn = 0, seen = 0;  // leader: the beats (sweeps of all teams) at the last look
   unsigned long long idle_since = 0;
   for (;;) {
     // the leader's warp picks; its word alternates, so that it is not
@@ -2041,9 +2043,9 @@ __global__ void __launch_bounds__(kEngineThreads, 1)
     if (rank == 0 && threadIdx.x < 32) {
       uint32_t pick = wave_pick(w, j.TX, j.TY, err, list, lane);
       if (lane == 0) {
-        const uint32_t done = ld_relaxed_u32(w.far + 1);
-        if (pick != kWaveIdle || done != seen || idle_since == 0) {
-          seen = done;
+        const uint32_t beats = ld_relaxed_u32(w.far + 1);
+        if (pick != kWaveIdle || beats != seen || idle_since == 0) {
+          seen = beats;
           idle_since = globaltimer_ns();
         } else if (globaltimer_ns() - idle_since > w.stall_ns) {
           atomicOr(err, 1u);
@@ -2076,7 +2078,6 @@ __global__ void __launch_bounds__(kEngineThreads, 1)
       if (worked) atomicOr(w.worked + r, 1u);
       __threadfence();  // the team's writes (its last barrier made them visible here), then `done`
       atomicExch(w.done + t, r);
-      atomicAdd(w.far + 1, 1u);
     }
   }
   add_counters(cx.cnt, st, lane);

@@ -134,10 +134,12 @@ struct WaveDev {
   uint32_t *claim;   // per tile: rounds taken by a team
   uint32_t *worked;  // per round: a launch of it improved a cell
   uint32_t *sweeps;  // per round: sweeps of its launches
-  uint32_t *far;     // [0] a reference lies too far away for `window`; [1] launches done
+  uint32_t *far;     // [0] a reference lies too far away for `window`; [1] sweeps of all teams, modulo 2^32
   uint32_t tiles;
   int32_t window;    // launches of tiles up to this many tiles apart keep their order
-  unsigned long long stall_ns;  // a team that waits this long for other teams' launches gives the run up
+  // A team that waits this long while no team ends a sweep gives the run up (a
+  // launch may take longer: a sweep's own waits are bounded by the barrier's).
+  unsigned long long stall_ns;
 };
 constexpr unsigned long long kWaveStallNs = 20000000000ull;
 constexpr uint32_t kWaveRounds = 1024;  // rounds the words hold

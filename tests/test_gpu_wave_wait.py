@@ -60,3 +60,19 @@ def test_jobs_without_teams_and_tiles_outside_are_refused(pp):
     small = _job(L, 150, 150, sc.dx, sc.dy, sc.max_time, d, tile=0)
     assert _run(L, small, -1, 40)[0] == L.PROPAG_ERR_INVALID
     assert _run(L, small, 1, 40)[0] == L.PROPAG_ERR_INVALID
+
+
+def test_long_launches_are_not_taken_for_a_stall(pp):
+    """A team waits for another one's launch as long as that one goes on: launches
+    that take many times the limit, a sweep every few microseconds."""
+    from py_propag import _lib as L
+    from py_propag import scenarios as S
+    size, tile = 1640, 410
+    sc = S.Scenario(size, size, 5.0, 5.0, 1.0e4, pp.demo_terrain(size, size), [(615, 615, 0.0)])
+    d = _device_scenario(pp, sc)
+    job = _job(L, size, size, sc.dx, sc.dy, sc.max_time, d, tile=tile)
+    rc, _, first, second = _run(L, job, -1, 2)
+    assert rc == 0, L.last_error()
+    assert first["status"] == second["status"] == 0 and first["burned"] > 20000
+    for k in SCHEDULE + WORK:
+        assert first[k] == second[k], k
