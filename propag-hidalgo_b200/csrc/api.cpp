@@ -13,7 +13,6 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <functional>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -23,6 +22,7 @@
 #include "io.hpp"
 #include "noalloc.hpp"
 #include "propag_b200.h"
+#include "team_plan.hpp"
 
 namespace propag {
 
@@ -37,6 +37,7 @@ cudaError_t launch_prep(const JobDev *jobs, uint32_t n_jobs, uint64_t max_cells,
                         const uint32_t *only_if, cudaStream_t stream);
 cudaError_t launch_ignite(const JobDev *jobs, uint32_t n_jobs, const uint32_t *only_if,
                           cudaStream_t stream);
+int engine_threads();  // the engine kernel's launch bound
 cudaError_t waves_max_ctas(int threads, size_t smem, int arith, int *n);
 cudaError_t launch_waves(const JobDev *job, const SlotDev *slots, uint32_t teams, uint32_t group, int threads,
                          size_t smem, uint32_t *err, StatsDev *stats, const WaveDev &w, uint32_t *redo, int arith,
@@ -343,72 +344,10 @@ extern "C" void propag_engine_destroy(propag_engine *e) {
   cudaGetLastError();  // leave no error of the teardown to the caller's next CUDA call
 }
 
-// CTAs of a group-mode team for a batch on `ctas` co-resident CTAs.  Jobs go to
-// the teams largest first, each to the team that is free first, so the number
-// of teams decides between many jobs at once on few CTAs each and few at once
-// on many.  A job of s x s cells takes in the mean about 7.6 us x s on any team
-// (its sweeps, each a chain of latencies) plus 0.229 us x s^2 / R on R CTAs, but
-// jobs of one size differ widely (a fire dies early or crosses the grid), and
-// with as many teams as jobs the batch waits for the longest one on its few
-// CTAs.  So the batch is played through with durations from a tenth of the mean
-// to 1.9 times it, spread evenly over the jobs (multiples of the golden ratio),
-// and the number of teams that ends first is taken.  Measured on twelve batches
-// of 5 to 256 members of 100^2 to 2048^2, three seeds each: 2.7 % above the best
-// number of teams in the mean, 13 % with every job at its mean.  64 members of
-// 1024^2: 128 / 132 / 159 ms in 16 teams of 9, 128 / 157 / 254 in 37 of 4; 24
-// members: 63 / 58 / 54 in 12 of 12, 94 / 90 / 83 in 24 of 6; 256 members of 512^2
-// keep 37 teams of 4 (106 / 94 / 119; 140 / 112 / 145 in 16 of 9).
-static int team_size(const std::vector<JobDev> &jobs, int ctas) {
-  std::vector<double> side(jobs.size());
-  for (size_t i = 0; i < jobs.size(); ++i) side[i] = std::sqrt((double)jobs[i].W * (double)jobs[i].H);
-  std::sort(side.begin(), side.end(), std::greater<double>());
-  int best = ctas;
-  double best_us = 0.0;
-  for (int teams : {1, 2, 3, 4, 6, 8, 12, 16, 24, 37, 49, 74}) {
-    if (teams > 1 && ((size_t)teams > jobs.size() || ctas / teams < 2)) break;
-    const int R = ctas / teams;
-    std::vector<double> ends((size_t)teams, 0.0);  // a min-heap of the teams' finishing times
-    double turn = 0.0;
-    for (double s : side) {
-      turn += 0.618034;
-      turn -= std::floor(turn);
-      std::pop_heap(ends.begin(), ends.end(), std::greater<double>());
-      ends.back() += (7.6 * s + 0.229 * s * s / R) * (0.1 + 1.8 * turn);
-      std::push_heap(ends.begin(), ends.end(), std::greater<double>());
-    }
-    const double us = *std::max_element(ends.begin(), ends.end());
-    if (teams == 1 || us < best_us) {
-      best_us = us;
-      best = R;
-    }
-  }
-  return std::max(best, 2);
-}
-
-// Several teams on one job (WaveDev in engine.cuh): how many, and the window
-// within which launches keep their sequence; no teams when the job has too few
-// tiles to run any of them at once.  A window of one tile of at least 257
-// cells, two of 129, three of 86 holds every reference of up to 256 cells'
-// offset: the longest lines of sight of the hilly and ridged scenarios are 160
-// to 218 steps, and a job with a longer one is run twice.  The number of teams
-// is what a simulation of the schedule with measured sweep times favours (in
-// sequence / 2 / 3 / 4 / 6 teams; 4096^2 with 20 ignitions: 478 / 265 / 208 / 186 /
-// 212 ms; 2048^2 with 20: 103 / 58 / 53 / 59 / 71, with one: 49 / 33 / 35 / 37 /
-// 45).
-struct WavePlan {
-  uint32_t teams = 0;
-  int window = 0;
-};
-static WavePlan wave_plan(const JobDev &j) {
-  WavePlan p;
-  const uint64_t tiles = (uint64_t)j.TX * (uint64_t)j.TY;
-  const int window = j.T >= 257 ? 1 : j.T >= 129 ? 2 : 3;
-  if (j.T < 86 || tiles > kWaveTiles || std::max(j.TX, j.TY) < 2 * window + 2 ||
-      (uint64_t)j.W * (uint64_t)j.H >= (1ull << 27))
-    return p;
-  p.window = window;
-  p.teams = j.n_ignitions < 2 ? 2 : tiles >= 100 ? 4 : 3;
-  return p;
+static std::vector<double> job_sides(const PropagJob *jobs, uint32_t n_jobs) {
+  std::vector<double> side(n_jobs);
+  for (uint32_t i = 0; i < n_jobs; ++i) side[i] = std::sqrt((double)jobs[i].width * (double)jobs[i].height);
+  return side;
 }
 
 static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, cudaStream_t stream,
@@ -487,7 +426,7 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
     // sweep.
     int ctas = 0;
     CK(engine_max_clusters(1, e->threads, global_tile_smem(e->threads), arith, true, &ctas));
-    if (ctas >= 8) csize = -team_size(jd, ctas);
+    if (ctas >= 8) csize = -team_size(job_sides(jobs, n_jobs), ctas);
   }
   if (csize == 0) {
     // among the cluster sizes that hold every job's tile, the one that runs
@@ -531,14 +470,15 @@ static int engine_run(propag_engine *e, const PropagJob *jobs, uint32_t n_jobs, 
     CK(engine_max_clusters(1, e->threads, smem, arith, true, &ctas));
     if (ctas < 2) return fail(PROPAG_ERR_CUDA, "group mode needs at least 2 resident CTAs");
     const int team = csize == PROPAG_CLUSTER_GROUPS ? 32 : std::max(2, -csize);
-    n_slots = std::min<uint32_t>(n_jobs, (uint32_t)std::max(1, ctas / team));
-    group = (uint32_t)ctas / n_slots;
+    const GroupSplit split = group_split(n_jobs, ctas, team);
+    n_slots = split.slots;
+    group = split.group;
     for (uint32_t i = 0; i < n_jobs; ++i) {
       jd[i].smem_tile = kSmemTileGlobal;
       tn_max = std::max<size_t>(tn_max, (size_t)tw[i] * (size_t)th[i]);
     }
     if (n_jobs == 1 && e->csize == 0 && !e->phantom && max_sweeps() == kMaxSweeps) {
-      waves = wave_plan(jd[0]);
+      waves = wave_plan(jobs[0].width, jobs[0].height, jd[0].T, jobs[0].n_ignitions);
       int wave_ctas = 0;
       if (waves.teams) CK(waves_max_ctas(e->threads, smem, arith, &wave_ctas));
       wave_group = waves.teams ? (uint32_t)wave_ctas / waves.teams : 0;
@@ -954,8 +894,7 @@ extern "C" int propag_autotune(const PropagJob *jobs, const PropagTerrainPtrs *t
                                uint32_t n_jobs, void *stream_ptr, int repeats, PropagOptions *best,
                                float *best_ms) {
   if (!jobs || n_jobs == 0 || !best) return fail(PROPAG_ERR_INVALID, "propag_autotune: no jobs or output");
-  int sms = 0;
-  int rc = ensure_device(-1, &sms);
+  int rc = ensure_device(-1, nullptr);
   if (rc) return rc;
   cudaStream_t stream = (cudaStream_t)stream_ptr;
   repeats = std::max(repeats, 1);
@@ -972,12 +911,17 @@ extern "C" int propag_autotune(const PropagJob *jobs, const PropagTerrainPtrs *t
     if (all) cands.push_back(c);
   }
   if (cands.empty()) cands.push_back(16);  // global-memory tiles: the largest cluster
-  // group mode: the automatic team size and teams of 24, 16, 8 and 4 CTAs, in
-  // case the jobs differ from what that estimate takes them to be (256 members
-  // of 1024^2: 381 ms with the automatic teams of 4, 376 with teams of 8)
-  cands.push_back(0);
-  for (int t : {24, 16, 8, 4})
-    if ((uint32_t)t * n_jobs > (uint32_t)sms) cands.push_back(-t);  // else the automatic one
+  int arith = jobs[0].arith == PROPAG_ARITH_REFERENCE ? 1 : 0, ctas = 0;
+  for (uint32_t i = 1; i < n_jobs; ++i)
+    if ((jobs[i].arith == PROPAG_ARITH_REFERENCE ? 1 : 0) != arith) arith = 2;
+  CK(engine_max_clusters(1, engine_threads(), global_tile_smem(engine_threads()), arith, true, &ctas));
+  if (ctas >= 8) {
+    const int T0 = jobs[0].tile ? jobs[0].tile : PROPAG_DEFAULT_TILE;
+    const bool waves = n_jobs == 1 && T0 > 0 && wave_plan(jobs[0].width, jobs[0].height, T0, jobs[0].n_ignitions).teams;
+    for (int c : autotune_groups(n_jobs, ctas, waves ? 0 : team_size(job_sides(jobs, n_jobs), ctas))) cands.push_back(c);
+  } else {
+    cands.push_back(0);
+  }
   cudaEvent_t a = nullptr, b = nullptr;
   CK(cudaEventCreate(&a));
   CK(cudaEventCreate(&b));
@@ -1018,9 +962,6 @@ extern "C" int propag_autotune(const PropagJob *jobs, const PropagTerrainPtrs *t
 // One job, the same kernels as engine_run, scratch in the fixed device array
 // of noalloc.cu.  No cudaMalloc/cudaFree/cudaMallocHost, no events, no host
 // heap on the success path.
-namespace propag {
-int engine_threads();  // engine.cu: the engine kernel's launch bound
-}
 static_assert(PROPAG_STATIC_MAX_CELLS == kStaticMaxCells, "header and scratch disagree");
 namespace {
 // Device address of the fixed scratch per device ordinal, taken once per

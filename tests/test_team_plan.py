@@ -1,0 +1,67 @@
+"""The rules that split a batch over the device (csrc/team_plan.hpp), on the
+host: what the autotuner times for every number of jobs, and that the splits
+use the CTAs they are given."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+SOURCE = r"""
+#include "team_plan.hpp"
+using namespace propag;
+extern "C" int plan_team(int n, const double *side, int ctas) { return team_size(std::vector<double>(side, side + n), ctas); }
+extern "C" void plan_split(uint32_t n, int ctas, int team, uint32_t *out) {
+  const GroupSplit g = group_split(n, ctas, team);
+  out[0] = g.slots;
+  out[1] = g.group;
+}
+extern "C" int plan_modes(uint32_t n, int ctas, int auto_team, int *out) {
+  const std::vector<int> m = autotune_groups(n, ctas, auto_team);
+  std::copy(m.begin(), m.end(), out);
+  return (int)m.size();
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def plan(tmp_path_factory):
+    d = tmp_path_factory.mktemp("plan")
+    (d / "p.cpp").write_text(SOURCE)
+    so = d / "p.so"
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I" + os.path.join(cuda, "include"),
+                    "-I" + os.path.join(ROOT, "propag-hidalgo_b200", "csrc"), str(d / "p.cpp"), "-o", str(so)],
+                   check=True)
+    return C.CDLL(str(so))
+
+
+def _split(plan, n, ctas, team):
+    out = (C.c_uint32 * 2)()
+    plan.plan_split(n, ctas, team, out)
+    return tuple(out)
+
+
+@pytest.mark.parametrize("ctas", [148, 132, 16])
+@pytest.mark.parametrize("side", [128.0, 1024.0])
+def test_autotuner_modes(plan, ctas, side):
+    for n in list(range(1, 160)) + [256, 1000, 5000]:
+        auto = plan.plan_team(n, (C.c_double * n)(*[side] * n), ctas)
+        assert 2 <= auto <= ctas
+        for auto_team in {auto, 0}:  # 0: the automatic mode is not one team a job's split
+            out = (C.c_int * 16)()
+            count = plan.plan_modes(n, ctas, auto_team, out)
+            modes = list(out)[:count]
+            assert modes[0] == 0 and all(m <= -2 for m in modes[1:])
+            splits = [_split(plan, n, ctas, -m) for m in modes[1:]] + (
+                [_split(plan, n, ctas, auto_team)] if auto_team else [])
+            assert len(set(splits)) == len(splits), n  # nothing is timed twice
+            if ctas // n >= 2:  # a team per job is among them
+                assert (n, ctas // n) in splits, n
+            for team in (24, 16, 8, 4):
+                if team <= ctas:
+                    assert _split(plan, n, ctas, team) in splits, (n, team)
+            for slots, group in splits:
+                assert 1 <= slots <= n and group >= 2 and slots * group <= ctas
