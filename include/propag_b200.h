@@ -207,13 +207,19 @@ int propag_selftest_group_wait(uint32_t *status);
  *
  * propag_selftest_atan2f_table: out[(a + max_a) + (b + max_b) (2 max_a + 1)]
  * = atan2f(a, b) for the integers |a| <= max_a, |b| <= max_b (the bearings
- * the reference's time_from computes between cells). */
+ * the reference's time_from computes between cells).
+ *
+ * propag_selftest_dead_ratio: for dead[i] and fuel model[i], the fire pass's
+ * product with the reciprocal of the model's moisture of extinction, CUDA's
+ * __fdividef of dead[i] and that moisture, and the moisture. */
 int propag_selftest_time_from(int arith, uint64_t n, const int32_t *fx, const int32_t *fy,
                               const float *ftime, const int32_t *tx, const int32_t *ty,
                               const float *smax, const float *azmax, const float *ecc, float dx,
                               float dy, float *out);
 int propag_selftest_cosf_table(uint32_t first_bits, uint64_t n, float *out);
 int propag_selftest_atan2f_table(int32_t max_a, int32_t max_b, float *out);
+int propag_selftest_dead_ratio(uint64_t n, const int32_t *model, const float *dead, float *product,
+                               float *quotient, float *mext);
 
 typedef struct PropagOptions {
   int32_t tile;    /* default super-grid tile side; 0 = PROPAG_DEFAULT_TILE,

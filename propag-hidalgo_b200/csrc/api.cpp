@@ -33,6 +33,8 @@ cudaError_t launch_fire(bool full, uint64_t n, const uint8_t *fuel, const float 
                         const float *ws, const float *waz, const float *slope,
                         const float *aspect, float *const outs[10], int sm_count,
                         cudaStream_t stream);
+cudaError_t launch_dead_ratio(uint64_t n, const int32_t *model, const float *dead, float *product, float *quotient,
+                              float *mext, cudaStream_t stream);
 cudaError_t launch_prep(const JobDev *jobs, uint32_t n_jobs, uint64_t max_cells, int sms,
                         const uint32_t *only_if, cudaStream_t stream);
 cudaError_t launch_ignite(const JobDev *jobs, uint32_t n_jobs, const uint32_t *only_if,
@@ -1467,6 +1469,24 @@ extern "C" int propag_selftest_time_from(int arith, uint64_t n, const int32_t *f
                       b.at<float>(5 * a), b.at<float>(6 * a), b.at<float>(7 * a), dx, dy, dy < 0,
                       b.at<float>(8 * a), nullptr));
   CK(cudaMemcpy(out, b.at<float>(8 * a), n * 4, cudaMemcpyDeviceToHost));
+  return PROPAG_OK;
+}
+
+extern "C" int propag_selftest_dead_ratio(uint64_t n, const int32_t *model, const float *dead, float *product,
+                                          float *quotient, float *mext) {
+  int rc = ensure_device(-1, nullptr);
+  if (rc) return rc;
+  if (n == 0) return PROPAG_OK;
+  if (!model || !dead || !product || !quotient || !mext) return fail(PROPAG_ERR_INVALID, "null argument");
+  DevBuf b;
+  const size_t a = align_up(n * 4, 256);
+  CK(b.reserve(5 * a, nullptr));
+  CK(cudaMemcpy(b.at<char>(0), model, n * 4, cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(b.at<char>(a), dead, n * 4, cudaMemcpyHostToDevice));
+  CK(launch_dead_ratio(n, b.at<int32_t>(0), b.at<float>(a), b.at<float>(2 * a), b.at<float>(3 * a),
+                       b.at<float>(4 * a), nullptr));
+  float *const outs[3] = {product, quotient, mext};
+  for (int k = 0; k < 3; ++k) CK(cudaMemcpy(outs[k], b.at<char>((2 + k) * a), n * 4, cudaMemcpyDeviceToHost));
   return PROPAG_OK;
 }
 

@@ -38,7 +38,7 @@ struct alignas(16) FuelConst {
   // double-float one does, and the range in which live_mext before max(., mext)
   // is not (fire.cu)
   float dead_min, live_min, live_above, live_below;
-  float mext_rcp;    // set by the kernels
+  float mext_rcp;    // __fdividef(1, mext_f), set by the kernels
   float dead_exact;  // 1: the dead sum is exact in both
 };
 static_assert(sizeof(FuelConst) == 44 * 4, "FuelConst layout");

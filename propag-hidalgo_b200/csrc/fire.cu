@@ -71,6 +71,13 @@ struct FireOut {
       residence_time, byrams, flame;
 };
 
+// 1 - rt of the dead fuel, (mext - dead_moist) / mext, as the product with the
+// model's mext_rcp: an operation of its own, whose relative error is at most
+// 2^-22 for the reciprocal (CUDA's bound for __fdividef is 2 ulp) and 2^-24 for
+// the product.  A test holds it to that and compares it with __fdividef(dead,
+// mext).
+__device__ __forceinline__ float dead_ratio(const FuelConst &F, float dead) { return dead * F.mext_rcp; }
+
 // eta_m (firelib.rs:1060-1076) with rt = moist / mext, as
 // u (2.93 - 5.45 u + 3.52 u^2), u = 1 - rt = (mext - moist) / mext.
 __device__ __forceinline__ float eta_of(float u) { return u * fmaf(u, fmaf(u, 3.52f, -5.45f), 2.93f); }
@@ -94,8 +101,8 @@ __device__ __forceinline__ void burn_cell(const FuelConst &F, const float m[5], 
   // rx_int_rbqig
   const float rbqig = F.R0 + dot5(F.R, m);
   const Moist w = moist_sums(F, m);
-  // not positive: life_moist >= life_mext.  2 ulp; operands in [2^-126, 2^126]
-  const float eta_dead = w.dead > 0.0f ? eta_of(w.dead * F.mext_rcp) : 0.0f;  // __fdividef(w.dead, mext), as below
+  // not positive: life_moist >= life_mext.  __fdividef: operands in [2^-126, 2^126]
+  const float eta_dead = w.dead > 0.0f ? eta_of(dead_ratio(F, w.dead)) : 0.0f;
   const float eta_live = w.live > 0.0f ? eta_of(__fdividef(w.live, w.lmext)) : 0.0f;
   const float rx = fmaf(F.rx_alive, eta_live, F.rx_dead * eta_dead);
   const float speed0 = __fdividef(rx * F.flux_ratio, rbqig);
@@ -201,7 +208,6 @@ __device__ __forceinline__ void load_catalog(float *cat) {
   for (int t = threadIdx.x; t < kMaxFuels * kWords; t += blockDim.x)
     cat[(t / kWords) * kCatStride + t % kWords] = src[t];
   __syncthreads();
-  // the reciprocal that the fast division by mext multiplies with
   if (threadIdx.x < kMaxFuels) {
     FuelConst *const f = reinterpret_cast<FuelConst *>(cat + threadIdx.x * kCatStride);
     f->mext_rcp = __fdividef(1.0f, f->mext_f);
@@ -304,6 +310,26 @@ static cudaError_t launch_fire_t(const Inputs &in, const Outputs &out, uint64_t 
   auto k1 = fire_kernel<kFull, Index>;
   k1<<<grid_for(n, threads, sm_count, ctas_per_sm(k1, threads)), threads, 0, stream>>>(in, out, (Index)0,
                                                                                     (Index)n);
+  return cudaGetLastError();
+}
+
+// For the test of dead_ratio: it, __fdividef and the divisor, for model[i] and dead[i].
+__global__ void dead_ratio_kernel(uint64_t n, const int32_t *model, const float *dead, float *product,
+                                  float *quotient, float *mext) {
+  __shared__ __align__(16) float cat[kMaxFuels * kCatStride];
+  load_catalog(cat);
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    const FuelConst &F = fuel_row(cat, (uint32_t)model[i] < kMaxFuels ? model[i] : 0);
+    product[i] = dead_ratio(F, dead[i]);
+    quotient[i] = __fdividef(dead[i], F.mext_f);
+    mext[i] = F.mext_f;
+  }
+}
+
+cudaError_t launch_dead_ratio(uint64_t n, const int32_t *model, const float *dead, float *product, float *quotient,
+                              float *mext, cudaStream_t stream) {
+  if (n == 0) return cudaSuccess;
+  dead_ratio_kernel<<<256, 256, 0, stream>>>(n, model, dead, product, quotient, mext);
   return cudaGetLastError();
 }
 

@@ -193,6 +193,7 @@ SIGNATURES = {
                                   [C.c_float, C.c_float, C.c_void_p]),
     "propag_selftest_cosf_table": (C.c_int, [C.c_uint32, C.c_uint64, C.c_void_p]),
     "propag_selftest_atan2f_table": (C.c_int, [C.c_int32, C.c_int32, C.c_void_p]),
+    "propag_selftest_dead_ratio": (C.c_int, [C.c_uint64] + [C.c_void_p] * 5),
     "propag_slope_aspect_device": (C.c_int, [C.c_uint32, C.c_uint32, C.c_double, C.c_double, C.c_void_p,
                                              C.c_void_p, C.c_void_p, C.c_void_p]),
     "propag_dmoist_device": (C.c_int, [C.c_uint64, C.c_int, C.c_int, C.POINTER(PropagWeatherPtrs),
