@@ -474,7 +474,10 @@ int64_t propag_rasterize_ignitions(const GeoReference *geo_ref, const FFITimeFea
  * to pixel space; the burning runs on the GPU with the same rules as the
  * host rasteriser above, and the rasters are bit-identical to its result.
  * All three are stream-ordered on `stream`; the device scratch they need is
- * allocated and released on that stream, from a pool that keeps up to 128 MiB.
+ * allocated and released on that stream, from a pool that keeps up to 128 MiB
+ * per device between calls.  propag_trim_scratch gives what is kept and not in
+ * use back (a caller whose own allocation fails, or that rasterises no more); the
+ * library does so itself when an allocation of its own fails.
  *
  * propag_rasterize_times_device writes the initial time raster of the
  * reference's rasterize_times (crates/propag/src/propag.rs:837-890):
@@ -500,6 +503,7 @@ int propag_rasterize_fuels_device(const FFIFuelFeature *fuels, uintptr_t fuels_l
  * waits for the stream and returns the number of such cells (< 0 on error). */
 int64_t propag_ignitions_from_times_device(const float *times, uint32_t width, uint32_t height,
                                            PropagIgnition *out, uint64_t max_out, void *stream);
+int propag_trim_scratch(void);
 
 /* GeoPackage layers as the reference's write_refs / write_boundaries write
  * them through GDAL (crates/propag/src/propag.rs:601-750), without GDAL:

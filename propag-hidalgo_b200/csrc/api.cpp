@@ -120,11 +120,24 @@ int ensure_device(int want, int *sms_out) {
 // device's own: the default pool gives freed memory back at every
 // synchronisation, so that each call paid for mapping its scratch again (3 ms
 // for the rasters of a 3001 x 2003 map, 0.1 ms from a pool that keeps it).  The
-// pool keeps at most kPoolKeep bytes, which scratch_trim gives back when an
-// allocation fails.  Safe with several threads and streams, as every pool.
+// pool keeps at most kPoolKeep bytes, which scratch_trim gives back: when an
+// allocation of the library fails, or the caller asks (propag_trim_scratch).
+// Safe with several threads and streams, as every pool.
 constexpr uint64_t kPoolKeep = 128ull << 20;
 std::mutex g_pool_mu;
 cudaMemPool_t g_pool[64] = {};
+
+// Gives the pools' unused memory back.
+cudaError_t scratch_trim() {
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  cudaError_t e = cudaSuccess;
+  for (cudaMemPool_t pool : g_pool)
+    if (pool) {
+      const cudaError_t r = cudaMemPoolTrimTo(pool, 0);
+      if (e == cudaSuccess) e = r;
+    }
+  return e;
+}
 
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t stream) {
   int dev = 0;
@@ -149,14 +162,13 @@ cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t stream) {
     }
     pool = g_pool[dev];
   }
-  return cudaMallocFromPoolAsync(p, bytes, pool, stream);
-}
-
-// Gives the pools' unused memory back.
-void scratch_trim() {
-  std::lock_guard<std::mutex> lk(g_pool_mu);
-  for (cudaMemPool_t pool : g_pool)
-    if (pool) cudaMemPoolTrimTo(pool, 0);
+  e = cudaMallocFromPoolAsync(p, bytes, pool, stream);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    scratch_trim();
+    e = cudaMallocFromPoolAsync(p, bytes, pool, stream);
+  }
+  return e;
 }
 
 struct DevBuf {
@@ -1807,6 +1819,11 @@ extern "C" int propag_rasterize_fuels_device(const FFIFuelFeature *fuels, uintpt
   int32_t *w = static_cast<int32_t *>(win.p);
   CK(launch_rasterize_winner(dev, W, H, w, sms, s));
   CK(launch_finish_codes(w, static_cast<const uint8_t *>(dev_value), result, W * H, sms, s));
+  return PROPAG_OK;
+}
+
+extern "C" int propag_trim_scratch(void) {
+  CK(scratch_trim());
   return PROPAG_OK;
 }
 

@@ -234,6 +234,7 @@ SIGNATURES = {
                                                 C.POINTER(GeoReference), C.c_void_p, C.c_void_p]),
     "propag_ignitions_from_times_device": (C.c_int64, [C.c_void_p, C.c_uint32, C.c_uint32, C.c_void_p,
                                                        C.c_uint64, C.c_void_p]),
+    "propag_trim_scratch": (C.c_int, []),
     "propag_write_geotiff": (C.c_int, [C.POINTER(GeoReference), C.c_void_p, C.c_char_p]),
     "propag_write_refs_gpkg": (C.c_int, [C.POINTER(GeoReference), C.c_void_p, C.c_void_p, C.c_void_p,
                                          C.c_char_p]),
