@@ -126,7 +126,7 @@ __device__ __forceinline__ float dm_pp_effect(const DmoistTables &T, int mi, flo
 
 // floor(rh / 5) clamped to [0, 20] and 9 - ceil(t / 5) clamped to [0, 8]: the
 // classes of the rounded product with 0.2f are those of the rounded quotient
-// for every float (checked over all of them).
+// for every float (a test compares all of them).
 __device__ __forceinline__ int dm_hcb(const DmoistTables &T, float t, float rh) {
   float hf = floorf(rh * 0.2f);
   hf = hf < 0.0f ? 0.0f : (hf > 20.0f ? 20.0f : hf);
@@ -180,8 +180,9 @@ __device__ __forceinline__ DmoistHour dm_hour(int month, int hour) {
 // The table's exposure row of a cell, or -1 (an aspect outside [0, 2 pi], or
 // NaN, on a slope).  The reference compares aspect * 180 / pi with 45, 135,
 // 225, 315 and 360 degrees and the slope's angle, atan(slope) * 180 / pi, with
-// 30 degrees; both are monotonic in float, so each comparison is one with the
-// first (last) float that passes it, found by a search over all floats.
+// 30 degrees; each comparison is one with the first (last) float that passes it
+// (a test compares the azimuths for every float, and the slopes for every float
+// around 30 degrees and a spread of all).
 __device__ __forceinline__ float dm_atan_pos(float y);
 __device__ __forceinline__ int dm_exposure(float slope, float aspect) {
   constexpr float k45 = 0x1.921fb6p-1f, k135 = 0x1.2d97c8p+1f, k225 = 0x1.f6a7a4p+1f, k315 = 0x1.5fdbbep+2f;
@@ -195,8 +196,11 @@ __device__ __forceinline__ int dm_exposure(float slope, float aspect) {
   return 2 * quarter + steep;
 }
 
-// x / 15 and x / 9 by the reciprocal and one residual correction: the
-// correctly rounded quotient for every float (checked over all of them).
+// x / 15 and x / 9 from the rounded reciprocal of the constant and the product's
+// residual by a fused multiply-add (Markstein 1990; Brisebarre, Muller and Raina
+// 2004, on division by a divisor known in advance): the correctly rounded
+// quotient for every finite float but -0, whose sign is lost (a test compares
+// all of them).  The ends' differences are finite and not below 0.001.
 __device__ __forceinline__ float dm_div15(float x) {
   const float r = 1.0f / 15.0f, q = x * r;
   return __fmaf_rn(__fmaf_rn(-15.0f, q, x), r, q);

@@ -2,7 +2,9 @@
 host, against the CPU restatement of the reference (crates/dmoist/src/
 lib.rs:55-715): equal bit for bit in every month a caller can pass, the ones
 outside 1..12 included, for which the reference has no shading correction (the
-corrected humidity class is NaN there, and every moisture zero)."""
+corrected humidity class is NaN there, and every moisture zero).  What it
+computes another way than the model's formulas -- divisions by constants,
+classes, limits of the exposures -- is compared with them float by float."""
 import ctypes as C
 import os
 import subprocess
@@ -81,6 +83,100 @@ def test_every_month(model, oracle, month):
             assert np.array_equal(g.view(np.uint32), w.view(np.uint32)), hour
         if not 1 <= month <= 12:
             assert not np.any(got[0])
+
+
+# Each function returns the number of floats for which the device code differs
+# from the model's formula.
+EXHAUSTIVE = r"""
+#include "dmoist_device.cuh"
+using namespace propag;
+static inline float as_float(uint32_t b) { float f; std::memcpy(&f, &b, 4); return f; }
+static inline uint32_t bits(float f) { uint32_t b; std::memcpy(&b, &f, 4); return b; }
+constexpr uint64_t kAll = 1ull << 32, kChunk = 1 << 16;
+template <typename F> static uint64_t over(uint64_t first, uint64_t last, uint64_t step, F differs) {
+  uint64_t n = 0;
+#pragma omp parallel for reduction(+ : n) schedule(static)
+  for (uint64_t c = first; c < last; c += kChunk * step) {
+    uint32_t k = 0;
+    for (uint32_t i = 0; i < kChunk; ++i) k += differs(as_float((uint32_t)(c + i * step)));
+    n += k;
+  }
+  return n;
+}
+// x / 15 and x / 9, finite x but -0 (see minus_zero)
+extern "C" uint64_t division() {
+  return over(0, kAll, 1, [](float x) -> uint32_t {
+    const uint32_t wrong = (bits(dm_div15(x)) ^ bits(x / 15.0f)) | (bits(dm_div9(x)) ^ bits(x / 9.0f));
+    return (wrong != 0u) & ((bits(x) & 0x7F800000u) != 0x7F800000u) & (bits(x) != 0x80000000u);
+  });
+}
+extern "C" int minus_zero() { return dm_div15(-0.0f) == 0.0f && dm_div9(-0.0f) == 0.0f; }
+// floor(x / 5) clamped to [0, 20], 9 - ceil(x / 5) clamped to [0, 8]; NaN: 0
+static inline int clamp_class(float v, float top) {
+  v = v < 0.0f ? 0.0f : (v > top ? top : v);
+  return v != v ? 0 : (int)v;
+}
+extern "C" uint64_t classes() {
+  return over(0, kAll, 1, [](float x) -> uint32_t {
+    return (clamp_class(floorf(x * 0.2f), 20.0f) != clamp_class(floorf(x / 5.0f), 20.0f)) |
+           (clamp_class(9.0f - ceilf(x * 0.2f), 8.0f) != clamp_class(9.0f - ceilf(x / 5.0f), 8.0f));
+  });
+}
+// the exposure row from an aspect and a slope in degrees (lib.rs:472-614)
+static inline float degrees(float rad) { return rad * 180.0f / 3.14159274101257324f; }
+static inline int exposure(float sdeg, float adeg) {
+  const float o = sdeg == 0.0f ? 180.0f : adeg;
+  const int steep = sdeg <= 30.0f ? 0 : 1;
+  if ((o >= 315.0f && o <= 360.0f) || (o >= 0.0f && o < 45.0f)) return steep;
+  if (o >= 45.0f && o < 135.0f) return 2 + steep;
+  if (o >= 135.0f && o < 225.0f) return 4 + steep;
+  if (o >= 225.0f && o < 315.0f) return 6 + steep;
+  return -1;
+}
+extern "C" uint64_t aspects(float slope) {
+  const float sdeg = degrees(dm_atan_pos(slope));
+  return over(0, kAll, 1, [=](float x) -> uint32_t { return dm_exposure(slope, x) != exposure(sdeg, degrees(x)); });
+}
+extern "C" uint64_t slopes(uint32_t first, uint64_t last, uint64_t step) {
+  return over(first, last, step, [](float x) -> uint32_t { return dm_exposure(x, 1.0f) != exposure(degrees(dm_atan_pos(x)), degrees(1.0f)); });
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def exhaustive(tmp_path_factory):
+    d = tmp_path_factory.mktemp("dmoist_all")
+    (d / "cuda_runtime.h").write_text(SHIM)
+    (d / "e.cpp").write_text(EXHAUSTIVE)
+    so = d / "e.so"
+    subprocess.run(["g++", "-O3", "-std=c++17", "-march=x86-64-v3", "-fopenmp", "-ffp-contract=off", "-shared", "-fPIC",
+                    "-I" + str(d), "-I" + CSRC, str(d / "e.cpp"), "-o", str(so)], check=True)
+    lib = C.CDLL(str(so))
+    for f in ("division", "classes", "aspects", "slopes"):
+        getattr(lib, f).restype = C.c_uint64
+    lib.aspects.argtypes = [C.c_float]
+    lib.slopes.argtypes = [C.c_uint32, C.c_uint64, C.c_uint64]
+    return lib
+
+
+def test_division_by_constants_for_every_finite_float(exhaustive):
+    """-0 alone gives +0 (a difference of the interpolation's ends below 0.001 is
+    not divided)."""
+    assert exhaustive.division() == 0
+    assert exhaustive.minus_zero()
+
+
+def test_humidity_and_temperature_classes_for_every_float(exhaustive):
+    assert exhaustive.classes() == 0
+
+
+def test_exposure_limits(exhaustive):
+    """The azimuths for every float, the slope of 30 degrees for every float from
+    0.5 to 1 and every 31st of all."""
+    assert exhaustive.aspects(0.4) == 0
+    bits = lambda v: int(np.float32(v).view(np.uint32))  # noqa: E731
+    assert exhaustive.slopes(bits(0.5), bits(1.0), 1) == 0
+    assert exhaustive.slopes(0, 1 << 32, 31) == 0
 
 
 @pytest.mark.gpu
