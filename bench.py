@@ -63,16 +63,13 @@ DRAM_TRAFFIC = {"config1": {"waves_kernel": 719.57e6 + 593.94e6,
                             "fire_kernel": 557.96e6 + 179.52e6}}
 
 
-def step_launches(width: int, height: int, tile: int, cluster: int) -> int:
-    """Kernels launched by a step: fire, prep, ignition, engine, post; for a
-    scenario of four tiles (six below 257 cells a tile, eight below 129) or more
-    along a side and no chosen cluster, several teams run it (waves_kernel) and
-    wave_end, prep, ignition and engine follow, which do nothing unless the
-    scenario has to be run again in sequence."""
-    tile = tile or 323
-    side = -(-max(width, height) // tile)
-    waves = cluster == 0 and tile >= 86 and side >= (4 if tile >= 257 else 6 if tile >= 129 else 8)
-    return 9 if waves else 5
+def step_launches(lib, eng) -> tuple[int, bool]:
+    """Kernels launched by a step -- the fire pass and what the engine says its
+    last run launched -- and whether several teams ran it (waves_kernel)."""
+    kernels, teams = C.c_uint32(), C.c_uint32()
+    if lib.propag_engine_last_run(eng, C.byref(kernels), C.byref(teams)) != 0:
+        raise SystemExit(lib.propag_last_error().decode())
+    return 1 + kernels.value, teams.value > 0
 
 
 def _log(msg: str) -> None:
@@ -678,8 +675,8 @@ def bench_b200(args):
     ach = prop_bytes / prop_s / 1e9
     fire_ach = FIRE_BYTES_PER_CELL * N / fire_s / 1e9
     known = WORK_EVALUATIONS.get(args.workload)
-    launches = step_launches(sc.width, sc.height, args.tile, args.cluster)
-    prop_kernel = "waves_kernel" if launches == 9 else "engine_kernel"
+    launches, waves = step_launches(lib, eng)
+    prop_kernel = "waves_kernel" if waves else "engine_kernel"
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": total_ms / args.steps, "higher_is_better": True,

@@ -301,6 +301,11 @@ int propag_engine_run(propag_engine *engine, const PropagJob *jobs, uint32_t n_j
  * Waits for the last run to finish. */
 int propag_engine_last_times(propag_engine *engine, float ms[3]);
 
+/* How the engine's last run was launched: the kernels it launched, and the teams
+ * that began its lone job together (0: one team per job; the device starts the
+ * job again with one team when its lines of sight turn out too long). */
+int propag_engine_last_run(const propag_engine *engine, uint32_t *kernels, uint32_t *teams);
+
 /* Self-test of the bounded waits of several teams on one job (no reference
  * counterpart): runs the job twice on one engine, first with the teams' limit
  * of waiting for one another while no team ends a sweep at limit_ms (else 20 s)

@@ -758,6 +758,16 @@ extern "C" int propag_selftest_wave_wait(const PropagJob *job, int64_t hold, uin
   return rc;
 }
 
+extern "C" int propag_engine_last_run(const propag_engine *e, uint32_t *kernels, uint32_t *teams) {
+  if (!e || !kernels || !teams) return fail(PROPAG_ERR_INVALID, "null argument");
+  if (!e->last_stats) return fail(PROPAG_ERR_INVALID, "the engine has not run");
+  // prep, ignition, engine, post; waves: prep, ignition, waves and their end,
+  // then prep, ignition and engine for a start in sequence, and post
+  *kernels = e->last_teams ? 8 : 4;
+  *teams = e->last_teams;
+  return PROPAG_OK;
+}
+
 extern "C" int propag_engine_last_times(propag_engine *e, float ms[3]) {
   if (!e || !ms) return fail(PROPAG_ERR_INVALID, "null argument");
   CK(cudaSetDevice(e->device));

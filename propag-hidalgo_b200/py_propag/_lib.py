@@ -186,6 +186,7 @@ SIGNATURES = {
     "propag_engine_destroy": (None, [C.c_void_p]),
     "propag_engine_run": (C.c_int, [C.c_void_p, C.POINTER(PropagJob), C.c_uint32, C.c_void_p,
                                     C.POINTER(PropagStats)]),
+    "propag_engine_last_run": (C.c_int, [C.c_void_p, C.POINTER(C.c_uint32), C.POINTER(C.c_uint32)]),
     "propag_engine_last_times": (C.c_int, [C.c_void_p, C.POINTER(C.c_float * 3)]),
     "propag_selftest_group_wait": (C.c_int, [C.POINTER(C.c_uint32)]),
     "propag_selftest_wave_wait": (C.c_int, [C.POINTER(PropagJob), C.c_int64, C.c_uint32, C.POINTER(PropagStats)]),
