@@ -259,7 +259,9 @@ struct Counters {
 // direct time when the line of sight is blocked or the candidate is not
 // faster -- and the sequential loop keeps the first strictly smaller offer;
 // so the result is the first minimum of the offers when it beats the cell's
-// own time.  The line of sight from the neighbour to its reference was walked
+// own time.  An offer that is NaN (of a neighbour whose fire is) is never the
+// smaller one there, and counts as infinite here: in a reduction by comparisons
+// it would hide the offers behind it.  The line of sight from the neighbour to its reference was walked
 // when it adopted the reference, and is read; only the walks the sequential
 // loop performs (candidate also faster than every earlier offer) are counted,
 // so the counters match the reference's order exactly.  Called by all 32
@@ -315,6 +317,7 @@ __device__ __forceinline__ Best evaluate_coop(const JobDev &j, const DirConst &d
         oref = nr;
       }
     }
+    offer = fminf(offer, kInf);  // NaN: infinite
   }
   // running best of the sequential loop before neighbour k (exclusive min)
   float pm = offer;
@@ -896,6 +899,7 @@ __device__ __forceinline__ Best evaluate_packed(const JobDev &j, const Hot &h,
         oref = n.ref;
       }
     }
+    offer = fminf(offer, kInf);  // NaN: infinite
   }
   // running best of the sequential loop before neighbour k (exclusive min),
   // and the first minimum of the offers
