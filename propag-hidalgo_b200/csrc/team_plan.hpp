@@ -13,47 +13,73 @@
 
 namespace propag {
 
-// CTAs of a group-mode team for a batch on `ctas` co-resident CTAs.  Jobs go to
-// the teams largest first, each to the team that is free first, so the number
-// of teams decides between many jobs at once on few CTAs each and few at once
-// on many.  A job of s x s cells takes in the mean about 7.6 us x s on any team
-// (its sweeps, each a chain of latencies) plus 0.229 us x s^2 / R on R CTAs, but
-// jobs of one size differ widely (a fire dies early or crosses the grid), and
-// with as many teams as jobs the batch waits for the longest one on its few
-// CTAs.  So the batch is played through with durations from a tenth of the mean
-// to 1.9 times it, spread evenly over the jobs (multiples of the golden ratio),
-// and the number of teams that ends first is taken.  Measured on twelve batches
-// of 5 to 256 members of 100^2 to 2048^2, three seeds each: 2.7 % above the best
-// number of teams in the mean, 13 % with every job at its mean.  64 members of
-// 1024^2: 128 / 132 / 159 ms in 16 teams of 9, 128 / 157 / 254 in 37 of 4; 24
-// members: 63 / 58 / 54 in 12 of 12, 94 / 90 / 83 in 24 of 6; 256 members of 512^2
-// keep 37 teams of 4 (106 / 94 / 119; 140 / 112 / 145 in 16 of 9).
-// Where members are alike the longest is no longer than the others, and teams as
-// small as the jobs allow would be a sixth faster (64 copies of one 1024^2
-// scenario: 126 ms in 16 of 9, 108 in 37 of 4; 64 of 512^2: 59 and 52; 200 of
-// 300^2: 49 and 41), which is less than they lose where members differ.
+// When the last of the jobs (sides, largest first) ends in `teams` teams of the
+// CTAs, us: jobs go to the teams largest first, each to the team that is free
+// first.  A job of s x s cells takes in the mean about 7.6 us x s on any team (its
+// sweeps, each a chain of latencies) plus 0.229 us x s^2 / R on R CTAs; differ:
+// times 2.25 u^1.25, the u spread evenly over (0, 1) (multiples of the golden
+// ratio): mean 1, a quarter of the jobs below 0.4, the longest 2.2.
+inline double batch_us(const std::vector<double> &side, int teams, int ctas, bool differ) {
+  const int R = ctas / teams;
+  std::vector<double> ends((size_t)teams, 0.0);  // a min-heap of the teams' finishing times
+  double turn = 0.0;
+  for (double s : side) {
+    turn += 0.618034;
+    turn -= std::floor(turn);
+    std::pop_heap(ends.begin(), ends.end(), std::greater<double>());
+    ends.back() += (7.6 * s + 0.229 * s * s / R) * (differ ? 2.25 * turn * std::sqrt(std::sqrt(turn)) : 1.0);
+    std::push_heap(ends.begin(), ends.end(), std::greater<double>());
+  }
+  return *std::max_element(ends.begin(), ends.end());
+}
+
+// CTAs of a group-mode team for a batch on `ctas` co-resident CTAs; side: the
+// jobs' sides (square roots of their cells), in any order.
 //
-// side: the jobs' sides (square roots of their cells), in any order.
+// The number of teams decides between many jobs at once on few CTAs each and few
+// at once on many.  Where jobs of one size take unequal time (a fire dies early or
+// crosses the grid; the members of a weather ensemble do) fewer teams than jobs
+// win: with a team per job the batch waits for its longest job on that job's few
+// CTAs.  Where they take the same time, a team per job wins, and every number that
+// does not divide the jobs into full rounds loses most.  Nothing tells the two
+// apart before the run, so both are played through for the numbers that make
+// full rounds (and a few small ones, for a batch of a few large jobs and many
+// small ones), and the number is taken whose larger loss is the smallest, with
+// 1.3 times the loss allowed where the jobs are alike, the rarer case.
+//
+// Measured, against the best number of teams: twelve batches of 5 to 256 ensemble
+// members and unrelated scenarios (three seeds) 1.03; 32 sizes of ensembles of 5 to
+// 50 members of 150^2 to 1024^2 (four seeds) 1.02, at most 1.10; the same with
+// copies of one member 1.26, at most 1.77.  The rule before, the number that ends
+// first when the jobs differ, of 1, 2, 3, 4, 6, 8, 12, 16, 24, 37, 49 and 74 teams:
+// 1.03, 1.12 (at most 1.55) and 1.64 (at most 1.90); a team per job up to 37: 1.41,
+// 1.20 (1.78) and 1.02.  20 members of 400^2: 12.9 ms in 10 teams, 15.6 in 20;
+// copies of one: 6.7 and 4.5 (7.7 in 16).  propag_autotune tries a team per job.
 inline int team_size(std::vector<double> side, int ctas) {
   std::sort(side.begin(), side.end(), std::greater<double>());
+  const int n = (int)std::min<size_t>(side.size(), 1u << 30), most = std::max(ctas / 2, 1);
+  std::vector<int> counts;
+  for (int t : {1, 2, 3, 4, 6})
+    if (t <= n && t <= most) counts.push_back(t);
+  const int k0 = std::max(1, (n + most - 1) / most);  // the fewest rounds
+  for (int k = k0; k < k0 + 8 && k <= n; ++k) counts.push_back((n + k - 1) / k);
+  std::sort(counts.begin(), counts.end());
+  counts.erase(std::unique(counts.begin(), counts.end()), counts.end());
+  std::vector<double> alike, differ;
+  for (int t : counts) {
+    alike.push_back(batch_us(side, t, ctas, false));
+    differ.push_back(batch_us(side, t, ctas, true));
+  }
+  const double alike_best = *std::min_element(alike.begin(), alike.end());
+  const double differ_best = *std::min_element(differ.begin(), differ.end());
   int best = ctas;
-  double best_us = 0.0;
-  for (int teams : {1, 2, 3, 4, 6, 8, 12, 16, 24, 37, 49, 74}) {
-    if (teams > 1 && ((size_t)teams > side.size() || ctas / teams < 2)) break;
-    const int R = ctas / teams;
-    std::vector<double> ends((size_t)teams, 0.0);  // a min-heap of the teams' finishing times
-    double turn = 0.0;
-    for (double s : side) {
-      turn += 0.618034;
-      turn -= std::floor(turn);
-      std::pop_heap(ends.begin(), ends.end(), std::greater<double>());
-      ends.back() += (7.6 * s + 0.229 * s * s / R) * (0.1 + 1.8 * turn);
-      std::push_heap(ends.begin(), ends.end(), std::greater<double>());
-    }
-    const double us = *std::max_element(ends.begin(), ends.end());
-    if (teams == 1 || us < best_us) {
-      best_us = us;
-      best = R;
+  double best_loss = 0.0, best_alike = 0.0;
+  for (size_t i = 0; i < counts.size(); ++i) {
+    const double loss = std::max(alike[i] / alike_best / 1.3, differ[i] / differ_best);
+    if (i == 0 || loss < best_loss || (loss == best_loss && alike[i] < best_alike)) {
+      best_loss = loss;
+      best_alike = alike[i];
+      best = ctas / counts[i];
     }
   }
   return std::max(best, 2);
@@ -100,8 +126,8 @@ inline GroupSplit group_split(uint32_t n_jobs, int ctas, int team) {
 
 // The group modes (PropagOptions.cluster) an autotuner times for a batch: the
 // automatic one (0), a team per job, and teams of 24, 16, 8 and 4 CTAs, in case
-// the jobs differ from what team_size takes them to be (64 copies of one 1024^2
-// scenario: 126 ms with its teams of 9, 108 with teams of 4); of those that split
+// the jobs differ from what team_size takes them to be (20 copies of one 400^2
+// scenario: 6.7 ms with its 10 teams, 4.5 with 20); of those that split
 // the CTAs alike, one.  auto_team: the automatic team size, 0 when the automatic
 // mode is another one (clusters, or several teams on a lone job).
 inline std::vector<int> autotune_groups(uint32_t n_jobs, int ctas, int auto_team) {

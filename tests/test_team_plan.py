@@ -65,3 +65,34 @@ def test_autotuner_modes(plan, ctas, side):
                     assert _split(plan, n, ctas, team) in splits, (n, team)
             for slots, group in splits:
                 assert 1 <= slots <= n and group >= 2 and slots * group <= ctas
+
+
+def _alike(sides, teams, ctas):
+    """The end of a batch whose jobs take their mean time, on teams of equal size."""
+    ends = [0.0] * teams
+    for s in sorted(sides, reverse=True):
+        i = ends.index(min(ends))
+        ends[i] += 7.6 * s + 0.229 * s * s / (ctas // teams)
+    return max(ends)
+
+
+@pytest.mark.parametrize("side", [64.0, 150.0, 400.0, 700.0, 1024.0, 2000.0])
+def test_team_size_where_jobs_are_alike(plan, side):
+    """The teams chosen for differing jobs lose at most a factor 1.85 where the jobs
+    are alike, of any number (1.9 and more for 5 to 40 jobs before)."""
+    ctas = 148
+    for n in list(range(1, 80)) + [100, 148, 200]:
+        team = plan.plan_team(n, (C.c_double * n)(*[side] * n), ctas)
+        slots, group = _split(plan, n, ctas, team)
+        best = min(_alike([side] * n, t, ctas) for t in range(1, min(n, ctas // 2) + 1))
+        assert _alike([side] * n, slots, ctas) <= 1.85 * best, (n, slots)
+
+
+def test_team_size_of_uneven_batches(plan):
+    """A few large jobs among many small ones: few teams, so that the large ones
+    get many CTAs."""
+    ctas = 148
+    for sides in ([4096.0] + [128.0] * 100, [3000.0] * 2 + [500.0] * 10, [2048.0] * 3 + [256.0] * 40):
+        team = plan.plan_team(len(sides), (C.c_double * len(sides))(*sides), ctas)
+        assert team >= 37
+    assert plan.plan_team(1, (C.c_double * 1)(4096.0), ctas) == ctas
