@@ -261,11 +261,11 @@ struct Counters {
 // so the result is the first minimum of the offers when it beats the cell's
 // own time.  An offer that is NaN (of a neighbour whose fire is) is never the
 // smaller one there, and counts as infinite here: in a reduction by comparisons
-// it would hide the offers behind it.  The line of sight from the neighbour to its reference was walked
-// when it adopted the reference, and is read; only the walks the sequential
-// loop performs (candidate also faster than every earlier offer) are counted,
-// so the counters match the reference's order exactly.  Called by all 32
-// lanes.
+// it would hide the offers behind it.  The line of sight from the neighbour to
+// its reference was walked when it adopted the reference, and is read; only the
+// walks the sequential loop performs (candidate also faster than every earlier
+// offer) are counted, so the counters match the reference's order exactly.
+// Called by all 32 lanes.
 template <int kArith, typename Acc>
 __device__ __forceinline__ Best evaluate_coop(const JobDev &j, const DirConst &dc, const Acc &acc,
                                               int x, int y, Best own, bool valid, uint32_t lane,
@@ -1950,7 +1950,8 @@ __global__ void __launch_bounds__(kEngineThreads, 1)
 //
 // Why: a sweep is a chain of latencies whose length hardly depends on the CTAs
 // that share it, and one tile's front is too small for 148 of them.  4096^2, 20
-// ignitions: 445 ms in sequence, 199 ms with four teams of 37 CTAs.
+// ignitions: 443 ms in sequence, 201 ms with four teams of 37 CTAs; 2048^2 with 20:
+// 184 and 98.
 constexpr uint32_t kWaveStop = 0xFFFFFFFFu, kWaveIdle = 0xFFFFFFFEu;
 constexpr unsigned long long kWavePickNs = 1000000ull;  // 1 ms: a team's members wait that long at their barrier
 

@@ -15,9 +15,9 @@
 // codes); 32-bit indices serve every grid below 2^32 cells.  The pass is bound
 // by instruction issue and the warps in flight (360 instructions a cell; 516
 // with double-float moisture sums for every cell and single-word table reads:
-// 280 us at 4096^2, 213 now).  Four cells per thread with 128-bit loads measured slower
-// (0.298 against 0.277 ms: four inlined copies of the cell code overflow the
-// instruction cache), and so did loading a cell's inputs while the cell before
+// 283 us at 4096^2, 215 now, each pass alone).  Four cells per thread with
+// 128-bit loads measured slower (0.298 against 0.277 ms: four inlined copies of
+// the cell code overflow the instruction cache), and so did loading a cell's inputs while the cell before
 // it is computed (0.247 against 0.235 ms: 48 registers instead of 32 leave 40
 // warps per SM instead of 64).  The fuel table sits in shared memory, a row's
 // fields in the order they are read.  Compiled without automatic multiply-add
@@ -239,7 +239,8 @@ __device__ __forceinline__ void one_cell(const float *cat, const Inputs &in, con
 // operations, so both give the same values for them).
 // Index: uint32_t when n + the grid's threads fit in 32 bits (cheaper
 // address arithmetic), else uint64_t.  Six CTAs an SM: 40 registers (44 to 47
-// without the bound: 240 us against 225 at 4096^2; 32 for eight CTAs: 230).
+// without the bound: 240 us against 225 at 4096^2 in one wave of CTAs; 32 for
+// eight CTAs: 230).
 template <bool kFull, typename Index>
 __global__ void __launch_bounds__(256, 6) fire_kernel(Inputs in, Outputs out, Index first, Index n) {
   __shared__ __align__(16) float cat[kMaxFuels * kCatStride];
@@ -292,9 +293,9 @@ static int ctas_per_sm(K kernel, int threads) {
 // small grid's table copies and partial last wave would cost more than they
 // balance.  Up to four times as many when a thread still has eight cells to
 // compute: equal shares take unequal time (patches that do not burn, divergent
-// cells), and 4096^2 cells ran 229 us in one wave, with the SMs' warps active
-// 80 % of the time, 209 in four, 214 in sixteen; 1.9 M cells 45 us in one, 46 in
-// four, 52 in sixteen.
+// cells), and 4096^2 cells ran 231 us in one wave, with the SMs' warps active
+// 80 % of the time, 215 in four, 219 in sixteen; 1.9 M cells 37 us in one, 43 in
+// sixteen.
 static unsigned grid_for(uint64_t items, int threads, int sm_count, int per_sm) {
   const uint64_t wave = (uint64_t)sm_count * (uint64_t)per_sm;
   const uint64_t waves = items / (wave * (uint64_t)threads * 8);

@@ -10,8 +10,9 @@
 // that error of a point where the rounding changes; then (none to one cell in a
 // thousand by model, 0.04 % over all of them on ordinary moistures) the
 // double-float sums decide, so that the results are the double-float ones bit
-// for bit: a propagation depends on its fire fields to the last bit.  (4096^2 in 225 us; without the check 209, with the double-float
-// sums inlined 240, with those cells put off to the thread's end 246.)
+// for bit: a propagation depends on its fire fields to the last bit.  (4096^2 in
+// 215 us; without the check 207, with the double-float sums inlined 229, and with
+// those cells put off to the thread's end 1.09 times as long.)
 #pragma once
 
 #include <cmath>

@@ -50,7 +50,9 @@ inline double batch_us(const std::vector<double> &side, int teams, int ctas, boo
 // Measured, against the best number of teams: twelve batches of 5 to 256 ensemble
 // members and unrelated scenarios (three seeds) 1.03; 32 sizes of ensembles of 5 to
 // 50 members of 150^2 to 1024^2 (four seeds) 1.02, at most 1.10; the same with
-// copies of one member 1.26, at most 1.77.  The rule before, the number that ends
+// copies of one member 1.26, at most 1.77.  (56 sizes, 5 to 40 members of 80^2 to
+// 668^2, five seeds: 1.03, at most 1.36 for 34 members of 139^2; copies 1.08, at
+// most 1.71.)  The rule before, the number that ends
 // first when the jobs differ, of 1, 2, 3, 4, 6, 8, 12, 16, 24, 37, 49 and 74 teams:
 // 1.03, 1.12 (at most 1.55) and 1.64 (at most 1.90); a team per job up to 37: 1.41,
 // 1.20 (1.78) and 1.02.  20 members of 400^2: 12.9 ms in 10 teams, 15.6 in 20;
@@ -90,11 +92,17 @@ inline int team_size(std::vector<double> side, int ctas) {
 // tiles to run any of them at once.  A window of one tile of at least 257
 // cells, two of 129, three of 86 holds every reference of up to 256 cells'
 // offset: the longest lines of sight of the hilly and ridged scenarios are 160
-// to 218 steps, and a job with a longer one is run twice.  The number of teams
-// is what a simulation of the schedule with measured sweep times favours (in
-// sequence / 2 / 3 / 4 / 6 teams; 4096^2 with 20 ignitions: 478 / 265 / 208 / 186 /
-// 212 ms; 2048^2 with 20: 103 / 58 / 53 / 59 / 71, with one: 49 / 33 / 35 / 37 /
-// 45).
+// to 218 steps, and a job with a longer one is begun again in sequence.  The
+// number of teams is what a simulation of the schedule with the sweep times
+// measured then favoured (in sequence / 2 / 3 / 4 / 6 teams; 4096^2 with 20
+// ignitions: 478 / 265 / 208 / 186 / 212 ms; 2048^2 with 20: 103 / 58 / 53 / 59 / 71,
+// with one: 49 / 33 / 35 / 37 / 45).
+//
+// Measured, in sequence on all CTAs against these teams: ridged 4096^2 with 20
+// ignitions (three seeds) 364 / 378 / 434 and 158 / 167 / 181 ms, hilly 2048^2 with
+// 20: 184 and 98, 1024^2 with one: 14.1 and 13.8.  On constant ground, where lines
+// of sight grow as wide as the fire, the run is begun twice: 1024^2 with one
+// ignition 121 and 137 ms, stopped after 7200 s 8.9 and 16.6, 2048^2 803 and 821.
 struct WavePlan {
   uint32_t teams = 0;
   int window = 0;
